@@ -267,7 +267,9 @@ int owt_state_restore(owt_handle *h);
  * OWT_OPT_FFT_STOCKHAM: 1 = the mixed precision's FP32 transforms use the
  *   shared-memory Stockham kernels (one pass per radix-2/3/4/5 stage) even
  *   where register-transform kernels exist for the line length (the two
- *   agree to FP32 rounding; this exists to compare them).
+ *   agree to FP32 rounding; this exists to compare them), and the FP64
+ *   transforms their FP64 Stockham kernels instead of the fixed-point ones
+ *   (they agree to FP64 rounding).
  * OWT_OPT_MEAN_SPLIT: mixed precision only; 1 (the default) = the FP32
  *   transforms carry the fluctuations, and the mean-flow terms of the Lamb
  *   vector (mean velocity x fluctuating vorticity and back) are formed mode

@@ -131,6 +131,7 @@ struct owt_handle {
   void *zbuf = nullptr, *lbuf = nullptr;
   void *twx[2] = {nullptr, nullptr}, *twz[2] = {nullptr, nullptr};
   owt::FftPlan px{}, pz{};
+  owt::FxTw *fxx = nullptr, *fxz = nullptr;  // twiddles of the fixed-point FP64 transforms
   // wall blowing/suction: v on the walls, [2][M] (bottom, top); null = no-slip
   double2 *vw = nullptr;
   bool vw_on = false;
@@ -176,7 +177,7 @@ struct owt_handle {
   void run_steps(int64_t n);
   int64_t per_step_launches = 0;
   bool force_dense = false;  // testing aid: always sweep the full band
-  bool fft_stockham = false; // FP32 transforms: shared-memory Stockham kernels instead of register ones
+  bool fft_stockham = false; // transforms by the shared-memory Stockham kernels instead of the register / fixed-point ones
   bool mean_split = true;    // mixed precision: the mean-flow terms of the Lamb vector mode by mode beside the transforms
   int host_chunks = 0;       // owt_time_integration_host: chunks of modes (0: the default)
   bool mean_smem = false;    // staged mean-mode solve in shared memory

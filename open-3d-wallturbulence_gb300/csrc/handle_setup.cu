@@ -299,6 +299,10 @@ void owt_handle::setup(const owt_params &prm) {
       (axis == 0 ? twx : twz)[prec] = d;
     }
   }
+  for (int axis = 0; axis < 2; ++axis) {  // fixed-point FP64 transforms
+    const FxPlan plan = fx_plan(axis == 0 ? NX2 : NZ2);
+    if (plan.cls >= 0) (axis == 0 ? fxx : fxz) = upload(fx_twiddles(plan), owned, st);
+  }
   for (double2 *ring : {v_ring, g_ring, hv_ring, hg_ring, q_ring})
     ck(cudaMemsetAsync(ring, 0, 3 * fs * sizeof(double2), st), "memset");
   for (double2 *f : {u, w, ox, oz, lx, ly, lz})

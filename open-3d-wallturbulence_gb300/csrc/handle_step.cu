@@ -33,6 +33,8 @@ XformArgs owt_handle::xform_args() const {
   a.twx = twx[precision]; a.twz = twz[precision];
   a.inv_nx2 = 1.0 / (double)NX2; a.inv_nz2 = 1.0 / (double)NZ2;
   a.stockham = fft_stockham ? 1 : 0;
+  a.fpx = fx_plan(NX2); a.fpz = fx_plan(NZ2);
+  a.fxx = fxx; a.fxz = fxz;
   return a;
 }
 

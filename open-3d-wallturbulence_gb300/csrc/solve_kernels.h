@@ -4,9 +4,13 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <map>
 #include <mutex>
+#include <tuple>
 
 #include "batch.cuh"
+#include "fft_fix.cuh"
 #include "owt_device.cuh"
 
 namespace owt {
@@ -132,8 +136,36 @@ struct XformArgs {
   FftPlan px, pz;
   const void *twx, *twz;  // tables of exp(-2 pi i k/L) in T precision
   double inv_nx2, inv_nz2;
-  int stockham;  // FP32: 1 = the shared-memory Stockham kernels even where register ones exist
+  int stockham;  // 1 = the shared-memory Stockham kernels even where register ones exist
+  // FP64 in fixed point (fft_fix.cuh): plans of the x and z lines (class -1:
+  // none) and their twiddle tables (fx_twiddles)
+  FxPlan fpx, fpz;
+  const FxTw *fxx, *fxz;
 };
+
+// Blocks of a persistent kernel that are resident at once on the current
+// device, found once per kernel, shape and device; at least 1.
+inline int resident_blocks(const void *kernel, int threads, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, const void *, int, size_t>, int> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+  std::lock_guard<std::mutex> lk(mu);
+  int &n = known[std::make_tuple(dev, kernel, threads, smem)];
+  if (n == 0) {
+    int sms = 0, per = 0;
+    n = 1;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) == cudaSuccess)
+      n = std::max(per, 1) * sms;
+  }
+  return n;
+}
+template <typename... A>
+inline int resident_blocks(void (*kernel)(A...), int threads, size_t smem) {
+  if (raise_smem_limit(kernel, smem) != cudaSuccess) return 1;
+  return resident_blocks(reinterpret_cast<const void *>(kernel), threads, smem);
+}
 
 bool band_supported(int kl, int ku);
 // d2f_bits against the hardware conversion on n samples (counts: see
@@ -203,6 +235,19 @@ struct RegXformKernels {
   size_t zsmem = 0, xsmem = 0;
 };
 RegXformKernels reg_xform_kernels(int L);
+// FP64 transform kernels in fixed point (transforms_fix.cuh) for line length
+// L: kernels, shapes and shared memory; ok = false where L has no plan.
+struct FxXformKernels {
+  bool ok = false;
+  void (*zback)(XformArgs) = nullptr, (*xlamb)(XformArgs) = nullptr, (*zfwd)(XformArgs) = nullptr;
+  void (*zback_b)(BatchTable<XformArgs>) = nullptr, (*xlamb_b)(BatchTable<XformArgs>) = nullptr,
+      (*zfwd_b)(BatchTable<XformArgs>) = nullptr;
+  int tx = 0, zthreads = 0, xthreads = 0, xlines = 0;  // kx columns per z block, (y, z) lines per x group
+  size_t zsmem = 0, xsmem = 0;
+};
+FxXformKernels fx_xform_kernels0(int L);  // by class of the plan
+FxXformKernels fx_xform_kernels1(int L);
+FxXformKernels fx_xform_kernels2(int L);
 // Stand-alone FP64 dealiased transforms of one field (zbuf / lbuf field 0 in
 // between): a.in[0] -> phys [y][z][x], and phys -> a.out[0].
 cudaError_t phys_prepare(const XformDims &d);

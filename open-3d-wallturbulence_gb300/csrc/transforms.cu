@@ -22,7 +22,11 @@
 //
 // Between kernels the z-padded, x-truncated planes live in HBM as
 // [field][y][z][kx] complex<T>.  T = double (FP64 step) or float (mixed).
+// The kernels here serve any line length; transforms_reg.cu (FP32) and
+// transforms_fix.cuh (FP64, in fixed point) have faster ones for most.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "mean_flow.cuh"
 #include "owt_device.cuh"
@@ -328,21 +332,36 @@ static int x_lines(const XformDims &d) {
 // FP32 lines with a two-pass factorisation (transforms_reg.cu) use the
 // register-transform kernels unless `stockham` is set; they keep TX = 12
 // columns per z block, and P (y, z) lines per x block of their own.
+// FP64 lines with a plan (fx_plan) use the fixed-point kernels
+// (transforms_fix.cuh) unless `stockham` is set; the FP64 kernels above serve
+// the other lengths (600 points and more, and those with a factor 27 or 25
+// left over).
 template <typename T>
 struct XformKernels {
   int P;
+  int tx;  // kx columns per z block
   void (*zback)(XformArgs), (*xlamb)(XformArgs), (*zfwd)(XformArgs);
   void (*zback_b)(BatchTable<XformArgs>), (*xlamb_b)(BatchTable<XformArgs>), (*zfwd_b)(BatchTable<XformArgs>);
   int zthreads, xthreads;
   size_t zsmem, xsmem;
   int xgrid;  // x-pass blocks at most (0: one block per group of P lines)
 };
+static FxXformKernels fx_kernels(int L) {
+  switch (fx_plan(L).cls) {
+    case 0: return fx_xform_kernels0(L);
+    case 1: return fx_xform_kernels1(L);
+    case 2: return fx_xform_kernels2(L);
+    default: return FxXformKernels{};
+  }
+}
+
 template <typename T>
 static XformKernels<T> kernels(const XformDims &d, bool stockham = false) {
   constexpr int PP = XCfg<T>::P;
   const bool z5 = d.NZ2 % 5 == 0, x5 = d.NX2 % 5 == 0;
   XformKernels<T> k;
   k.P = x_lines<T>(d);
+  k.tx = XCfg<T>::TX;
   k.zthreads = d.NZ2;
   k.xthreads = d.NX2;
   k.zsmem = smem_z<T>(d);
@@ -375,6 +394,22 @@ static XformKernels<T> kernels(const XformDims &d, bool stockham = false) {
       k.xgrid = rx.xgrid;
     }
   }
+  if (sizeof(T) == sizeof(double) && !stockham) {
+    const FxXformKernels fz = fx_kernels(d.NZ2), fx = fx_kernels(d.NX2);
+    if (fz.ok) {
+      k.zback = fz.zback; k.zfwd = fz.zfwd; k.zback_b = fz.zback_b; k.zfwd_b = fz.zfwd_b;
+      k.tx = fz.tx;
+      k.zthreads = fz.zthreads;
+      k.zsmem = fz.zsmem;
+    }
+    if (fx.ok) {
+      k.xlamb = fx.xlamb; k.xlamb_b = fx.xlamb_b;
+      k.xthreads = fx.xthreads;
+      k.xsmem = fx.xsmem;
+      k.P = fx.xlines;
+      k.xgrid = resident_blocks(fx.xlamb, fx.xthreads, fx.xsmem);
+    }
+  }
   return k;
 }
 
@@ -384,16 +419,16 @@ template <typename T>
 static void lamb_part_t(const XformArgs &a, int part, cudaStream_t st) {
   const XformDims &d = a.d;
   const XformKernels<T> k = kernels<T>(d, a.stockham != 0);
-  constexpr int TX = XCfg<T>::TX;
+  const int gx = (d.NXH + k.tx - 1) / k.tx;
   if (part == 0) {
-    k.zback<<<dim3((d.NXH + TX - 1) / TX, d.NY, 6), k.zthreads, k.zsmem, st>>>(a);
+    k.zback<<<dim3(gx, d.NY, 6), k.zthreads, k.zsmem, st>>>(a);
   } else if (part == 1) {
     const size_t nl = (size_t)d.NY * d.NZ2;
     size_t grid = (nl + k.P - 1) / k.P;
     if (k.xgrid > 0 && grid > (size_t)k.xgrid) grid = k.xgrid;
     k.xlamb<<<(unsigned)grid, k.xthreads, k.xsmem, st>>>(a);
   } else if (part == 2) {
-    k.zfwd<<<dim3((d.NXH + TX - 1) / TX, d.NY, 3), k.zthreads, k.zsmem, st>>>(a);
+    k.zfwd<<<dim3(gx, d.NY, 3), k.zthreads, k.zsmem, st>>>(a);
   } else if (a.mean_split) {
     launch_mean_lamb(a, st);
   }
@@ -443,13 +478,11 @@ void launch_lamb_part(const XformArgs &a, int precision, int part, cudaStream_t 
 // 3 (mean-flow terms); the grids of the one-channel launches, flattened.
 template <typename T>
 static int lamb_blocks_t(const XformDims &d, int part, bool stockham) {
-  const int gx = (d.NXH + XCfg<T>::TX - 1) / XCfg<T>::TX;
+  const XformKernels<T> k = kernels<T>(d, stockham);
+  const int gx = (d.NXH + k.tx - 1) / k.tx;
   if (part == 0) return gx * d.NY * 6;
   if (part == 2) return gx * d.NY * 3;
-  if (part == 1) {
-    const int P = kernels<T>(d, stockham).P;
-    return (int)(((size_t)d.NY * d.NZ2 + P - 1) / P);
-  }
+  if (part == 1) return (int)(((size_t)d.NY * d.NZ2 + k.P - 1) / k.P);
   return ((d.NZ * d.NXH + 255) / 256) * d.NY;
 }
 int lamb_batch_blocks(const XformDims &d, int precision, int part, bool stockham) {
@@ -490,9 +523,8 @@ cudaError_t phys_prepare(const XformDims &d) {
 // a.in[0] (spectral [y][kz][kx], FP64 tables) -> phys [y][z][x]; zbuf field 0 in between.
 void launch_fourier2physical(const XformArgs &a, double *phys, cudaStream_t st) {
   const XformDims &d = a.d;
-  const XformKernels<double> k = kernels<double>(d);
-  constexpr int TX = XCfg<double>::TX;
-  k.zback<<<dim3((d.NXH + TX - 1) / TX, d.NY, 1), d.NZ2, smem_z<double>(d), st>>>(a);
+  const XformKernels<double> k = kernels<double>(d, a.stockham != 0);
+  k.zback<<<dim3((d.NXH + k.tx - 1) / k.tx, d.NY, 1), k.zthreads, k.zsmem, st>>>(a);
   const size_t nl = (size_t)d.NY * d.NZ2;
   const unsigned blocks = (unsigned)((nl + 2 * kPhysQ - 1) / (2 * kPhysQ));
   if (d.NX2 % 5 == 0) k_xback_phys<true><<<blocks, d.NX2, smem_phys(d), st>>>(a, phys);
@@ -501,13 +533,12 @@ void launch_fourier2physical(const XformArgs &a, double *phys, cudaStream_t st) 
 // phys [y][z][x] -> a.out[0] (spectral); lbuf field 0 in between.
 void launch_physical2fourier(const XformArgs &a, const double *phys, cudaStream_t st) {
   const XformDims &d = a.d;
-  const XformKernels<double> k = kernels<double>(d);
-  constexpr int TX = XCfg<double>::TX;
+  const XformKernels<double> k = kernels<double>(d, a.stockham != 0);
   const size_t nl = (size_t)d.NY * d.NZ2;
   const unsigned blocks = (unsigned)((nl + 2 * kPhysQ - 1) / (2 * kPhysQ));
   if (d.NX2 % 5 == 0) k_xfwd_phys<true><<<blocks, d.NX2, smem_phys(d), st>>>(a, phys);
   else k_xfwd_phys<false><<<blocks, d.NX2, smem_phys(d), st>>>(a, phys);
-  k.zfwd<<<dim3((d.NXH + TX - 1) / TX, d.NY, 1), d.NZ2, smem_z<double>(d), st>>>(a);
+  k.zfwd<<<dim3((d.NXH + k.tx - 1) / k.tx, d.NY, 1), k.zthreads, k.zsmem, st>>>(a);
 }
 
 size_t lamb_zbuf_bytes(const XformDims &d, int precision) {

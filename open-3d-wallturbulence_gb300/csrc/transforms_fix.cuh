@@ -1,0 +1,474 @@
+// Transform kernels of the FP64 step with 64-bit fixed-point line transforms
+// (fft_fix.cuh): the three kernels, data layouts and dealiasing of
+// transforms.cu (src/FFT.cpp:49-194, src/solver.cpp:262-304), FP64 in memory
+// and in the physical-space products, for the line lengths with a plan
+// (fx_plan).  One translation unit per plan class instantiates them
+// (transforms_fix0.cu, ...), so that the register budget of a kernel is that
+// of its largest radix and the units compile in parallel.
+//
+// A line of A B points has T = max(A, B) threads; every thread of a block
+// takes part in every barrier, those beyond the number of a pass's transforms
+// idle in it.
+//
+//  k_zback_fx : block (kTX kx columns, y, field), column fastest in the
+//               thread index so that rows of kx coalesce; the padded z line
+//               is gathered straight into pass-1 registers.
+//  k_xlamb_fx : persistent; per group of P (y, z) lines: 3P packed backward
+//               lines, products in FP64 in shared memory, 3P/2 packed
+//               forward lines, the real-pair unpack; the next group's input
+//               is prefetched into L2.
+//  k_zfwd_fx  : as k_zback_fx, forward.
+//
+// Measured at 384x257x384 (lines of 576 points), FP64 kernels -> these:
+// z backward 10.74 -> 1.64 ms, x pass 27.99 -> 7.85 ms, z forward
+// 5.27 -> 0.95 ms; at 128x129x128 0.496 -> 0.095, 1.189 -> 0.470 and
+// 0.255 -> 0.061 ms.  The z passes are bound by integer issue at half of the
+// DRAM rate.  The x pass is latency bound (1.3 instructions a clock, the FP64
+// pipe of the conversions and products 43% busy, 15 warps an SM): its 24-point
+// transforms fit 128 registers with 90 bytes of spills, so that three blocks
+// are resident (two at 168 registers: 12.2 ms, before the zero thirds were
+// left out).
+#pragma once
+#include <cuda_runtime.h>
+
+#include "batch.cuh"
+#include "fft_fix.cuh"
+#include "owt_device.cuh"
+#include "solve_kernels.h"
+
+namespace owt {
+
+// Block shapes by plan class: kx columns per z block, (y, z) lines per x
+// group, and the resident blocks asked of the register allocator.
+template <int CLS> struct FxCfg;
+template <> struct FxCfg<0> { static constexpr int T = 12, TX = 8, P = 4, ZB = 6, XB = 4; };
+template <> struct FxCfg<1> { static constexpr int T = 18, TX = 8, P = 2, ZB = 3, XB = 4; };
+template <> struct FxCfg<2> { static constexpr int T = 24, TX = 8, P = 2, ZB = 2, XB = 3; };
+
+__device__ __forceinline__ fxc fx_bits(double2 v) {
+  return fxc{__double_as_longlong(v.x), __double_as_longlong(v.y)};
+}
+
+__device__ __forceinline__ FxTw fx_ldg(const FxTw *p) {
+  const int4 v = __ldg(reinterpret_cast<const int4 *>(p));
+  return FxTw{v.x, v.y, v.z, v.w};
+}
+
+// The rest of pass 1 once the line's scale is known: x (doubles' bits) to
+// integers, N-point transform, output r times twiddle(r) to store(r, value).
+template <int N, bool BACKWARD, class Twiddle, class Store>
+__device__ __forceinline__ void fx_line_pass1(fxc *x, const FxScale &s, Twiddle twiddle, Store store) {
+  fx_for<0, N>([&](auto rc) {
+    constexpr int r = decltype(rc)::value;
+    if constexpr (!BACKWARD || N % 3 != 0 || r < N / 3 || r >= 2 * N / 3)
+      x[r] = fxc{fx_from_bits(x[r].x, s), fx_from_bits(x[r].y, s)};
+  });
+  fx_dft<N, BACKWARD>(x);
+  store(0, fx_quarter(x[0]));
+  fx_for<1, N>([&](auto rc) {
+    constexpr int r = decltype(rc)::value;
+    store(r, fx_twiddle<BACKWARD>(x[r], twiddle(r)));
+  });
+}
+
+// Shared memory of a z block: the transposes of TX lines ([a'][b][column]),
+// the bounds and scales of its lines.
+template <int CLS>
+__host__ __device__ constexpr size_t fx_zsmem(int L) {
+  return (size_t)FxCfg<CLS>::TX * (L * sizeof(fxc) + FxCfg<CLS>::T * sizeof(FxBound) + sizeof(FxScale));
+}
+
+// One block of line transforms along z.  load(r, s) gives slot s = t + N2 r of
+// this thread's column (r a compile-time index), store(r, s, value, scale)
+// takes output slot s = t + N1 r.  The middle third of the slots is zero in a
+// backward transform's input and unused in a forward transform's output.
+template <int CLS, bool BACKWARD, class Load, class Store>
+__device__ __forceinline__ void fx_z_lines(const FxPlan p, const FxTw *__restrict__ tw, Load load, Store store) {
+  constexpr int TX = FxCfg<CLS>::TX;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int L = p.A * p.B, N1 = BACKWARD ? p.A : p.B, N2 = BACKWARD ? p.B : p.A;
+  fxc *S = reinterpret_cast<fxc *>(smraw);
+  FxBound *bd = reinterpret_cast<FxBound *>(S + (size_t)TX * L);
+  FxScale *sc = reinterpret_cast<FxScale *>(bd + TX * FxCfg<CLS>::T);
+  const int c = threadIdx.x % TX, t = threadIdx.x / TX;
+  if (!BACKWARD) tw += L;
+  fx_radix<CLS>(N1, [&](auto n) {
+    constexpr int N = decltype(n)::value;
+    fxc x[N];
+    fx_for<0, N>([&](auto rc) { x[decltype(rc)::value] = fxc{0, 0}; });
+    if (t < N2) {
+      fx_for<0, N>([&](auto rc) {
+        constexpr int r = decltype(rc)::value;
+        if constexpr (!BACKWARD || N % 3 != 0 || r < N / 3 || r >= 2 * N / 3) x[r] = fx_bits(load(rc, t + N2 * r));
+      });
+      bd[t * TX + c] = fx_bound<N>(x);
+    }
+    __syncthreads();
+    if (t < N2) {
+      const FxScale s = fx_scale(N2, [&](int k) { return bd[k * TX + c]; });
+      if (t == 0) sc[c] = s;
+      fx_line_pass1<N, BACKWARD>(x, s, [&](int r) { return fx_ldg(tw + r * N2 + t); },
+                                 [&](int r, fxc v) { S[(r * N2 + t) * TX + c] = v; });
+    }
+  });
+  __syncthreads();
+  if (t < N1)
+    fx_radix<CLS>(N2, [&](auto n) {
+      constexpr int N = decltype(n)::value;
+      fxc y[N];
+      fx_for<0, N>([&](auto rc) { y[decltype(rc)::value] = S[(t * N + decltype(rc)::value) * TX + c]; });
+      fx_dft<N, BACKWARD>(y);
+      const FxScale s = sc[c];
+      fx_for<0, N>([&](auto rc) {
+        constexpr int r = decltype(rc)::value;
+        if constexpr (BACKWARD || N % 3 != 0 || r < N / 3 || r >= 2 * N / 3) store(rc, t + N1 * r, y[r], s);
+      });
+    });
+}
+
+template <int CLS>
+__device__ __forceinline__ void zback_fx_body(const XformArgs &a, const int bx, const int j, const int f) {
+  const XformDims d = a.d;
+  const int i = bx * FxCfg<CLS>::TX + threadIdx.x % FxCfg<CLS>::TX;
+  const bool col = i < d.NXH;
+  const double2 *base = a.in[f];
+  if (a.ring_mask & (1 << f)) base += (size_t)ring_head(*a.step) * a.fs;
+  const double2 *src = base + (size_t)j * d.NZ * d.NXH + i;
+  double2 *dst = reinterpret_cast<double2 *>(a.zbuf) + ((size_t)f * d.NY + j) * d.NZ2 * d.NXH + i;
+  fx_z_lines<CLS, true>(
+      a.fpz, a.fxz,
+      [&](auto, int s) {  // slot of the padded line: k < NZH -> k, k > NZH -> k + NZH, the Nyquist row dropped
+        const int kz = s < d.NZH ? s : s > d.NZ ? s - d.NZH : -1;
+        return col && kz >= 0 ? src[(size_t)kz * d.NXH] : make_double2(0.0, 0.0);
+      },
+      [&](auto, int s, fxc v, const FxScale &sc) {
+        const FxOut o = fx_out(sc);
+        if (col) dst[(size_t)s * d.NXH] = make_double2(fx_to_double(v.x, o), fx_to_double(v.y, o));
+      });
+}
+
+template <int CLS>
+__device__ __forceinline__ void zfwd_fx_body(const XformArgs &a, const int bx, const int j, const int f) {
+  const XformDims d = a.d;
+  const int i = bx * FxCfg<CLS>::TX + threadIdx.x % FxCfg<CLS>::TX;
+  const bool col = i < d.NXH;
+  const double2 *src = reinterpret_cast<const double2 *>(a.lbuf) + ((size_t)f * d.NY + j) * d.NZ2 * d.NXH + i;
+  double2 *dst = a.out[f] + (size_t)j * d.NZ * d.NXH + i;
+  fx_z_lines<CLS, false>(
+      a.fpz, a.fxz, [&](auto, int s) { return col ? src[(size_t)s * d.NXH] : make_double2(0.0, 0.0); },
+      [&](auto, int s, fxc v, const FxScale &sc) {  // keep slots k < NZH (kz k) and NZ + k (kz k + NZH)
+        const int kz = s < d.NZH ? s : s >= d.NZ ? s - d.NZH : -1;
+        if (col && kz >= 0) {
+          const double w = a.inv_nz2 * fx_factor(sc);
+          dst[(size_t)kz * d.NXH] = make_double2(__dmul_rn(__ll2double_rn(v.x), w), __dmul_rn(__ll2double_rn(v.y), w));
+        }
+      });
+}
+
+// ---------------------------------------------------------------------------
+// x pass
+// ---------------------------------------------------------------------------
+// Point m = t + N2 r of the packed line of two real lines' spectra A, B
+// (hermitian_pair of owt_device.cuh): UPPER (r in the upper third) takes the
+// conjugate half, the padding slot 2 NX2/3 included as zero.  have, have_b:
+// the lines exist (else zeros).
+template <bool UPPER>
+__device__ __forceinline__ double2 fx_hermitian(const double2 *__restrict__ A, size_t fstride, bool have, int m, int NXH,
+                                                int NX2, bool have_b = true) {
+  const int mp = UPPER ? NX2 - m : m;
+  double2 x = make_double2(0.0, 0.0), y = x;
+  if (have && mp < NXH) {
+    x = __ldg(A + mp);
+    if (have_b) y = __ldg(A + fstride + mp);
+  }
+  if (UPPER) return make_double2(x.x + y.y, y.x - x.y);
+  if (m == 0) x.y = y.y = 0.0;
+  return make_double2(x.x - y.y, x.y + y.x);
+}
+
+// Shared memory: 3P lines of LS values (transposes with odd row stride, or
+// the line itself), the twiddle tables (one where A = B), bounds and scales.
+__host__ __device__ constexpr int fx_row(int B) { return B | 1; }
+__host__ __device__ constexpr int fx_xline(int A, int B) {
+  return A * fx_row(B) > B * fx_row(A) ? A * fx_row(B) : B * fx_row(A);
+}
+__host__ __device__ constexpr int fx_xtables(int A, int B) { return (A == B ? 1 : 2) * A * B; }
+template <int CLS>
+constexpr size_t fx_xsmem(int A, int B) {
+  constexpr int P = FxCfg<CLS>::P;
+  return 3 * P * (size_t)fx_xline(A, B) * sizeof(fxc) + (size_t)fx_xtables(A, B) * sizeof(FxTw) +
+         3 * P * ((size_t)FxCfg<CLS>::T * sizeof(FxBound) + sizeof(FxScale));
+}
+
+// Pass 1 of line q's transform on input in(r, s) (s = t + N2 r), its
+// transposes to R[r RS + t] of its line; the line's scale to sc[q].  act: the
+// thread has a transform in this pass.  All threads call it.
+template <int CLS, bool BACKWARD, class In>
+__device__ __forceinline__ void fx_x_pass1(const FxPlan p, bool act, int q, int t, In in, fxc *R, const FxTw *tw,
+                                           FxBound *bd, FxScale *sc) {
+  const int N1 = BACKWARD ? p.A : p.B, N2 = BACKWARD ? p.B : p.A, RS = fx_row(N2);
+  bd += q * p.T;
+  fx_radix<CLS>(N1, [&](auto n) {
+    constexpr int N = decltype(n)::value;
+    fxc x[N];
+    // (set on both paths: left undefined where !act, they would be kept in
+    // local memory around the loop over groups)
+    fx_for<0, N>([&](auto rc) { x[decltype(rc)::value] = fxc{0, 0}; });
+    if (act) {
+      fx_for<0, N>([&](auto rc) {
+        constexpr int r = decltype(rc)::value;
+        if constexpr (!BACKWARD || N % 3 != 0 || r < N / 3 || r >= 2 * N / 3)
+          x[r] = fx_bits(in(std::integral_constant<bool, (r >= 2 * N / 3)>{}, t + N2 * r));
+      });
+      bd[t] = fx_bound<N>(x);
+    }
+    __syncthreads();
+    if (act) {
+      const FxScale s = fx_scale(N2, [&](int k) { return bd[k]; });
+      if (t == 0) sc[q] = s;
+      fx_line_pass1<N, BACKWARD>(x, s, [&](int r) { return tw[r * N2 + t]; },
+                                 [&](int r, fxc v) { R[r * RS + t] = v; });
+    }
+  });
+}
+
+// Backward pass 2 of line q: point t + A r as FP64, in place (R: the line).
+template <int CLS>
+__device__ __forceinline__ void fx_x_pass2_back(const FxPlan p, bool act, int t, fxc *R, const FxScale *sc) {
+  const int A = p.A;
+  fx_radix<CLS>(p.B, [&](auto n) {
+    constexpr int N = decltype(n)::value, RS = fx_row(N);
+    fxc y[N];
+    fx_for<0, N>([&](auto rc) { y[decltype(rc)::value] = fxc{0, 0}; });
+    if (act) {
+      fx_for<0, N>([&](auto rc) { y[decltype(rc)::value] = R[t * RS + decltype(rc)::value]; });
+      fx_dft<N, true>(y);
+    }
+    __syncthreads();
+    if (act) {
+      const FxOut o = fx_out(*sc);
+      double2 *D = reinterpret_cast<double2 *>(R);
+      fx_for<0, N>([&](auto rc) {
+        constexpr int r = decltype(rc)::value;
+        D[t + A * r] = make_double2(fx_to_double(y[r].x, o), fx_to_double(y[r].y, o));
+      });
+    }
+  });
+}
+
+// Forward pass 2: spectrum slot t + B r, integers, from the transposes at R
+// into the line at out (the middle third is not read).  No barrier.
+template <int CLS>
+__device__ __forceinline__ void fx_x_pass2_fwd(const FxPlan p, int t, const fxc *R, fxc *out) {
+  const int B = p.B;
+  fx_radix<CLS>(p.A, [&](auto n) {
+    constexpr int N = decltype(n)::value, RS = fx_row(N);
+    fxc y[N];
+    fx_for<0, N>([&](auto rc) { y[decltype(rc)::value] = R[t * RS + decltype(rc)::value]; });
+    fx_dft<N, false>(y);
+    fx_for<0, N>([&](auto rc) {
+      constexpr int r = decltype(rc)::value;
+      if constexpr (N % 3 != 0 || r < N / 3 || r >= 2 * N / 3) out[t + B * r] = y[r];
+    });
+  });
+}
+
+template <int CLS>
+__device__ __forceinline__ void xlamb_fx_group(const XformArgs &a, const size_t line0, fxc *R, const FxTw *tw,
+                                               FxBound *bd, FxScale *sc) {
+  constexpr int P = FxCfg<CLS>::P, NF = P + P / 2;
+  const XformDims d = a.d;
+  const FxPlan p = a.fpx;
+  const int A = p.A, B = p.B, LS = fx_xline(A, B);
+  const int q = threadIdx.x / p.T, t = threadIdx.x - q * p.T;
+  const size_t nlines = (size_t)d.NY * d.NZ2, fstride = nlines * d.NXH;
+  // 1. backward pass 1: packed line q = pair P + l holds fields (2 pair, 2 pair + 1)
+  {
+    const int pair = q / P, l = q - pair * P;
+    const bool have = line0 + l < nlines;
+    const double2 *Af = reinterpret_cast<const double2 *>(a.zbuf) + (size_t)(2 * pair) * fstride + (line0 + l) * d.NXH;
+    fx_x_pass1<CLS, true>(
+        p, t < B, q, t,
+        [&](auto upper, int s) { return fx_hermitian<decltype(upper)::value>(Af, fstride, have, s, d.NXH, d.NX2); },
+        R + q * LS, tw, bd, sc);
+  }
+  __syncthreads();
+  // 2. backward pass 2
+  fx_x_pass2_back<CLS>(p, t < A, t, R + q * LS, sc + q);
+  __syncthreads();
+  // 3. lamb = u x omega (no fused multiply-add, as the reference's separate
+  // products), packed as (lx + i ly) in line l and (lz_l + i lz_l+1) in line
+  // P + l/2, in place: one thread owns point xx of every line
+  double2 *D = reinterpret_cast<double2 *>(R);
+  for (int xx = threadIdx.x; xx < A * B; xx += blockDim.x) {
+    double2 uv[P], wox[P], oyz[P];
+#pragma unroll
+    for (int l = 0; l < P; ++l) {
+      uv[l] = D[(0 * P + l) * LS + xx];
+      wox[l] = D[(1 * P + l) * LS + xx];
+      oyz[l] = D[(2 * P + l) * LS + xx];
+    }
+#pragma unroll
+    for (int l = 0; l < P; l += 2) {
+      double lz[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double u = uv[l + h].x, v = uv[l + h].y, w = wox[l + h].x, ox = wox[l + h].y, oy = oyz[l + h].x,
+                     oz = oyz[l + h].y;
+        const double lx = __dsub_rn(__dmul_rn(v, oz), __dmul_rn(w, oy));
+        const double ly = __dsub_rn(__dmul_rn(w, ox), __dmul_rn(u, oz));
+        lz[h] = __dsub_rn(__dmul_rn(u, oy), __dmul_rn(v, ox));
+        D[(l + h) * LS + xx] = make_double2(lx, ly);
+      }
+      D[(P + l / 2) * LS + xx] = make_double2(lz[0], lz[1]);
+    }
+  }
+  __syncthreads();
+  // 4. forward pass 1 of the NF product lines, transposes into lines NF + q
+  fx_x_pass1<CLS, false>(
+      p, q < NF && t < A, q, t, [&](auto, int s) { return D[q * LS + s]; }, R + (NF + q) * LS,
+      A == B ? tw : tw + A * B, bd, sc);
+  __syncthreads();
+  // 5. forward pass 2 into line q
+  if (q < NF && t < B) fx_x_pass2_fwd<CLS>(p, t, R + (NF + q) * LS, R + q * LS);
+  __syncthreads();
+  // 6. unpack the real-pair spectra, keep kx < NXH, scale by 1/NX2:
+  // Xa = (Z[m] + conj Z[-m]) / 2 ; Xb = (Z[m] - conj Z[-m]) / (2i)
+  double2 *lb = reinterpret_cast<double2 *>(a.lbuf);
+  const double half = 0.5 * a.inv_nx2;
+  for (int idx = threadIdx.x; idx < P * d.NXH; idx += blockDim.x) {
+    const int l = idx / d.NXH, km = idx - l * d.NXH;
+    const size_t line = line0 + l;
+    if (line >= nlines) continue;
+    const int mc = (km == 0) ? 0 : d.NX2 - km;
+    {
+      const double w = half * fx_factor(sc[l]);
+      const fxc zm = R[l * LS + km], zc = R[l * LS + mc];
+      lb[line * d.NXH + km] =
+          make_double2(__dmul_rn(__ll2double_rn(zm.x + zc.x), w), __dmul_rn(__ll2double_rn(zm.y - zc.y), w));
+      lb[fstride + line * d.NXH + km] =
+          make_double2(__dmul_rn(__ll2double_rn(zm.y + zc.y), w), __dmul_rn(__ll2double_rn(zc.x - zm.x), w));
+    }
+    {
+      const double w = half * fx_factor(sc[P + l / 2]);
+      const fxc zm = R[(P + l / 2) * LS + km], zc = R[(P + l / 2) * LS + mc];
+      const long long vx = (l & 1) ? zm.y + zc.y : zm.x + zc.x, vy = (l & 1) ? zc.x - zm.x : zm.y - zc.y;
+      lb[2 * fstride + line * d.NXH + km] =
+          make_double2(__dmul_rn(__ll2double_rn(vx), w), __dmul_rn(__ll2double_rn(vy), w));
+    }
+  }
+}
+
+// Fetch the input lines line0 .. line0 + P - 1 of the six fields into L2.
+template <int P>
+__device__ __forceinline__ void fx_prefetch_lines(const XformArgs &a, size_t line0) {
+  const size_t nlines = (size_t)a.d.NY * a.d.NZ2, fstride = nlines * a.d.NXH;
+  const int nl = nlines - line0 < (size_t)P ? (int)(nlines - line0) : P;
+  const int per = (nl * a.d.NXH + 7) / 8;  // 128-byte lines per field
+  for (int idx = threadIdx.x; idx < 6 * per; idx += blockDim.x) {
+    const int f = idx / per, o = idx - f * per;
+    const double2 *src = reinterpret_cast<const double2 *>(a.zbuf) + (size_t)f * fstride + line0 * a.d.NXH + 8 * o;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(src));
+  }
+}
+
+// The groups g0, g0 + step, ... < ngroups; args(g, line0) gives the arguments
+// and first line of group g (several channels, all of one plan, in the batch).
+template <int CLS, class Args>
+__device__ __forceinline__ void xlamb_fx_run(int g0, int step, int ngroups, Args args) {
+  constexpr int P = FxCfg<CLS>::P;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  size_t line0;
+  const XformArgs &a0 = args(g0 < ngroups ? g0 : 0, line0);
+  const int A = a0.fpx.A, B = a0.fpx.B;
+  fxc *R = reinterpret_cast<fxc *>(smraw);
+  FxTw *tw = reinterpret_cast<FxTw *>(R + 3 * P * fx_xline(A, B));
+  const int ntw = fx_xtables(A, B);
+  FxBound *bd = reinterpret_cast<FxBound *>(tw + ntw);
+  FxScale *sc = reinterpret_cast<FxScale *>(bd + 3 * P * FxCfg<CLS>::T);
+  for (int k = threadIdx.x; k < ntw; k += blockDim.x) tw[k] = a0.fxx[k];
+  for (int g = g0; g < ngroups; g += step) {
+    __syncthreads();  // the last group's spectra are read (the first: the table is written)
+    const XformArgs &ag = args(g, line0);
+    if (g + step < ngroups) {
+      size_t nline0;
+      const XformArgs &an = args(g + step, nline0);
+      fx_prefetch_lines<P>(an, nline0);
+    }
+    xlamb_fx_group<CLS>(ag, line0, R, tw, bd, sc);
+  }
+}
+
+template <int CLS>
+__global__ void __launch_bounds__(FxCfg<CLS>::TX *FxCfg<CLS>::T, FxCfg<CLS>::ZB)
+    k_zback_fx(const __grid_constant__ XformArgs a) {
+  zback_fx_body<CLS>(a, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+template <int CLS>
+__global__ void __launch_bounds__(FxCfg<CLS>::TX *FxCfg<CLS>::T, FxCfg<CLS>::ZB)
+    k_zfwd_fx(const __grid_constant__ XformArgs a) {
+  zfwd_fx_body<CLS>(a, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+template <int CLS>
+__global__ void __launch_bounds__(3 * FxCfg<CLS>::P *FxCfg<CLS>::T, FxCfg<CLS>::XB)
+    k_xlamb_fx(const __grid_constant__ XformArgs a) {
+  constexpr int P = FxCfg<CLS>::P;
+  const int ngroups = (int)(((size_t)a.d.NY * a.d.NZ2 + P - 1) / P);
+  const XformArgs *pa = &a;
+  xlamb_fx_run<CLS>(blockIdx.x, gridDim.x, ngroups, [pa](int g, size_t &line0) -> const XformArgs & {
+    line0 = (size_t)g * P;
+    return *pa;
+  });
+}
+
+// Batched: as the kernels of transforms.cu, blocks numbered channel by channel.
+template <int CLS>
+__global__ void __launch_bounds__(FxCfg<CLS>::TX *FxCfg<CLS>::T, FxCfg<CLS>::ZB)
+    k_zback_fx_batch(const __grid_constant__ BatchTable<XformArgs> t) {
+  const int c = batch_channel(t.start, t.n, blockIdx.x);
+  const XformArgs &a = t.a[c];
+  const int gx = (a.d.NXH + FxCfg<CLS>::TX - 1) / FxCfg<CLS>::TX, lb = blockIdx.x - t.start[c], r = lb / gx;
+  zback_fx_body<CLS>(a, lb - r * gx, r % a.d.NY, r / a.d.NY);
+}
+template <int CLS>
+__global__ void __launch_bounds__(FxCfg<CLS>::TX *FxCfg<CLS>::T, FxCfg<CLS>::ZB)
+    k_zfwd_fx_batch(const __grid_constant__ BatchTable<XformArgs> t) {
+  const int c = batch_channel(t.start, t.n, blockIdx.x);
+  const XformArgs &a = t.a[c];
+  const int gx = (a.d.NXH + FxCfg<CLS>::TX - 1) / FxCfg<CLS>::TX, lb = blockIdx.x - t.start[c], r = lb / gx;
+  zfwd_fx_body<CLS>(a, lb - r * gx, r % a.d.NY, r / a.d.NY);
+}
+template <int CLS>
+__global__ void __launch_bounds__(3 * FxCfg<CLS>::P *FxCfg<CLS>::T, FxCfg<CLS>::XB)
+    k_xlamb_fx_batch(const __grid_constant__ BatchTable<XformArgs> t) {
+  xlamb_fx_run<CLS>(blockIdx.x, gridDim.x, t.start[t.n], [&](int g, size_t &line0) -> const XformArgs & {
+    const int c = batch_channel(t.start, t.n, g);
+    line0 = (size_t)(g - t.start[c]) * FxCfg<CLS>::P;
+    return t.a[c];
+  });
+}
+
+// The kernels of a class for z lines of NZ2 and x lines of NX2 points (each
+// used where the line's plan is of this class).
+template <int CLS>
+FxXformKernels fx_kernels_of_class(int L) {
+  const FxPlan p = fx_plan(L);
+  FxXformKernels k;
+  if (p.cls != CLS) return k;
+  k.ok = true;
+  k.zback = k_zback_fx<CLS>;
+  k.zfwd = k_zfwd_fx<CLS>;
+  k.xlamb = k_xlamb_fx<CLS>;
+  k.zback_b = k_zback_fx_batch<CLS>;
+  k.zfwd_b = k_zfwd_fx_batch<CLS>;
+  k.xlamb_b = k_xlamb_fx_batch<CLS>;
+  k.tx = FxCfg<CLS>::TX;
+  k.zthreads = FxCfg<CLS>::TX * p.T;
+  k.zsmem = fx_zsmem<CLS>(L);
+  k.xlines = FxCfg<CLS>::P;
+  k.xthreads = 3 * FxCfg<CLS>::P * p.T;
+  k.xsmem = fx_xsmem<CLS>(p.A, p.B);
+  return k;
+}
+
+}  // namespace owt
