@@ -28,6 +28,8 @@
 //               fill masks where the forward's masked solves apply.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "adjoint_kernels.h"
 #include "owt_device.cuh"
 #include "setup_host.h"
@@ -220,33 +222,61 @@ static size_t adj_smem_x(const XformDims &d) { return 2 * (size_t)ANPAIR * AP * 
 size_t adj_zbuf_values(const XformDims &d) { return 9 * (size_t)d.NY * d.NZ2 * d.NXH; }
 size_t adj_lbuf_values(const XformDims &d) { return 6 * (size_t)d.NY * d.NZ2 * d.NXH; }
 
-// the instances for the channel's line lengths
+// The instances for the channel's line lengths: fixed point where the length
+// has a plan, else the FP64 kernels above.
 struct AdjXformKernels {
   void (*zback)(AdjXformArgs), (*xlamb)(AdjXformArgs), (*zfwd)(AdjXformArgs);
+  int tx, xlines, zthreads, xthreads;
+  size_t zsmem, xsmem;
+  bool persistent;  // the x pass runs the resident blocks
 };
-static AdjXformKernels adj_kernels(const XformDims &d) {
+static FxAdjKernels fx_adj_kernels(int L) {
+  switch (fx_plan(L).cls) {
+    case 0: return fx_adj_kernels0(L);
+    case 1: return fx_adj_kernels1(L);
+    case 2: return fx_adj_kernels2(L);
+    default: return FxAdjKernels{};
+  }
+}
+static AdjXformKernels adj_kernels(const XformDims &d, bool stockham) {
   const bool z5 = d.NZ2 % 5 == 0, x5 = d.NX2 % 5 == 0;
-  return {z5 ? k_zback_adj<true> : k_zback_adj<false>, x5 ? k_xlamb_adj<true> : k_xlamb_adj<false>,
-          z5 ? k_zfwd_adj<true> : k_zfwd_adj<false>};
+  AdjXformKernels k{z5 ? k_zback_adj<true> : k_zback_adj<false>, x5 ? k_xlamb_adj<true> : k_xlamb_adj<false>,
+                    z5 ? k_zfwd_adj<true> : k_zfwd_adj<false>, ATX, AP, d.NZ2, d.NX2, adj_smem_z(d), adj_smem_x(d),
+                    false};
+  if (stockham) return k;
+  const FxAdjKernels fz = fx_adj_kernels(d.NZ2), fx = fx_adj_kernels(d.NX2);
+  if (fz.ok) {
+    k.zback = fz.zback; k.zfwd = fz.zfwd;
+    k.tx = fz.tx; k.zthreads = fz.zthreads; k.zsmem = fz.zsmem;
+  }
+  if (fx.ok) {
+    k.xlamb = fx.xlamb;
+    k.xlines = fx.xlines; k.xthreads = fx.xthreads; k.xsmem = fx.xsmem;
+    k.persistent = true;
+  }
+  return k;
 }
 
 cudaError_t adj_lamb_prepare(const XformDims &d) {
-  const AdjXformKernels k = adj_kernels(d);
-  cudaError_t e = raise_smem_limit(k.zback, adj_smem_z(d));
-  if (e == cudaSuccess) e = raise_smem_limit(k.zfwd, adj_smem_z(d));
-  if (e == cudaSuccess) e = raise_smem_limit(k.xlamb, adj_smem_x(d));
+  cudaError_t e = cudaSuccess;
+  for (int stockham = 0; stockham < 2 && e == cudaSuccess; ++stockham) {
+    const AdjXformKernels k = adj_kernels(d, stockham != 0);
+    e = raise_smem_limit(k.zback, k.zsmem);
+    if (e == cudaSuccess) e = raise_smem_limit(k.zfwd, k.zsmem);
+    if (e == cudaSuccess) e = raise_smem_limit(k.xlamb, k.xsmem);
+  }
   return e;
 }
 
 void launch_adj_lamb(const AdjXformArgs &a, cudaStream_t st) {
   const XformDims &d = a.d;
-  const AdjXformKernels k = adj_kernels(d);
-  dim3 gz((d.NXH + ATX - 1) / ATX, d.NY, 9);
-  k.zback<<<gz, d.NZ2, adj_smem_z(d), st>>>(a);
-  const size_t nl = (size_t)d.NY * d.NZ2;
-  k.xlamb<<<(unsigned)((nl + AP - 1) / AP), d.NX2, adj_smem_x(d), st>>>(a);
-  dim3 gf((d.NXH + ATX - 1) / ATX, d.NY, 6);
-  k.zfwd<<<gf, d.NZ2, adj_smem_z(d), st>>>(a);
+  const AdjXformKernels k = adj_kernels(d, a.stockham != 0);
+  const int gx = (d.NXH + k.tx - 1) / k.tx;
+  k.zback<<<dim3(gx, d.NY, 9), k.zthreads, k.zsmem, st>>>(a);
+  size_t grid = ((size_t)d.NY * d.NZ2 + k.xlines - 1) / k.xlines;
+  if (k.persistent) grid = std::min(grid, (size_t)resident_blocks(k.xlamb, k.xthreads, k.xsmem));
+  k.xlamb<<<(unsigned)grid, k.xthreads, k.xsmem, st>>>(a);
+  k.zfwd<<<dim3(gx, d.NY, 6), k.zthreads, k.zsmem, st>>>(a);
 }
 
 // ---------------------------------------------------------------------------

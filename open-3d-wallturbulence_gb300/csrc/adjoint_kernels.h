@@ -41,7 +41,23 @@ struct AdjXformArgs {
   FftPlan px, pz;
   const double2 *twx, *twz;
   double inv_n;           // 1 / (NX2 NZ2)
+  // fixed-point transforms: plans (class -1: none) and twiddles of the lines;
+  // stockham: the FP64 kernels even where there is a plan
+  FxPlan fpx, fpz;
+  const FxTw *fxx, *fxz;
+  int stockham;
 };
+// Kernels of the fixed-point form for line length L (adjoint_fix.cuh), by
+// class of the plan; ok = false where L has none.
+struct FxAdjKernels {
+  bool ok = false;
+  void (*zback)(AdjXformArgs) = nullptr, (*xlamb)(AdjXformArgs) = nullptr, (*zfwd)(AdjXformArgs) = nullptr;
+  int tx = 0, zthreads = 0, xthreads = 0, xlines = 0;
+  size_t zsmem = 0, xsmem = 0;
+};
+FxAdjKernels fx_adj_kernels0(int L);
+FxAdjKernels fx_adj_kernels1(int L);
+FxAdjKernels fx_adj_kernels2(int L);
 
 // Adjoint of solve_mean + solve_friction_force.
 struct AdjMeanArgs {

@@ -465,12 +465,29 @@ inline FxTw fx_tw_entry(int k, int L) {
 }
 // The twiddle table of a plan: w_L^(a b) at a B + b (a < A, b < B) for the
 // backward transforms, then at L + b A + a for the forward ones (pass-1 output
-// slowest, thread fastest in both).
+// slowest, thread fastest in both).  Angles beyond an eighth of the circle
+// (where 4 divides L) come by symmetry: cosl and sinl in 128 bits are software
+// on some hosts.
 inline std::vector<FxTw> fx_twiddles(const FxPlan &p) {
   const int L = p.A * p.B;
-  std::vector<FxTw> t((size_t)2 * L);
+  std::vector<FxTw> w((size_t)L), t((size_t)2 * L);
+  const int direct = L % 4 == 0 ? L / 8 : L % 2 == 0 ? L / 4 : L / 2;  // the others follow by symmetry
+  for (int k = 0; k <= direct; ++k) w[k] = fx_tw_entry(k, L);
+  auto entry = [&](auto &self, int k) -> FxTw {
+    if (k <= direct) return w[k];
+    if (2 * k > L) {
+      const FxTw e = self(self, L - k);
+      return FxTw{e.c1, e.c0, -e.s1, -e.s0};
+    }
+    if (4 * k > L) {
+      const FxTw e = self(self, L / 2 - k);
+      return FxTw{-e.c1, -e.c0, e.s1, e.s0};
+    }
+    const FxTw e = self(self, L / 4 - k);
+    return FxTw{e.s1, e.s0, e.c1, e.c0};
+  };
   for (int a = 0; a < p.A; ++a)
-    for (int b = 0; b < p.B; ++b) t[(size_t)a * p.B + b] = t[(size_t)L + (size_t)b * p.A + a] = fx_tw_entry(a * b, L);
+    for (int b = 0; b < p.B; ++b) t[(size_t)a * p.B + b] = t[(size_t)L + (size_t)b * p.A + a] = entry(entry, a * b);
   return t;
 }
 

@@ -97,6 +97,8 @@ void owt_handle::adjoint_step(const double2 *tp, double wgt) {
   xa.zbuf = adj.zbuf; xa.lbuf = adj.lbuf; xa.px = px; xa.pz = pz;
   xa.twx = static_cast<const double2 *>(twx[0]); xa.twz = static_cast<const double2 *>(twz[0]);
   xa.inv_n = 1.0 / ((double)NX2 * (double)NZ2);
+  xa.fpx = fx_plan(NX2); xa.fpz = fx_plan(NZ2); xa.fxx = fxx; xa.fxz = fxz;
+  xa.stockham = fft_stockham ? 1 : 0;
   launch_adj_lamb(xa, st);
 
   AdjMeanArgs ma{};
