@@ -383,19 +383,14 @@ int owt_drag_backward(owt_handle *h, double grad_objective, double *grad_bottom,
  *    (interleaved), line index fastest: [y][line] (a whole field in the
  *    library's device layout is nlines = NZ * NX/2).
  *  - Grid: y = tanh(alpha_mesh s)/tanh(alpha_mesh), NY points.
- *  - Scratch: a file-scope static device array of 256 KiB + 2 *
- *    OWT_NOALLOC_MAX_VALUES * 16 bytes (32.25 MiB), held on every GPU that
- *    loads the library until the process exits.  Requests beyond NY <=
- *    OWT_NOALLOC_MAX_NY or NY * nlines <= OWT_NOALLOC_MAX_VALUES are rejected
- *    with OWT_ERR_INVALID and a message in owt_last_error(NULL).
- *  - The first call on a device looks up that array's device address (once
- *    per device, with the device current) and keeps it; make that first call
- *    before any stream capture, and do not use the entry point across a
- *    cudaDeviceReset, which invalidates the kept address.
- *  - Every call rebuilds the operator tables it reads (then the scratch) for
- *    its own (NY, alpha_mesh) before using them; calls share the one array,
- *    so calls that can overlap on the GPU (different streams without
- *    ordering between them) race and give wrong results.
+ *  - Everything it needs lives in the shared memory of its blocks: no device
+ *    memory is held between calls, calls on different streams are
+ *    independent, and each call builds the operator for its own (NY,
+ *    alpha_mesh).  Requests beyond NY <= OWT_NOALLOC_MAX_NY or NY * nlines <=
+ *    OWT_NOALLOC_MAX_VALUES are rejected with OWT_ERR_INVALID and a message in
+ *    owt_last_error(NULL).
+ *  - d_out may be d_in (a block reads its lines before it writes them), but
+ *    must not overlap it otherwise.
  *  - Asynchronous on `stream` (a cudaStream_t, NULL for the legacy default
  *    stream); errors of the launch are returned, device-side ones appear at
  *    the caller's next synchronisation. */

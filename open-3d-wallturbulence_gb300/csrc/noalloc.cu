@@ -4,20 +4,28 @@
 // memory to their own pool allocator and forbid allocations from elsewhere,
 // and tight loops that cannot accept the implicit device-wide
 // synchronisation cudaMalloc and cudaFree bring.  owt_dy1_noalloc serves
-// them: it needs no handle (creating one allocates) and keeps its scratch in
-// a file-scope static __device__ array of fixed size.  That array is reserved
-// on every GPU that loads this library, for the life of the process.
+// them: it needs no handle (creating one allocates) and keeps everything in
+// the shared memory of its blocks.
 //
 // What it computes is the handle-based DY1 (owt_dy_apply with order 1):
 // out = diag(c11) A1^-1 B1 in along y, for every line, with the compact first
 // derivative of src/compdiff.hpp:11-69 and c11 = 1/(dy/ds) of
-// src/solver.cpp:77,94 on the grid y = tanh(alpha s)/tanh(alpha).  Each call
-// first rebuilds the A1 band factors, B1 rows and c11 for its (NY, alpha) in
-// the static array (one small kernel, noalloc_setup.h), then runs the
-// derivative kernel.
+// src/solver.cpp:77,94 on the grid y = tanh(alpha s)/tanh(alpha).
+//
+// One launch.  Each block builds the tables for (NY, alpha) itself
+// (noalloc_setup.h) and takes a tile of lines, all NY rows of which stay in
+// shared memory: B1 on the way in, the band solve in place, c11 on the way
+// out.  Bound by FP64 issue: a line component costs five FP64 operations a
+// row in the solve, which is sequential in y, and five in the two parallel
+// phases around it.  A tile is ceil(lines / SMs) lines, so that every SM
+// works on one, at most 64 (one thread per component) and what fits beside
+// the tables.  129 rows x 4096 lines: 633 us with one thread building the
+// tables in a kernel of its own and a scratch array in device memory, 106 us
+// now (the same bits).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <mutex>
 #include <string>
 
@@ -27,50 +35,96 @@
 
 namespace owt {
 
-// Layout of the static array: [setup region][bf: MAX values][yscr: MAX values]
-constexpr size_t NOALLOC_SETUP_BYTES = 256 * 1024;
-static_assert(noalloc_setup_bytes() <= NOALLOC_SETUP_BYTES, "setup tables exceed their region");
 static_assert(kNoallocMaxNY == OWT_NOALLOC_MAX_NY, "table layout and the entry point's limit disagree");
-constexpr size_t NOALLOC_SCRATCH_BYTES =
-    NOALLOC_SETUP_BYTES + 2 * (size_t)OWT_NOALLOC_MAX_VALUES * sizeof(double2);
 
-static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
+constexpr int kNoallocThreads = 128;
+constexpr size_t kNoallocSmem = 226 * 1024;
 
-// One thread builds the operator tables for (NY, alpha) in the array.
-__global__ void k_noalloc_setup(unsigned char *base, int NY, double alpha) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const NoallocSetup s = noalloc_layout(base);
-  noalloc_assemble(s, NY, alpha);
-  noalloc_factor(s, NY);
+// Shared memory: tables, then the tile [row][line][component].
+__host__ __device__ constexpr size_t noalloc_tables_bytes(int NY) { return (noalloc_setup_bytes(NY) + 15) / 16 * 16; }
+constexpr size_t noalloc_smem(int NY, int lines) {
+  return noalloc_tables_bytes(NY) + (size_t)NY * lines * sizeof(double2);
 }
+static_assert(noalloc_smem(kNoallocMaxNY, 1) <= kNoallocSmem, "the longest line does not fit");
 
-// One thread per line: bf = B1 f, band solve with A1, out = c11 * d.
-__global__ void __launch_bounds__(128) k_dy1_noalloc(unsigned char *base, int NY, int nlines,
-                                                     const double2 *__restrict__ in, double2 *__restrict__ out) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= nlines) return;
-  const NoallocSetup s = noalloc_layout(base);
-  double2 *bf = reinterpret_cast<double2 *>(base + NOALLOC_SETUP_BYTES);
-  double2 *yscr = bf + OWT_NOALLOC_MAX_VALUES;
-  const int M = nlines;
-  for (int j = 0; j < NY; ++j) {
+__global__ void __launch_bounds__(kNoallocThreads)
+    k_dy1_noalloc(int NY, int nlines, int tile, double alpha, const double2 *in, double2 *out) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ int state[2];
+  constexpr int KV = kNoallocKV;
+  constexpr uint8_t kWide = 0x80;  // in piv: U has entries beyond two rows up in this column
+  const NoallocSetup s = noalloc_layout(sm, NY);
+  double2 *T = reinterpret_cast<double2 *>(sm + noalloc_tables_bytes(NY));
+  const int t = threadIdx.x, line0 = blockIdx.x * tile;
+  const int nl = nlines - line0 < tile ? nlines - line0 : tile;
+  noalloc_assemble(s, NY, alpha, t, kNoallocThreads);
+  __syncthreads();
+  // B1 rows of the tile by all warps but the first, which factors A1 meanwhile
+  for (int e = t - 32; e >= 0 && e < NY * nl; e += kNoallocThreads - 32) {
+    const int j = e / nl, l = e - j * nl;
     double2 acc = make_double2(0.0, 0.0);
 #pragma unroll
-    for (int e = 0; e < 5; ++e) {
-      const double b = s.bval[j * 5 + e];
+    for (int q = 0; q < 4; ++q) {
+      const double b = s.bval[j * 5 + q];
+      const double2 f = in[(size_t)s.bcol[j * 5 + q] * nlines + line0 + l];
       if (b != 0.0) {
-        const double2 f = in[(size_t)s.bcol[j * 5 + e] * M + m];
         acc.x += b * f.x;
         acc.y += b * f.y;
       }
     }
-    bf[(size_t)j * M + m] = acc;
+    T[j * tile + l] = acc;
   }
-  auto rhs = [&](int p) -> double2 { return bf[(size_t)p * M + m]; };
-  auto ys = [&](int p, double2 y) { yscr[(size_t)p * M + m] = y; };
-  auto yl = [&](int p) -> double2 { return yscr[(size_t)p * M + m]; };
-  auto outf = [&](int c, double2 d) { out[(size_t)c * M + m] = make_double2(s.c11[c] * d.x, s.c11[c] * d.y); };
-  band_solve<2, 2>(s.ab, s.piv, NY, 1, 0, rhs, ys, yl, outf);
+  noalloc_factor_block(s, NY, t, kNoallocThreads, state, [] { __syncthreads(); });
+  for (int j = t; j < NY; j += kNoallocThreads)
+    if (s.ab[j] != 0.0 || s.ab[NY + j] != 0.0) s.piv[j] |= kWide;
+  __syncthreads();
+  // the band solve, one thread per line and component, in place
+  if (t < 2 * nl) {
+    double *x = reinterpret_cast<double *>(T) + t;
+    const int ld = 2 * tile;
+    {
+      double w0 = x[0], w1 = x[ld], w2 = x[2 * ld];
+#pragma unroll 4
+      for (int j = 0; j < NY; ++j) {
+        const int off = s.piv[j] & 3;
+        if (off == 1) {
+          const double q = w0; w0 = w1; w1 = q;
+        } else if (off == 2) {
+          const double q = w0; w0 = w2; w2 = q;
+        }
+        x[j * ld] = w0;
+        const double y = w0;
+        w0 = w1 - s.ab[(KV + 1) * NY + j] * y;
+        w1 = w2 - s.ab[(KV + 2) * NY + j] * y;
+        w2 = j + 3 < NY ? x[(j + 3) * ld] : 0.0;
+      }
+    }
+    {
+      auto at = [&](int j) { return j >= 0 ? x[j * ld] : 0.0; };
+      double w0 = x[(NY - 1) * ld], w1 = at(NY - 2), w2 = at(NY - 3), w3 = at(NY - 4), w4 = at(NY - 5);
+#pragma unroll 4
+      for (int j = NY - 1; j >= 0; --j) {
+        const double v = w0 * s.ab[KV * NY + j];
+        x[j * ld] = v;
+        w0 = w1 - s.ab[(KV - 1) * NY + j] * v;
+        w1 = w2 - s.ab[(KV - 2) * NY + j] * v;
+        w2 = w3;
+        w3 = w4;
+        if (s.piv[j] & kWide) {
+          w2 -= s.ab[NY + j] * v;
+          w3 -= s.ab[j] * v;
+        }
+        w4 = at(j - 5);
+      }
+    }
+  }
+  __syncthreads();
+  for (int e = t; e < NY * nl; e += kNoallocThreads) {
+    const int j = e / nl, l = e - j * nl;
+    const double c = s.c11[j];
+    const double2 d = T[j * tile + l];
+    out[(size_t)j * nlines + line0 + l] = make_double2(c * d.x, c * d.y);
+  }
 }
 
 }  // namespace owt
@@ -79,12 +133,10 @@ __global__ void __launch_bounds__(128) k_dy1_noalloc(unsigned char *base, int NY
 void owt_set_thread_error(const std::string &m);
 
 namespace {
-// Device address of the static array, looked up once per device on the first
-// call with that device current.  It belongs to the device's primary context:
-// after cudaDeviceReset it would be stale, so this entry point must not be
-// used across a device reset.
+// Per device: its SMs, and whether the kernel's shared-memory limit is raised
+// there (once per device, with that device current).
 std::mutex g_noalloc_mu;
-unsigned char *g_noalloc_ptr[256] = {nullptr};
+int g_noalloc_sms[256] = {0};
 }  // namespace
 
 extern "C" int owt_dy1_noalloc(int64_t NY, int64_t nlines, double alpha_mesh, const double *d_in, double *d_out,
@@ -105,23 +157,25 @@ extern "C" int owt_dy1_noalloc(int64_t NY, int64_t nlines, double alpha_mesh, co
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess || dev < 0 || dev >= 256) return fail(OWT_ERR_CUDA, std::string("cudaGetDevice: ") + cudaGetErrorString(e));
-  unsigned char *base = nullptr;
+  int sms = 0;
   {
-    // once per device, with that device current: the device address of the
-    // static array (its host-side name is only a stand-in)
     std::lock_guard<std::mutex> lk(g_noalloc_mu);
-    if (!g_noalloc_ptr[dev]) {
-      void *p = nullptr;
-      e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-      if (e != cudaSuccess) return fail(OWT_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
-      g_noalloc_ptr[dev] = static_cast<unsigned char *>(p);
+    if (!g_noalloc_sms[dev]) {
+      int n = 0;
+      e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_dy1_noalloc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNoallocSmem);
+      if (e != cudaSuccess) return fail(OWT_ERR_CUDA, std::string("kernel attributes: ") + cudaGetErrorString(e));
+      g_noalloc_sms[dev] = n > 0 ? n : 1;
     }
-    base = g_noalloc_ptr[dev];
+    sms = g_noalloc_sms[dev];
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  k_noalloc_setup<<<1, 32, 0, st>>>(base, (int)NY, alpha_mesh);
-  k_dy1_noalloc<<<(unsigned)((nlines + 127) / 128), 128, 0, st>>>(
-      base, (int)NY, (int)nlines, reinterpret_cast<const double2 *>(d_in), reinterpret_cast<double2 *>(d_out));
+  const int fits = (int)((kNoallocSmem - noalloc_tables_bytes((int)NY)) / ((size_t)NY * sizeof(double2)));
+  const int tile = (int)std::min<int64_t>({(nlines + sms - 1) / sms, fits, kNoallocThreads / 2});
+  k_dy1_noalloc<<<(unsigned)((nlines + tile - 1) / tile), kNoallocThreads, noalloc_smem((int)NY, tile), st>>>(
+      (int)NY, (int)nlines, tile, alpha_mesh, reinterpret_cast<const double2 *>(d_in),
+      reinterpret_cast<double2 *>(d_out));
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail(OWT_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
   return OWT_OK;
