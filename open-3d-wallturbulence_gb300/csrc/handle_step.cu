@@ -363,11 +363,29 @@ void owt_handle::to_device(const double *host, double2 *dst) {
   check_launch("layout transpose");
 }
 
+// The device address of a host array the kernels can read and write directly
+// (pinned or registered memory, 16-byte aligned), or null.
+static double2 *device_view(const double *p) {
+  if (reinterpret_cast<uintptr_t>(p) % 16 != 0) return nullptr;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
+  return static_cast<double2 *>(at.devicePointer);
+}
+
+// Pinned arrays are written by the transpose itself over the host link (a field
+// of 303 MB in 1.8 ms; through the staging buffer and a copy engine, which at
+// times ran at a tenth of the link's rate, 4 to 25 ms); others go through the
+// staging buffer.
 void owt_handle::to_host(const double2 *src, double *host) {
-  launch_transpose(src, stage, NY, M, st);  // [NY][M] -> [M][NY]
+  double2 *direct = device_view(host);
+  launch_transpose(src, direct ? direct : stage, NY, M, st);  // [NY][M] -> [M][NY]
   ++launches;
   check_launch("layout transpose");
-  ck(cudaMemcpyAsync(host, stage, fs * sizeof(double2), cudaMemcpyDeviceToHost, st), "D2H");
+  if (!direct) ck(cudaMemcpyAsync(host, stage, fs * sizeof(double2), cudaMemcpyDeviceToHost, st), "D2H");
   ck(cudaStreamSynchronize(st), "D2H");
 }
 
@@ -473,19 +491,6 @@ void owt_handle::host_step_prepare() {
   for (cudaEvent_t *e : {&hs.up_done, &hs.after_modes, &hs.down_done})
     ck(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "event");
   hs.ready = true;
-}
-
-// The device address of a host array the kernels can read directly (pinned
-// or registered memory, 16-byte aligned), or null.
-static const double2 *device_view(const double *p) {
-  if (reinterpret_cast<uintptr_t>(p) % 16 != 0) return nullptr;
-  cudaPointerAttributes at{};
-  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
-  return static_cast<const double2 *>(at.devicePointer);
 }
 
 // Uploads, by chunks of Fourier modes: the modes with |kz| in a range are
@@ -621,9 +626,11 @@ void owt_handle::step_host(const double *const *hist, const double *means, const
   double *outs[2] = {v_out, g_out};
   double2 *src[2] = {v_ring + (size_t)hn * fs, g_ring + (size_t)hn * fs};
   for (int b = 0; b < 2; ++b) {
-    launch_transpose(src[b], hs.dstage[b], NY, M, hs.down);  // [NY][M] -> [M][NY]
+    double2 *direct = device_view(outs[b]);
+    launch_transpose(src[b], direct ? direct : hs.dstage[b], NY, M, hs.down);  // [NY][M] -> [M][NY]
     ++launches;
-    ck(cudaMemcpyAsync(outs[b], hs.dstage[b], fs * sizeof(double2), cudaMemcpyDeviceToHost, hs.down), "D2H");
+    if (!direct)
+      ck(cudaMemcpyAsync(outs[b], hs.dstage[b], fs * sizeof(double2), cudaMemcpyDeviceToHost, hs.down), "D2H");
   }
   ck(cudaEventRecord(hs.down_done, hs.down), "downloads done");
   ck(cudaStreamWaitEvent(st, hs.down_done, 0), "downloads wait");
