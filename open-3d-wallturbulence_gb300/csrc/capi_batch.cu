@@ -94,8 +94,8 @@ struct owt_batch {
       const ModeBatchShape sh = modes_batch_shape(v);
       std::vector<int> blocks(hs.size(), 0);
       for (size_t i = 0; i < hs.size(); ++i) {
-        const long long threads = sh.quad ? 4LL * hs[i]->Uq : 2LL * hs[i]->M;
-        blocks[i] = (int)((threads + sh.block - 1) / sh.block);
+        const long long threads = sh.mapping == kMapQuad ? 4LL * hs[i]->Uq : 2LL * hs[i]->M;
+        blocks[i] = sh.mapping == kMapStream ? 2 * str_groups(hs[i]->Uq) : (int)((threads + sh.block - 1) / sh.block);
       }
       for (auto &t : make_tables(args, blocks, by_size(sparse == 1))) {
         const int total = t->start[t->n];
@@ -237,7 +237,7 @@ struct owt_batch {
       ck(cudaEventCreate(&e0), "event");
       ck(cudaEventCreate(&e1), "event");
       float best = 1e30f;
-      for (int v = 0; v < modes_batch_variant_count(); ++v) {
+      for (int v = 0; v < modes_variant_count(); ++v) {
         build_modes(v, true);
         launch_modes_all(st);  // warm-up
         ck(cudaEventRecord(e0, st), "event");
@@ -296,6 +296,7 @@ int owt_batch_create(owt_handle *const *handles, int count, owt_batch **out) {
         if (handles[r] == h) throw OwtError(OWT_ERR_INVALID, "a handle appears twice in the batch");
       ck(cudaStreamSynchronize(h->st), "batch");
       h->recompute_dirty_q();
+      if (h->sparse_v) h->build_streams();
       ck(cudaStreamSynchronize(h->st), "batch");
       b->hs.push_back(h);
     }

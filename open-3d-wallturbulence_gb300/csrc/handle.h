@@ -123,6 +123,12 @@ struct owt_handle {
   owt::BandDev bv, bg, b1, b2;
   int *rhs_node_v = nullptr, *rb_col = nullptr, *b1_col = nullptr, *b2_col = nullptr, *rbv_col = nullptr;
   double *rbv_val = nullptr;
+  int *vptr = nullptr, *gptr = nullptr;  // right-hand sides by last node (StrRow)
+  owt::StrRow *vrows = nullptr, *grows = nullptr;
+  // packed factor streams, built before the handle's first own step
+  owt::StrBuffers str;
+  int n_vrows = 0, n_grows = 0;
+  void build_streams();
   double *rb_val = nullptr, *b1_val = nullptr, *b2_val = nullptr;
   // scratch
   double2 *sg = nullptr, *dg = nullptr, *yv = nullptr, *yg = nullptr, *sv = nullptr;

@@ -202,6 +202,41 @@ void owt_handle::setup(const owt_params &prm) {
   }
   phase("pattern check");
   rhs_node_v = upload(tv.rhs_node, owned, st);
+  {
+    // the same right-hand sides row by row of a sweep over the nodes
+    auto sweep_rows = [&](const std::vector<int> &col, const std::vector<double> &val, int per, int n, auto has, int reach,
+                          int *&ptr, StrRow *&rows, int &count) {
+      std::vector<std::vector<StrRow>> at(NY);
+      for (int p = 0; p < n; ++p) {
+        if (!has(p)) continue;
+        StrRow r{};
+        r.p = p;
+        int last = 0;
+        for (int e = 0; e < per; ++e)
+          if (val[(size_t)p * per + e] != 0.0) last = std::max(last, col[(size_t)p * per + e]);
+        for (int e = 0; e < per; ++e) {
+          const double v = val[(size_t)p * per + e];
+          if (v == 0.0) continue;
+          const int back = last - col[(size_t)p * per + e];
+          if (back >= reach) throw OwtError(OWT_ERR_INVALID, "right-hand side row wider than its window");
+          r.w[4 - back] = v;
+        }
+        at[last].push_back(r);
+      }
+      std::vector<int> first(NY + 1, 0);
+      std::vector<StrRow> all;
+      for (int j = 0; j < NY; ++j) {
+        all.insert(all.end(), at[j].begin(), at[j].end());
+        first[j + 1] = (int)all.size();
+      }
+      ptr = upload(first, owned, st);
+      rows = upload(all, owned, st);
+      count = (int)all.size();
+    };
+    sweep_rows(tv.rbv_col, tv.rbv_val, 4, tv.n, [&](int p) { return tv.rhs_node[p] == kRhsTable; }, 3, vptr, vrows,
+               n_vrows);
+    sweep_rows(tg.rb_col, tg.rb_val, 5, tg.n, [](int) { return true; }, 5, gptr, grows, n_grows);
+  }
   rbv_col = upload(tv.rbv_col, owned, st);
   rbv_val = upload(tv.rbv_val, owned, st);
   rb_col = upload(tg.rb_col, owned, st);
@@ -252,8 +287,11 @@ void owt_handle::setup(const owt_params &prm) {
   hv_ring = dalloc<double2>(3 * fs, owned);
   hg_ring = dalloc<double2>(3 * fs, owned);
   q_ring = dalloc<double2>(3 * fs, owned);
-  for (double2 **f : {&u, &w, &ox, &oz, &lx, &ly, &lz, &sg, &dg, &sv, &bf, &yscr, &tmpA, &tmpB, &tmpC, &stage})
+  for (double2 **f : {&u, &w, &ox, &oz, &lx, &ly, &lz, &sv, &bf, &yscr, &tmpA, &tmpB, &tmpC, &stage})
     *f = dalloc<double2>(fs, owned);
+  // rows of mode-kernel scratch: the modes, or the lanes of the stream mapping's warps
+  const size_t row = std::max((size_t)M, str_scratch_values(Uq));
+  for (double2 **f : {&sg, &dg}) *f = dalloc<double2>((size_t)NY * row, owned);
   lm = dalloc<float2>(3 * fs, owned);
   {
     std::vector<double> wyh(NY, 0.0);
@@ -269,8 +307,8 @@ void owt_handle::setup(const owt_params &prm) {
     wy = upload(wyh, owned, st);
     ic_partial = dalloc<double>(ic_partial_values(), owned);
   }
-  yv = dalloc<double2>((size_t)bv.n * M, owned);
-  yg = dalloc<double2>((size_t)bg.n * M, owned);
+  yv = dalloc<double2>((size_t)bv.n * row, owned);
+  yg = dalloc<double2>((size_t)bg.n * row, owned);
   U_ring = dalloc<double2>(3 * (size_t)NY, owned);
   W_ring = dalloc<double2>(3 * (size_t)NY, owned);
   lxm_ring = dalloc<double2>(3 * (size_t)NY, owned);

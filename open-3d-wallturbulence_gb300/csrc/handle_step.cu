@@ -121,6 +121,8 @@ ModeArgs owt_handle::mode_args() const {
   a.rs_v = bv.rscale; a.rs_gi = rs_gi;
   a.sg = sg; a.dg = dg; a.yv = yv; a.yg = yg; a.sv = sv;
   a.rbv_col = rbv_col; a.rbv_val = rbv_val;
+  a.vf = str.vf; a.vb = str.vb; a.gf = str.gf; a.gb = str.gb; a.vrs = str.vrs; a.grs = str.grs;
+  a.vptr = vptr; a.gptr = gptr; a.vrows = vrows; a.grows = grows;
   a.c11h = c11h; a.c21h = c21h; a.c22h = c22h; a.nc21h = nc21h; a.nc22h = nc22h;
   a.step = d_step;
   a.vw = vw_on ? vw : nullptr;
@@ -175,8 +177,30 @@ void owt_handle::run_steps(int64_t n) {
   check_launch("time step");
 }
 
+// The factors of the stream mapping (a handle stepped only inside a batch never
+// needs them).
+void owt_handle::build_streams() {
+  if (str.vf || !(sparse_v || sparse_v6)) return;
+  const StrSizes z = str_sizes(bv.n, bg.n, sparse_v6);
+  const size_t g = (size_t)str_groups(Uq);
+  g_alloc_counter = &device_bytes;
+  struct Reset { ~Reset() { g_alloc_counter = nullptr; } } reset_counter;
+  StrBuffers b;
+  b.vf = dalloc<double>(z.vf * g, owned);
+  b.vb = dalloc<double>(z.vb * g, owned);
+  b.gf = dalloc<double>(z.gf * g, owned);
+  b.gb = dalloc<double>(z.gb * g, owned);
+  b.vrs = dalloc<double>((size_t)n_vrows * Uq, owned);
+  b.grs = dalloc<double>((size_t)n_grows * Uq, owned);
+  launch_str_pack(mode_args(), sparse_v6, b, n_vrows, n_grows, st);
+  launches += 4;
+  check_launch("factor streams");
+  str = b;
+}
+
 void owt_handle::ensure_tuned() {
   if (tuned) return;
+  build_streams();
   tuned = true;
   if (!initialized) {
     autotune_modes();

@@ -40,16 +40,9 @@ void modes_dense_launch(const ModeArgs &a, cudaStream_t st) {
   k_modes<kVKL, kVKU, 6, 6, false, false, 128, 3><<<(unsigned)((2 * (long long)a.M + bs - 1) / bs), bs, 0, st>>>(a);
 }
 
-// masked solve with the sixth-order fill (one variant: the sixth-order option
-// is not autotuned)
-void modes_sixth_launch(const ModeArgs &a, cudaStream_t st) {
-  const int bs = 128;
-  k_modes<kVKL, kVKU, 6, 6, true, false, 128, 3, VMasks6><<<(unsigned)((2 * (long long)a.M + bs - 1) / bs), bs, 0, st>>>(a);
-}
-
 ModeBatchShape modes_pair_batch_shape(int v) {
   const Variant &x = kVariants[v];
-  return {x.block, false, resident(x.batch, x.block)};
+  return {x.block, kMapPair, resident(x.batch, x.block)};
 }
 void modes_pair_batch_launch(int v, const BatchTable<ModeArgs> &t, int *work, int grid, cudaStream_t st) {
   const Variant &x = kVariants[v];
@@ -57,7 +50,7 @@ void modes_pair_batch_launch(int v, const BatchTable<ModeArgs> &t, int *work, in
 }
 
 ModeBatchShape modes_dense_batch_shape() {
-  return {128, false, resident(k_modes_batch<kVKL, kVKU, 6, 6, false, false, 128, 3>, 128)};
+  return {128, kMapPair, resident(k_modes_batch<kVKL, kVKU, 6, 6, false, false, 128, 3>, 128)};
 }
 void modes_dense_batch_launch(const BatchTable<ModeArgs> &t, int *work, int grid, cudaStream_t st) {
   k_modes_batch<kVKL, kVKU, 6, 6, false, false, 128, 3><<<grid, 128, 0, st>>>(t, work);

@@ -35,7 +35,7 @@ void modes_quad_launch(int v, const ModeArgs &a, cudaStream_t st) {
 
 ModeBatchShape modes_quad_batch_shape(int v) {
   const Variant &x = kVariants[v];
-  return {x.block, true, resident(x.batch, x.block)};
+  return {x.block, kMapQuad, resident(x.batch, x.block)};
 }
 void modes_quad_batch_launch(int v, const BatchTable<ModeArgs> &t, int *work, int grid, cudaStream_t st) {
   const Variant &x = kVariants[v];

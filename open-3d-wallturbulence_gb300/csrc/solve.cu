@@ -305,23 +305,16 @@ bool band_supported(int kl, int ku) {
   return (kl == kVKL && ku == kVKU) || (kl == 6 && ku == 6) || (kl == 2 && ku == 2);
 }
 
-// Mode-kernel variants live in modes_pair.cu and modes_quad.cu (separate
-// translation units so they compile in parallel); this dispatches by index.
-// Variants: the pair mapping's, then the quad mapping's, then those for
-// single-channel launches only (modes_split.cu; batches choose among the
-// first two families).
-int modes_variant_count() { return modes_pair_count() + modes_quad_count() + modes_split_count(); }
-int modes_batch_variant_count() { return modes_pair_count() + modes_quad_count(); }
-bool modes_variant_is_quad(int v) {
-  if (v < modes_pair_count()) return false;
-  v -= modes_pair_count();
-  return v < modes_quad_count() || modes_split_is_quad(v - modes_quad_count());
-}
+// Mode-kernel variants live in modes_pair.cu, modes_quad.cu and modes_stream.cu
+// (separate translation units so they compile in parallel); this dispatches by
+// index, in that order.
+int modes_variant_count() { return modes_pair_count() + modes_quad_count() + modes_stream_count(); }
+// variants whose launches can be limited to a range of unique modes
+bool modes_variant_is_quad(int v) { return v >= modes_pair_count(); }
 const char *modes_variant_name(int v) {
   if (v < modes_pair_count()) return modes_pair_name(v);
   v -= modes_pair_count();
-  if (v < modes_quad_count()) return modes_quad_name(v);
-  return modes_split_name(v - modes_quad_count());
+  return v < modes_quad_count() ? modes_quad_name(v) : modes_stream_name(v - modes_quad_count());
 }
 void launch_modes(const ModeArgs &a, int klv, int kuv, int klg, int kug, bool sparse, int variant, cudaStream_t st) {
   if (!(klv == kVKL && kuv == kVKU && klg == 6 && kug == 6)) return;
@@ -329,19 +322,23 @@ void launch_modes(const ModeArgs &a, int klv, int kuv, int klg, int kug, bool sp
   if (variant < modes_pair_count()) { modes_pair_launch(variant, a, st); return; }
   variant -= modes_pair_count();
   if (variant < modes_quad_count()) modes_quad_launch(variant, a, st);
-  else modes_split_launch(variant - modes_quad_count(), a, st);
+  else modes_stream_launch(variant - modes_quad_count(), a, false, st);
 }
 
 // Batched mode kernel: variant -1 is the full-band solve.
 ModeBatchShape modes_batch_shape(int variant) {
   if (variant < 0) return modes_dense_batch_shape();
   if (variant < modes_pair_count()) return modes_pair_batch_shape(variant);
-  return modes_quad_batch_shape(variant - modes_pair_count());
+  variant -= modes_pair_count();
+  if (variant < modes_quad_count()) return modes_quad_batch_shape(variant);
+  return modes_stream_batch_shape(variant - modes_quad_count());
 }
 void launch_modes_batch(const BatchTable<ModeArgs> &t, int variant, int *work, int grid, cudaStream_t st) {
-  if (variant < 0) modes_dense_batch_launch(t, work, grid, st);
-  else if (variant < modes_pair_count()) modes_pair_batch_launch(variant, t, work, grid, st);
-  else modes_quad_batch_launch(variant - modes_pair_count(), t, work, grid, st);
+  if (variant < 0) { modes_dense_batch_launch(t, work, grid, st); return; }
+  if (variant < modes_pair_count()) { modes_pair_batch_launch(variant, t, work, grid, st); return; }
+  variant -= modes_pair_count();
+  if (variant < modes_quad_count()) modes_quad_batch_launch(variant, t, work, grid, st);
+  else modes_stream_batch_launch(variant - modes_quad_count(), t, work, grid, st);
 }
 
 // Every factored system must keep its interior fill inside the masks of its
@@ -380,7 +377,7 @@ void launch_check_pattern(int which, const double *ab, const uint8_t *piv, int n
   else
     k_check_pattern<6, 6, 2, 0, GMasks><<<(U + 127) / 128, 128, 0, st>>>(ab, piv, n, U, bad);
 }
-void launch_modes_sixth(const ModeArgs &a, cudaStream_t st) { modes_sixth_launch(a, st); }
+void launch_modes_sixth(const ModeArgs &a, cudaStream_t st) { modes_stream_launch(0, a, true, st); }
 
 // dst[p U + u] = scale[u] src[p U + u] (setup: per-mode factors folded into
 // a [row][unique mode] table)

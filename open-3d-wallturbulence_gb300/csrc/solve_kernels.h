@@ -33,6 +33,13 @@ inline cudaError_t raise_smem_limit(F *func, size_t bytes) {
   return cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// A row of the mode systems' right-hand sides for a sweep over the nodes: row p
+// is the sum of w[i] r_(j-4+i) with j the last node it needs.
+struct StrRow {
+  int p;
+  double w[5];
+};
+
 struct ModeArgs {
   int NY, NZ, NXH, NZH, M, U;
   int u0, u1;  // quad mapping: unique modes u0 <= u < u1 only (0, U: all)
@@ -54,6 +61,12 @@ struct ModeArgs {
   // metric coefficients with the unscaling of the solved h d1, h^2 d2:
   // c11/h, c21/h, c22/h^2, nu c21/h, nu c22/h^2 [NY]
   const double *c11h, *c21h, *c22h, *nc21h, *nc22h;
+  // packed factor streams (modes_stream.cuh): v- and omega_y-system, forward
+  // and backward, and the rows whose last node is j at ptr[j] .. ptr[j + 1]
+  const double *vf, *vb, *gf, *gb;
+  const double *vrs, *grs;  // row scales in the order of vrows, grows [rows][U]
+  const int *vptr, *gptr;
+  const StrRow *vrows, *grows;
 };
 
 struct MeanArgs {
@@ -180,12 +193,23 @@ void launch_band_factor(int kl, int ku, double *ab, uint8_t *piv, int n, int U, 
                         const double *t2, const double *s1, const double *s2, double *rscale, int *info,
                         cudaStream_t st, int kernel = 0);
 void launch_modes(const ModeArgs &a, int klv, int kuv, int klg, int kug, bool sparse, int variant, cudaStream_t st);
+// Packed factor streams: doubles per group of 16 unique modes, groups, complex
+// values of a scratch row, and the packing of every group.
+struct StrSizes {
+  size_t vf, vb, gf, gb;
+};
+StrSizes str_sizes(int n_v, int n_g, bool sixth);
+int str_groups(int U);
+size_t str_scratch_values(int U);
+struct StrBuffers {
+  double *vf = nullptr, *vb = nullptr, *gf = nullptr, *gb = nullptr, *vrs = nullptr, *grs = nullptr;
+};
+void launch_str_pack(const ModeArgs &a, bool sixth, const StrBuffers &s, int nvrows, int ngrows, cudaStream_t st);
 int modes_pair_count();  // variants below this index use the pair mapping, the others the quad mapping
 void launch_modes_sixth(const ModeArgs &a, cudaStream_t st);  // masked solve with the sixth-order fill
 // dst[p U + u] = scale[u] src[p U + u], p < n
 void launch_scale_by_mode(double *dst, const double *src, const double *scale, int n, int U, cudaStream_t st);
-int modes_variant_count();        // single-channel launches: pair, quad, split mappings
-int modes_batch_variant_count();  // batched launches: pair and quad mappings
+int modes_variant_count();  // pair, quad and stream mappings
 bool modes_variant_is_quad(int v);
 const char *modes_variant_name(int v);
 void launch_check_pattern(int which, const double *ab, const uint8_t *piv, int n, int U, int *bad,
@@ -280,9 +304,10 @@ static_assert(sizeof(BatchTable<NLArgs>) <= 32764, "nonlinear batch table exceed
 // Mode kernel: work items of `block` threads, a persistent grid of resident
 // blocks taking items from the counter pair `work` (zero before the first
 // launch; each launch leaves it zero).  variant -1 is the full-band solve.
+enum ModeMapping { kMapPair, kMapQuad, kMapStream };  // 2 threads per mode, 4 per unique mode, streams
 struct ModeBatchShape {
   int block;  // threads per work item
-  bool quad;  // 4 threads per unique mode (else 2 per mode)
+  ModeMapping mapping;
   int grid;   // resident blocks on the device
 };
 ModeBatchShape modes_batch_shape(int variant);
