@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(128) k_adj_nl(AdjNLArgs a) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const double b = a.b1t_val[j * 8 + e];
-      if (b != 0.0) {
+      if (nonzero(b)) {
         const double2 x = a.ws[(size_t)a.b1t_col[j * 8 + e] * M + m];
         q.x += b * x.x;
         q.y += b * x.y;
@@ -332,7 +332,7 @@ __global__ void k_adj_mean(AdjMeanArgs a) {
     const double s = icg * a.rs_g[(size_t)p * a.U];
     for (int e = 0; e < 5; ++e) {
       const double b = a.rb_val[p * 5 + e];
-      if (b != 0.0) {
+      if (nonzero(b)) {
         double2 &d = sb[a.rb_col[p * 5 + e]];
         d.x += b * s * z.x;
         d.y += b * s * z.y;
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(64) k_adj_modes(AdjModeArgs a) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const double b = a.rbv_val[p * 4 + q];
-          if (b != 0.0) D(a.svb)[E(a.rbv_col[p * 4 + q])] += b * r;
+          if (nonzero(b)) D(a.svb)[E(a.rbv_col[p * 4 + q])] += b * r;
         }
       } else if (tag == kRhsWallBottom) {
         D(a.grad)[2 * (size_t)m + comp] += r;
@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(64) k_adj_modes(AdjModeArgs a) {
 #pragma unroll
       for (int e = 0; e < 5; ++e) {
         const double b = a.rb_val[p * 5 + e];
-        if (b != 0.0) D(a.sgb)[E(a.rb_col[p * 5 + e])] += b * r;
+        if (nonzero(b)) D(a.sgb)[E(a.rb_col[p * 5 + e])] += b * r;
       }
     };
     band_solve_t<KLG, KUG>(a.ab_g, a.piv_g, a.n_g, a.U, u, rhs, ys, yl, out);

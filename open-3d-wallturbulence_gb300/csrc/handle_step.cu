@@ -44,8 +44,7 @@ NLArgs owt_handle::nl_args(bool record_mean) const {
   a.kx = kx; a.kz = kz; a.c11 = c11;
   a.lx = lx; a.ly = ly; a.lz = lz;
   a.hv_ring = hv_ring; a.hg_ring = hg_ring;
-  a.ab1 = b1.ab; a.piv1 = b1.piv; a.b1_col = b1_col; a.b1_val = b1_val;
-  a.fscr = bf;
+  a.ab1 = b1.ab; a.piv1 = b1.piv; a.b1_val = b1_val;
   a.yscr = yscr;
   a.lx_mean = record_mean ? lxm_ring : nullptr;
   a.lz_mean = record_mean ? lzm_ring : nullptr;

@@ -442,7 +442,7 @@ __device__ __forceinline__ void str_g(const ModeArgs &a, const StrLane &L, int w
         double acc = 0.0;
 #pragma unroll
         for (int i = 0; i < 5; ++i)
-          if (i != 2 || w.w[2] != 0.0) acc = fma(w.w[i], r[i], acc);  // no centre tap in the first derivative's rows
+          if (i != 2 || nonzero(w.w[2])) acc = fma(w.w[i], r[i], acc);  // no centre tap in the first derivative's rows
         yg[32 * w.p] = __dmul_rn(acc, sc);
       }
     }

@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kNoallocThreads)
     for (int q = 0; q < 4; ++q) {
       const double b = s.bval[j * 5 + q];
       const double2 f = in[(size_t)s.bcol[j * 5 + q] * nlines + line0 + l];
-      if (b != 0.0) {
+      if (nonzero(b)) {
         acc.x += b * f.x;
         acc.y += b * f.y;
       }
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kNoallocThreads)
   }
   noalloc_factor_block(s, NY, t, kNoallocThreads, state, [] { __syncthreads(); });
   for (int j = t; j < NY; j += kNoallocThreads)
-    if (s.ab[j] != 0.0 || s.ab[NY + j] != 0.0) s.piv[j] |= kWide;
+    if (nonzero(s.ab[j]) || nonzero(s.ab[NY + j])) s.piv[j] |= kWide;
   __syncthreads();
   // the band solve, one thread per line and component, in place
   if (t < 2 * nl) {

@@ -12,6 +12,10 @@ namespace owt {
 // Ring slot of history level 0 at step counter s (level l is (head + l) mod 3).
 __device__ __forceinline__ int ring_head(long long s) { return (int)((2 * (s % 3)) % 3); }
 
+// x != 0 by its bits: a comparison of doubles is an FP64 instruction, and one
+// of those takes a warp 64 clocks.
+__device__ __forceinline__ bool nonzero(double x) { return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) != 0; }
+
 // ---------------------------------------------------------------------------
 // Complex values: double2 / float2 with the arithmetic the kernels need.
 // ---------------------------------------------------------------------------

@@ -558,73 +558,190 @@ void launch_mean_batch(const BatchTable<MeanArgs> &t, bool smem, size_t smem_byt
 // nonlinear_source (src/solver.cpp:240-260), one thread per real component of
 // a mode (lanes 2m, 2m+1 are Re, Im of mode m; A1 and B1 are real):
 //   Hg = i kz lx - i kx lz,   Hv = -k^2 ly - c11 A1^-1 B1 (i kx lx + i kz lz)
-// written to the level-0 slot.  Pass 1 forms this lane's component of
-// f = i kx lx + i kz lz once per row (scratch) and Hg; pass 2 applies B1 (at
-// most four taps per row, checked at setup) inside the right-hand side of the
-// A1 band solve and writes Hv from its output.  Component c of i z is
-// (2c - 1) times the other component of z.  The lane of component 0 of mode
-// (0, 0) also records the new mean Lamb vector (src/solver.cpp:296-302).
+// written to the level-0 slot.  One sweep up forms this lane's component of
+// f = i kx lx + i kz lz and Hg row by row, B1 f from the last five f, and the
+// forward elimination two rows behind; one sweep down solves and writes Hv.
+// Component c of i z is (2c - 1) times the other component of z.  The first
+// block also records the new mean Lamb vector (src/solver.cpp:296-302).
+//
+// Bound by FP64 issue (15 operations a node and component, 64 clocks each for
+// a warp) where the modes are few: the operator tables of one block are in
+// shared memory, and what a row reads from memory is fetched four rows ahead.
+// 384x257x384 1.28 -> 1.19 ms,
+// 128x129x128 0.334 -> 0.140, 32x65x32 0.105 -> 0.056 (before: f and B1 f through
+// memory, each row's reads where they are used).
+//
+// Rows of B1 (setup_host.cpp): columns 0..3 in row 0, 0 and 2 in row 1, i -+ 2
+// and i -+ 1 in between, and the mirror image at the top.
 // ---------------------------------------------------------------------------
+// threads a block: 64 spread a small channel (or a batch of them) over every SM,
+// 256 share one copy of the tables where the modes fill the GPU anyway
+constexpr int kNLThreads = 64, kNLThreadsLarge = 256;
+inline int nl_threads(const NLArgs &a) { return 2 * a.M >= 152 * 4 * kNLThreadsLarge ? kNLThreadsLarge : kNLThreads; }
+// per row: B1 entries (4), L (2), 1/U_jj, U above the diagonal (4), c11
+constexpr int kNLRow = 12;
+constexpr size_t nl_smem_bytes(int NY) { return (size_t)NY * (kNLRow * sizeof(double) + 1) + 8; }
+constexpr size_t kNLSmem = 220 * 1024;  // larger tables are read from device memory
+
+template <bool SMEM>
 __device__ __forceinline__ void nl_body(const NLArgs &a, const int tid) {
-  const int m = tid >> 1, comp = tid & 1;
-  if (m >= a.M) return;
   const int M = a.M, NY = a.NY;
-  const int k = m / a.NXH, i = m - k * a.NXH;
-  const double sgn = comp ? 1.0 : -1.0;
-  const double kx = a.kx[i], kz = a.kz[k];
-  const double skx = sgn * kx, skz = sgn * kz;
-  const double k2 = kx * kx + kz * kz;
-  const int h = ring_head(*a.step);
-  const size_t fs = (size_t)NY * M;
-  const double *lx = reinterpret_cast<const double *>(a.lx), *ly = reinterpret_cast<const double *>(a.ly);
-  const double *lz = reinterpret_cast<const double *>(a.lz);
-  double *hv = reinterpret_cast<double *>(a.hv_ring + (size_t)h * fs) + comp;
-  double *hg = reinterpret_cast<double *>(a.hg_ring + (size_t)h * fs) + comp;
-  double *f = reinterpret_cast<double *>(a.fscr) + comp;
-  double *y = reinterpret_cast<double *>(a.yscr) + comp;
-  auto E = [&](int j) { return 2 * ((size_t)j * M + m); };
-  const int oc = 1 - comp;
-  for (int j = 0; j < NY; ++j) {
-    const size_t e = E(j);
-    const double x = lx[e + oc], z = lz[e + oc];
-    f[e] = skx * x + skz * z;
-    hg[e] = skz * x - skx * z;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double *tab = reinterpret_cast<double *>(smraw);
+  uint8_t *spiv = reinterpret_cast<uint8_t *>(tab + (size_t)NY * kNLRow);
+  if (SMEM) {
+    for (int e = threadIdx.x; e < NY * kNLRow; e += blockDim.x) {
+      const int j = e / kNLRow, q = e - j * kNLRow;
+      // rows of the band storage (LAPACK layout, KV = 4): 5, 6 L; 4 .. 0 U
+      tab[e] = q < 4 ? a.b1_val[j * 5 + q] : q < 6 ? a.ab1[(size_t)(q + 1) * NY + j]
+               : q < 11 ? a.ab1[(size_t)(10 - q) * NY + j] : a.c11[j];
+    }
+    for (int j = threadIdx.x; j < NY; j += blockDim.x) spiv[j] = a.piv1[j];
+    __syncthreads();
   }
-  auto rhs = [&](int p) -> double {
-    double acc = 0.0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) acc += a.b1_val[p * 5 + q] * f[E(a.b1_col[p * 5 + q])];
-    return acc;
-  };
-  auto ys = [&](int p, double v) { y[E(p)] = v; };
-  auto yl = [&](int p) -> double { return y[E(p)]; };
-  auto out = [&](int c, double d) {
-    const size_t e = E(c);
-    hv[e] = -k2 * ly[e + comp] - a.c11[c] * d;
-  };
-  band_solve<2, 2>(a.ab1, a.piv1, NY, 1, 0, rhs, ys, yl, out);
-  if (m == 0 && comp == 0 && a.lx_mean) {
-    for (int j = 0; j < NY; ++j) {
+  auto b1 = [&](int j, int q) { return SMEM ? tab[j * kNLRow + q] : a.b1_val[j * 5 + q]; };
+  auto lo = [&](int j, int t) { return SMEM ? tab[j * kNLRow + 3 + t] : a.ab1[(size_t)(4 + t) * NY + j]; };
+  auto up = [&](int j, int t) { return SMEM ? tab[j * kNLRow + 6 + t] : a.ab1[(size_t)(4 - t) * NY + j]; };
+  auto c11 = [&](int j) { return SMEM ? tab[j * kNLRow + 11] : a.c11[j]; };
+  auto piv = [&](int j) { return SMEM ? (int)spiv[j] : (int)a.piv1[j]; };
+  const int h = ring_head(*a.step);
+  if (a.lx_mean && tid < (int)blockDim.x) {  // the channel's first block
+    for (int j = tid; j < NY; j += blockDim.x) {
       a.lx_mean[(size_t)h * NY + j] = a.lx[(size_t)j * M];
       a.lz_mean[(size_t)h * NY + j] = a.lz[(size_t)j * M];
     }
   }
+  const int m = tid >> 1, comp = tid & 1;
+  if (m >= M) return;
+  const int k = m / a.NXH, i = m - k * a.NXH;
+  const double sgn = comp ? 1.0 : -1.0;
+  const double kx = a.kx[i], kz = a.kz[k];
+  const double skx = sgn * kx, skz = sgn * kz;
+  const double k2 = fma(kx, kx, kz * kz);
+  const size_t fs = (size_t)NY * M, ld = 2 * (size_t)M;
+  const double *lx = reinterpret_cast<const double *>(a.lx) + 2 * (size_t)m + 1 - comp;
+  const double *lz = reinterpret_cast<const double *>(a.lz) + 2 * (size_t)m + 1 - comp;
+  const double *ly = reinterpret_cast<const double *>(a.ly) + tid;
+  double *hv = reinterpret_cast<double *>(a.hv_ring + (size_t)h * fs) + tid;
+  double *hg = reinterpret_cast<double *>(a.hg_ring + (size_t)h * fs) + tid;
+  double *y = reinterpret_cast<double *>(a.yscr) + tid;
+  const int n = NY - 1;
+  auto at = [&](int j) { return (size_t)(j < n ? (j > 0 ? j : 0) : n) * ld; };
+  // f of the last five rows, the newest last; the next four rows of lx, lz
+  double f[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, nx[4], nz[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    nx[q] = lx[at(q)];
+    nz[q] = lz[at(q)];
+  }
+  auto push = [&](int j) {
+    const double x = nx[0], z = nz[0];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      nx[q] = nx[q + 1];
+      nz[q] = nz[q + 1];
+    }
+    nx[3] = lx[at(j + 4)];
+    nz[3] = lz[at(j + 4)];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) f[q] = f[q + 1];
+    f[4] = fma(skx, x, __dmul_rn(skz, z));
+    hg[at(j)] = fma(skz, x, -__dmul_rn(skx, z));
+  };
+  auto inner = [&](int r) {  // row r of B1 f with f = f_(r-2) .. f_(r+2)
+    return fma(b1(r, 3), f[4], fma(b1(r, 2), f[3], fma(b1(r, 1), f[1], __dmul_rn(b1(r, 0), f[0]))));
+  };
+#pragma unroll
+  for (int j = 0; j < 5; ++j) push(j);
+  double w0 = fma(b1(0, 3), f[3], fma(b1(0, 2), f[2], fma(b1(0, 1), f[1], __dmul_rn(b1(0, 0), f[0]))));
+  double w1 = fma(b1(1, 1), f[2], __dmul_rn(b1(1, 0), f[0]));
+  double w2 = inner(2);
+  auto eliminate = [&](int c, double next) {
+    const int off = piv(c);
+    if (off == 1) {
+      const double q = w0; w0 = w1; w1 = q;
+    } else if (off == 2) {
+      const double q = w0; w0 = w2; w2 = q;
+    }
+    y[(size_t)c * ld] = w0;
+    const double v = w0;
+    w0 = fma(-lo(c, 1), v, w1);
+    w1 = fma(-lo(c, 2), v, w2);
+    w2 = next;
+  };
+#pragma unroll 4
+  for (int j = 5; j <= n; ++j) {
+    push(j);
+    eliminate(j - 5, inner(j - 2));
+  }
+  // columns n - 4 .. n; the rows still to come are n - 1 and n (f = f_(n-4) .. f_n)
+  eliminate(n - 4, fma(b1(n - 1, 1), f[4], __dmul_rn(b1(n - 1, 0), f[2])));
+  eliminate(n - 3, fma(b1(n, 3), f[4], fma(b1(n, 2), f[3], fma(b1(n, 1), f[2], __dmul_rn(b1(n, 0), f[1])))));
+  eliminate(n - 2, 0.0);
+  eliminate(n - 1, 0.0);
+  y[(size_t)n * ld] = w0;
+  // the next four rows of y beyond the window, and of ly
+  double u[5], ny[4], nl[4];
+#pragma unroll
+  for (int q = 0; q < 5; ++q) u[q] = y[at(n - q)];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    ny[q] = y[at(n - 5 - q)];
+    nl[q] = ly[at(n - q)];
+  }
+#pragma unroll 4
+  for (int c = n; c >= 0; --c) {
+    const double d = u[0] * up(c, 0);
+    hv[(size_t)c * ld] = fma(-c11(c), d, -__dmul_rn(k2, nl[0]));
+    u[0] = fma(-up(c, 1), d, u[1]);
+    u[1] = fma(-up(c, 2), d, u[2]);
+    u[2] = u[3];
+    u[3] = u[4];
+    const double u3 = up(c, 3), u4 = up(c, 4);
+    if (nonzero(u3) || nonzero(u4)) {  // only beside the row interchanges
+      u[2] = fma(-u3, d, u[2]);
+      u[3] = fma(-u4, d, u[3]);
+    }
+    u[4] = ny[0];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      ny[q] = ny[q + 1];
+      nl[q] = nl[q + 1];
+    }
+    ny[3] = y[at(c - 9)];
+    nl[3] = ly[at(c - 4)];
+  }
 }
 
-__global__ void __launch_bounds__(128) k_nl(const __grid_constant__ NLArgs a) {
-  nl_body(a, blockIdx.x * blockDim.x + threadIdx.x);
+template <bool SMEM>
+__global__ void __launch_bounds__(kNLThreadsLarge) k_nl(const __grid_constant__ NLArgs a) {
+  nl_body<SMEM>(a, blockIdx.x * blockDim.x + threadIdx.x);
 }
-__global__ void __launch_bounds__(128) k_nl_batch(const __grid_constant__ BatchTable<NLArgs> t) {
+template <bool SMEM>
+__global__ void __launch_bounds__(kNLThreads) k_nl_batch(const __grid_constant__ BatchTable<NLArgs> t) {
   const int c = batch_channel(t.start, t.n, blockIdx.x);
-  nl_body(t.a[c], (blockIdx.x - t.start[c]) * 128 + threadIdx.x);
+  nl_body<SMEM>(t.a[c], (blockIdx.x - t.start[c]) * kNLThreads + threadIdx.x);
 }
 
-void launch_nl(const NLArgs &a, cudaStream_t st) {
-  const int bs = 128, gs = (2 * a.M + bs - 1) / bs;
-  k_nl<<<gs, bs, 0, st>>>(a);
+cudaError_t nl_prepare(int NY) {
+  const size_t b = nl_smem_bytes(NY);
+  if (b > kNLSmem) return cudaSuccess;
+  const cudaError_t e = raise_smem_limit(k_nl<true>, b);
+  return e == cudaSuccess ? raise_smem_limit(k_nl_batch<true>, b) : e;
 }
-int nl_batch_blocks(const NLArgs &a) { return (2 * a.M + 127) / 128; }
-void launch_nl_batch(const BatchTable<NLArgs> &t, cudaStream_t st) { k_nl_batch<<<t.start[t.n], 128, 0, st>>>(t); }
+void launch_nl(const NLArgs &a, cudaStream_t st) {
+  const int bs = nl_threads(a), gs = (2 * a.M + bs - 1) / bs;
+  const size_t b = nl_smem_bytes(a.NY);
+  if (b <= kNLSmem) k_nl<true><<<gs, bs, b, st>>>(a);
+  else k_nl<false><<<gs, bs, 0, st>>>(a);
+}
+int nl_batch_blocks(const NLArgs &a) { return (2 * a.M + kNLThreads - 1) / kNLThreads; }
+void launch_nl_batch(const BatchTable<NLArgs> &t, cudaStream_t st) {
+  size_t b = 0;
+  for (int c = 0; c < t.n; ++c) b = std::max(b, nl_smem_bytes(t.a[c].NY));
+  if (b <= kNLSmem) k_nl_batch<true><<<t.start[t.n], kNLThreads, b, st>>>(t);
+  else k_nl_batch<false><<<t.start[t.n], kNLThreads, 0, st>>>(t);
+}
 
 // ---------------------------------------------------------------------------
 // d = A_n^-1 B_n f along y for every mode (raw compact derivative on the
@@ -640,7 +757,7 @@ __global__ void __launch_bounds__(128) k_dapply(DApplyArgs a) {
 #pragma unroll
     for (int e = 0; e < 5; ++e) {
       const double b = a.b_val[j * 5 + e];
-      if (b != 0.0) {
+      if (nonzero(b)) {
         const double2 f = a.in[(size_t)a.b_col[j * 5 + e] * M + m];
         acc.x += b * f.x;
         acc.y += b * f.y;
@@ -683,7 +800,7 @@ __global__ void __launch_bounds__(128) k_dy2(DY2Args a) {
 #pragma unroll
     for (int e = 0; e < 5; ++e) {
       const double b = bv[p * 5 + e];
-      if (b != 0.0) acc += b * in[E(bc[p * 5 + e])];
+      if (nonzero(b)) acc += b * in[E(bc[p * 5 + e])];
     }
     return acc;
   };

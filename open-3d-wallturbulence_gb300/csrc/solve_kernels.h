@@ -93,8 +93,8 @@ struct NLArgs {
   const double2 *lx, *ly, *lz;
   double2 *hv_ring, *hg_ring;
   const double *ab1; const uint8_t *piv1;
-  const int *b1_col; const double *b1_val;
-  double2 *fscr, *yscr;        // B1 operand and forward-sweep scratch [NY][M] each
+  const double *b1_val;
+  double2 *yscr;               // forward-sweep scratch [NY][M]
   double2 *lx_mean, *lz_mean;  // rings [3][NY], or null
   const long long *step;
 };
@@ -317,6 +317,7 @@ size_t mean_smem_bytes(int NY, int n_g);
 void launch_mean_batch(const BatchTable<MeanArgs> &t, bool smem, size_t smem_bytes, cudaStream_t st);
 void launch_advance_batch(const StepCounters &c, cudaStream_t st);
 int nl_batch_blocks(const NLArgs &a);
+cudaError_t nl_prepare(int NY);  // its shared memory, before any launch or capture
 void launch_nl_batch(const BatchTable<NLArgs> &t, cudaStream_t st);
 // Transforms: part 0 z backward, 1 x pass, 2 z forward, 3 mean-flow terms
 // (mixed precision).  The channels of a table share the precision, NZ2 (parts
