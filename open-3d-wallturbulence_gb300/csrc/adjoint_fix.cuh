@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(5 * FxAdjCfg<CLS>::P *FxCfg<CLS>::T, FxAdjCfg<
       fx_x_pass1<CLS, true>(
           p, t < B, q, t,
           [&](auto upper, int s) {
-            return fx_hermitian<decltype(upper)::value>(Af, fstride, have, s, d.NXH, d.NX2, pair < 4);
+            return fx_bits(fx_hermitian<decltype(upper)::value>(Af, fstride, have, s, d.NXH, d.NX2, pair < 4));
           },
           R + q * LS, tw, bd, sc);
     }
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(5 * FxAdjCfg<CLS>::P *FxCfg<CLS>::T, FxAdjCfg<
     __syncthreads();
     // 3. forward transforms
     fx_x_pass1<CLS, false>(
-        p, q < NF && t < A, q, t, [&](auto, int s) { return D[q * LS + s]; }, R + (NF + (q < NF ? q : 0)) * LS,
+        p, q < NF && t < A, q, t, [&](auto, int s) { return fx_bits(D[q * LS + s]); }, R + (NF + (q < NF ? q : 0)) * LS,
         A == B ? tw : tw + A * B, bd, sc);
     __syncthreads();
     if (q < NF && t < B) fx_x_pass2_fwd<CLS>(p, t, R + (NF + q) * LS, R + q * LS);

@@ -351,12 +351,13 @@ OWT_HD long long fx_from_bits(long long bits, const FxScale &s) {
   return (v ^ sg) - sg;
 }
 
-// 2^k for |k| <= 1022
+// 2^k; 0 or infinity beyond the normal range
 OWT_HD double fx_pow2(int k) {
+  const int f = k < -1022 ? 0 : k > 1023 ? 0x7ff : k + 1023;
 #ifdef __CUDA_ARCH__
-  return __hiloint2double((k + 1023) << 20, 0);
+  return __hiloint2double(f << 20, 0);
 #else
-  const long long b = (long long)(k + 1023) << 52;
+  const long long b = (long long)f << 52;
   double d;
   __builtin_memcpy(&d, &b, 8);
   return d;
@@ -381,6 +382,83 @@ __device__ __forceinline__ double fx_to_double(long long n, FxOut o) {
   return __hiloint2double((int)((unsigned)(hi ? hi + o.dhi : 0) | o.nan), __double2loint(d));
 }
 #endif
+
+// ---------------------------------------------------------------------------
+// Products of two lines in physical space and the transform back, all in
+// integers.  A line's integers after a transform are 2^k x with k = e - 2 and
+// at most 61 bits; the product of u and o (of lines with k_u, k_o) is
+// fx_product(u << 1, o << 2) = u o 2^-61, rounded, 2^(k_u + k_o - 61) times the
+// real product.
+// ---------------------------------------------------------------------------
+OWT_HD long long fx_product(int ah, int al, int bh, int bl) {  // words of fx_split
+  const long long cr = fx_wide(al, bh) + (fx_wide(ah, bl) + 0x80000000ll);
+  return fx_wide(ah, bh) + (cr >> 32);
+}
+OWT_HD long long fx_shift_right(long long x, int d) {  // rounded, 0 <= d <= 62
+  return (x + ((1ll << d) >> 1)) >> d;
+}
+// k of a line after its transform; a line of zeros does not limit the scale
+// of the products it enters.
+OWT_HD int fx_k(const FxScale &s) { return s.rsh == 4096 ? 1 << 14 : s.e - 2; }
+// Right shifts of the six products of a (y, z) line for k of the (u, v),
+// (w, ox) and (oy, oz) lines, and the scales of (lx, ly) and of lz.
+struct FxProducts {
+  int s02, s12, s11;  // lx = v oz - w oy, ly = w ox - u oz
+  int z02, z01;       // lz = u oy - v ox
+  int kxy, kz;
+};
+OWT_HD int fx_min(int a, int b) { return a < b ? a : b; }
+// kz_other: the lz scale of the line that shares lz's transform
+OWT_HD int fx_kz(int k0, int k1, int k2) { return fx_min(k0 + k2, k0 + k1) - 61; }
+OWT_HD FxProducts fx_products(int k0, int k1, int k2, int kz_other) {
+  FxProducts p;
+  const int c02 = k0 + k2, c12 = k1 + k2, c11 = 2 * k1, c01 = k0 + k1;
+  const int c = fx_min(c02, fx_min(c12, c11)), z = fx_min(fx_min(c02, c01), kz_other + 61);
+  p.s02 = fx_min(c02 - c, 62);
+  p.s12 = fx_min(c12 - c, 62);
+  p.s11 = fx_min(c11 - c, 62);
+  p.z02 = fx_min(c02 - z, 62);
+  p.z01 = fx_min(c01 - z, 62);
+  p.kxy = c - 61;
+  p.kz = z - 61;
+  return p;
+}
+// Bound of a thread's integers (below 2^62) in units of 2^38.
+template <int N>
+OWT_HD unsigned fx_bound_int(const fxc *x) {
+  unsigned s = 0;
+  auto add = [&](long long v) {
+    const int hi = fx_hi(v);
+    s += ((unsigned)(hi ^ (hi >> 31)) >> 6) + 1u;
+  };
+  fx_for<0, N>([&](auto c) {
+    add(x[decltype(c)::value].x);
+    add(x[decltype(c)::value].y);
+  });
+  return s;
+}
+// The line's scale for integers that are 2^k x, and the shift that gives it.
+template <class B>
+OWT_HD FxScale fx_scale_int(int n, B b, int k, bool finite, int &shift) {
+  unsigned s = 0, s1 = 0;
+  for (int t = 0; t < n; ++t) {
+    const unsigned v = b(t);
+    s += (v >> 5) + 1u;
+    s1 = s1 > v ? s1 : v;
+  }
+#ifdef __CUDA_ARCH__
+  const int lgs = 32 - __clz((int)s), lg1 = 32 - __clz((int)s1);
+#else
+  const int lgs = 32 - __builtin_clz(s), lg1 = 32 - __builtin_clz(s1);
+#endif
+  shift = fx_min(23 - lg1, 20 - lgs);
+  FxScale r;
+  r.rsh = 0;
+  r.e = k + shift;
+  r.finite = finite;
+  return r;
+}
+OWT_HD long long fx_rescale(long long x, int left, int right) { return fx_shift_right(x, right) << left; }
 
 // ---------------------------------------------------------------------------
 // Lengths.  L = A B with A and B from the radices below, A a multiple of 3

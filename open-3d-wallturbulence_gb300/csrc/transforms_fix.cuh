@@ -1,10 +1,10 @@
 // Transform kernels of the FP64 step with 64-bit fixed-point line transforms
 // (fft_fix.cuh): the three kernels, data layouts and dealiasing of
-// transforms.cu (src/FFT.cpp:49-194, src/solver.cpp:262-304), FP64 in memory
-// and in the physical-space products, for the line lengths with a plan
-// (fx_plan).  One translation unit per plan class instantiates them
-// (transforms_fix0.cu, ...), so that the register budget of a kernel is that
-// of its largest radix and the units compile in parallel.
+// transforms.cu (src/FFT.cpp:49-194, src/solver.cpp:262-304), FP64 in memory,
+// for the line lengths with a plan (fx_plan).  One translation unit per plan
+// class instantiates them (transforms_fix0.cu, ...), so that the register
+// budget of a kernel is that of its largest radix and the units compile in
+// parallel.
 //
 // A line of A B points has T = max(A, B) threads; every thread of a block
 // takes part in every barrier, those beyond the number of a pass's transforms
@@ -14,20 +14,22 @@
 //               thread index so that rows of kx coalesce; the padded z line
 //               is gathered straight into pass-1 registers.
 //  k_xlamb_fx : persistent; per group of P (y, z) lines: 3P packed backward
-//               lines, products in FP64 in shared memory, 3P/2 packed
+//               lines, products in shared memory (integers too), 3P/2 packed
 //               forward lines, the real-pair unpack; the next group's input
 //               is prefetched into L2.
 //  k_zfwd_fx  : as k_zback_fx, forward.
 //
 // Measured at 384x257x384 (lines of 576 points), FP64 kernels -> these:
-// z backward 10.74 -> 1.64 ms, x pass 27.99 -> 7.85 ms, z forward
-// 5.27 -> 0.95 ms; at 128x129x128 0.496 -> 0.095, 1.189 -> 0.470 and
+// z backward 10.74 -> 1.65 ms, x pass 27.99 -> 7.21 ms, z forward
+// 5.27 -> 0.96 ms; at 128x129x128 0.496 -> 0.095, 1.189 -> 0.388 and
 // 0.255 -> 0.061 ms.  The z passes are bound by integer issue at half of the
-// DRAM rate.  The x pass is latency bound (1.3 instructions a clock, the FP64
-// pipe of the conversions and products 43% busy, 15 warps an SM): its 24-point
-// transforms fit 128 registers with 90 bytes of spills, so that three blocks
-// are resident (two at 168 registers: 12.2 ms, before the zero thirds were
-// left out).
+// DRAM rate, the x pass by latency (about 1.4 instructions a clock whatever the
+// number of resident blocks; a fifth of the stalls are its barriers, an eighth
+// instruction fetch).  In the x pass FP64 products of converted values took
+// 7.85 and 0.42 ms: a conversion is an FP64 instruction, and the FP64 pipe was
+// 43% busy.  Block shapes were measured over the classes (three blocks an SM
+// instead of two for the x pass of class 2: 12.2 -> 7.9 ms with the zero thirds
+// left out; z blocks of 4 or 16 columns 5 to 25% slower).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -41,7 +43,7 @@ namespace owt {
 // Block shapes by plan class: kx columns per z block, (y, z) lines per x
 // group, and the resident blocks asked of the register allocator.
 template <int CLS> struct FxCfg;
-template <> struct FxCfg<0> { static constexpr int T = 12, TX = 8, P = 4, ZB = 6, XB = 4; };
+template <> struct FxCfg<0> { static constexpr int T = 12, TX = 8, P = 4, ZB = 8, XB = 5; };
 template <> struct FxCfg<1> { static constexpr int T = 18, TX = 8, P = 2, ZB = 3, XB = 4; };
 template <> struct FxCfg<2> { static constexpr int T = 24, TX = 8, P = 2, ZB = 2, XB = 3; };
 
@@ -56,13 +58,15 @@ __device__ __forceinline__ FxTw fx_ldg(const FxTw *p) {
 
 // The rest of pass 1 once the line's scale is known: x (doubles' bits) to
 // integers, N-point transform, output r times twiddle(r) to store(r, value).
-template <int N, bool BACKWARD, class Twiddle, class Store>
+// INT: x are integers of that scale already.
+template <int N, bool BACKWARD, bool INT, class Twiddle, class Store>
 __device__ __forceinline__ void fx_line_pass1(fxc *x, const FxScale &s, Twiddle twiddle, Store store) {
-  fx_for<0, N>([&](auto rc) {
-    constexpr int r = decltype(rc)::value;
-    if constexpr (!BACKWARD || N % 3 != 0 || r < N / 3 || r >= 2 * N / 3)
-      x[r] = fxc{fx_from_bits(x[r].x, s), fx_from_bits(x[r].y, s)};
-  });
+  if constexpr (!INT)
+    fx_for<0, N>([&](auto rc) {
+      constexpr int r = decltype(rc)::value;
+      if constexpr (!BACKWARD || N % 3 != 0 || r < N / 3 || r >= 2 * N / 3)
+        x[r] = fxc{fx_from_bits(x[r].x, s), fx_from_bits(x[r].y, s)};
+    });
   fx_dft<N, BACKWARD>(x);
   store(0, fx_quarter(x[0]));
   fx_for<1, N>([&](auto rc) {
@@ -107,7 +111,7 @@ __device__ __forceinline__ void fx_z_lines(const FxPlan p, const FxTw *__restric
     if (t < N2) {
       const FxScale s = fx_scale(N2, [&](int k) { return bd[k * TX + c]; });
       if (t == 0) sc[c] = s;
-      fx_line_pass1<N, BACKWARD>(x, s, [&](int r) { return fx_ldg(tw + r * N2 + t); },
+      fx_line_pass1<N, BACKWARD, false>(x, s, [&](int r) { return fx_ldg(tw + r * N2 + t); },
                                  [&](int r, fxc v) { S[(r * N2 + t) * TX + c] = v; });
     }
   });
@@ -202,10 +206,11 @@ constexpr size_t fx_xsmem(int A, int B) {
 
 // Pass 1 of line q's transform on input in(r, s) (s = t + N2 r), its
 // transposes to R[r RS + t] of its line; the line's scale to sc[q].  act: the
-// thread has a transform in this pass.  All threads call it.
-template <int CLS, bool BACKWARD, class In>
+// thread has a transform in this pass.  All threads call it.  INT: the input
+// is the integers of products, at the scale and finiteness pk, ok of the line.
+template <int CLS, bool BACKWARD, bool INT = false, class In>
 __device__ __forceinline__ void fx_x_pass1(const FxPlan p, bool act, int q, int t, In in, fxc *R, const FxTw *tw,
-                                           FxBound *bd, FxScale *sc) {
+                                           FxBound *bd, FxScale *sc, int pk = 0, bool ok = true) {
   const int N1 = BACKWARD ? p.A : p.B, N2 = BACKWARD ? p.B : p.A, RS = fx_row(N2);
   bd += q * p.T;
   fx_radix<CLS>(N1, [&](auto n) {
@@ -218,22 +223,35 @@ __device__ __forceinline__ void fx_x_pass1(const FxPlan p, bool act, int q, int 
       fx_for<0, N>([&](auto rc) {
         constexpr int r = decltype(rc)::value;
         if constexpr (!BACKWARD || N % 3 != 0 || r < N / 3 || r >= 2 * N / 3)
-          x[r] = fx_bits(in(std::integral_constant<bool, (r >= 2 * N / 3)>{}, t + N2 * r));
+          x[r] = in(std::integral_constant<bool, (r >= 2 * N / 3)>{}, t + N2 * r);
       });
-      bd[t] = fx_bound<N>(x);
+      if constexpr (INT) bd[t].s = fx_bound_int<N>(x);
+      else bd[t] = fx_bound<N>(x);
     }
     __syncthreads();
     if (act) {
-      const FxScale s = fx_scale(N2, [&](int k) { return bd[k]; });
+      FxScale s;
+      if constexpr (INT) {
+        int shift;
+        s = fx_scale_int(N2, [&](int k) { return bd[k].s; }, pk, ok, shift);
+        const int left = max(shift, 0), right = max(-shift, 0);
+        fx_for<0, N>([&](auto rc) {
+          fxc &v = x[decltype(rc)::value];
+          v = fxc{fx_rescale(v.x, left, right), fx_rescale(v.y, left, right)};
+        });
+      } else {
+        s = fx_scale(N2, [&](int k) { return bd[k]; });
+      }
       if (t == 0) sc[q] = s;
-      fx_line_pass1<N, BACKWARD>(x, s, [&](int r) { return tw[r * N2 + t]; },
-                                 [&](int r, fxc v) { R[r * RS + t] = v; });
+      fx_line_pass1<N, BACKWARD, INT>(x, s, [&](int r) { return tw[r * N2 + t]; },
+                                      [&](int r, fxc v) { R[r * RS + t] = v; });
     }
   });
 }
 
-// Backward pass 2 of line q: point t + A r as FP64, in place (R: the line).
-template <int CLS>
+// Backward pass 2 of line q: point t + A r, in place (R: the line), as FP64 or
+// (INT) as integers of scale fx_k(*sc).
+template <int CLS, bool INT = false>
 __device__ __forceinline__ void fx_x_pass2_back(const FxPlan p, bool act, int t, fxc *R, const FxScale *sc) {
   const int A = p.A;
   fx_radix<CLS>(p.B, [&](auto n) {
@@ -245,7 +263,10 @@ __device__ __forceinline__ void fx_x_pass2_back(const FxPlan p, bool act, int t,
       fx_dft<N, true>(y);
     }
     __syncthreads();
-    if (act) {
+    if (!act) return;
+    if constexpr (INT) {
+      fx_for<0, N>([&](auto rc) { R[t + A * decltype(rc)::value] = y[decltype(rc)::value]; });
+    } else {
       const FxOut o = fx_out(*sc);
       double2 *D = reinterpret_cast<double2 *>(R);
       fx_for<0, N>([&](auto rc) {
@@ -289,45 +310,76 @@ __device__ __forceinline__ void xlamb_fx_group(const XformArgs &a, const size_t 
     const double2 *Af = reinterpret_cast<const double2 *>(a.zbuf) + (size_t)(2 * pair) * fstride + (line0 + l) * d.NXH;
     fx_x_pass1<CLS, true>(
         p, t < B, q, t,
-        [&](auto upper, int s) { return fx_hermitian<decltype(upper)::value>(Af, fstride, have, s, d.NXH, d.NX2); },
+        [&](auto upper, int s) {
+          return fx_bits(fx_hermitian<decltype(upper)::value>(Af, fstride, have, s, d.NXH, d.NX2));
+        },
         R + q * LS, tw, bd, sc);
   }
   __syncthreads();
   // 2. backward pass 2
-  fx_x_pass2_back<CLS>(p, t < A, t, R + q * LS, sc + q);
+  fx_x_pass2_back<CLS, true>(p, t < A, t, R + q * LS, sc + q);
   __syncthreads();
-  // 3. lamb = u x omega (no fused multiply-add, as the reference's separate
-  // products), packed as (lx + i ly) in line l and (lz_l + i lz_l+1) in line
-  // P + l/2, in place: one thread owns point xx of every line
-  double2 *D = reinterpret_cast<double2 *>(R);
-  for (int xx = threadIdx.x; xx < A * B; xx += blockDim.x) {
-    double2 uv[P], wox[P], oyz[P];
-#pragma unroll
-    for (int l = 0; l < P; ++l) {
-      uv[l] = D[(0 * P + l) * LS + xx];
-      wox[l] = D[(1 * P + l) * LS + xx];
-      oyz[l] = D[(2 * P + l) * LS + xx];
-    }
+  // 3. lamb = u x omega in integers, packed as (lx + i ly) in line l and
+  // (lz_l + i lz_l+1) in line P + l/2, in place: one thread owns point xx of
+  // every line
+  int pk = 0;
+  bool ok = true;
+  {
+    FxProducts pr[P];
 #pragma unroll
     for (int l = 0; l < P; l += 2) {
-      double lz[2];
+      int k[2][3];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const double u = uv[l + h].x, v = uv[l + h].y, w = wox[l + h].x, ox = wox[l + h].y, oy = oyz[l + h].x,
-                     oz = oyz[l + h].y;
-        const double lx = __dsub_rn(__dmul_rn(v, oz), __dmul_rn(w, oy));
-        const double ly = __dsub_rn(__dmul_rn(w, ox), __dmul_rn(u, oz));
-        lz[h] = __dsub_rn(__dmul_rn(u, oy), __dmul_rn(v, ox));
-        D[(l + h) * LS + xx] = make_double2(lx, ly);
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) k[h][i] = fx_k(sc[i * P + l + h]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) pr[l + h] = fx_products(k[h][0], k[h][1], k[h][2], fx_kz(k[1 - h][0], k[1 - h][1], k[1 - h][2]));
+    }
+    // scale and finiteness of this thread's forward line
+#pragma unroll
+    for (int l = 0; l < P; ++l) {
+      const bool f = sc[l].finite && sc[P + l].finite && sc[2 * P + l].finite;
+      if (q == l) {
+        pk = pr[l].kxy;
+        ok = f;
       }
-      D[(P + l / 2) * LS + xx] = make_double2(lz[0], lz[1]);
+      if (q == P + l / 2) {
+        pk = pr[l].kz;
+        ok = ok && f;
+      }
+    }
+    for (int xx = threadIdx.x; xx < A * B; xx += blockDim.x) {
+#pragma unroll
+      for (int l = 0; l < P; l += 2) {
+        long long lz[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const fxc uv = R[(l + h) * LS + xx], wox = R[(P + l + h) * LS + xx], oyz = R[(2 * P + l + h) * LS + xx];
+          const FxProducts &c = pr[l + h];
+          int uh, ul, vh, vl, wh, wl, xh, xl, yh, yl, zh, zl;
+          fx_split(uv.x << 1, uh, ul);
+          fx_split(uv.y << 1, vh, vl);
+          fx_split(wox.x << 1, wh, wl);
+          fx_split(wox.y << 2, xh, xl);
+          fx_split(oyz.x << 2, yh, yl);
+          fx_split(oyz.y << 2, zh, zl);
+          const long long lx = fx_shift_right(fx_product(vh, vl, zh, zl), c.s02) -
+                               fx_shift_right(fx_product(wh, wl, yh, yl), c.s12);
+          const long long ly = fx_shift_right(fx_product(wh, wl, xh, xl), c.s11) -
+                               fx_shift_right(fx_product(uh, ul, zh, zl), c.s02);
+          lz[h] = fx_shift_right(fx_product(uh, ul, yh, yl), c.z02) - fx_shift_right(fx_product(vh, vl, xh, xl), c.z01);
+          R[(l + h) * LS + xx] = fxc{lx, ly};
+        }
+        R[(P + l / 2) * LS + xx] = fxc{lz[0], lz[1]};
+      }
     }
   }
   __syncthreads();
   // 4. forward pass 1 of the NF product lines, transposes into lines NF + q
-  fx_x_pass1<CLS, false>(
-      p, q < NF && t < A, q, t, [&](auto, int s) { return D[q * LS + s]; }, R + (NF + q) * LS,
-      A == B ? tw : tw + A * B, bd, sc);
+  fx_x_pass1<CLS, false, true>(
+      p, q < NF && t < A, q, t, [&](auto, int s) { return R[q * LS + s]; }, R + (NF + q) * LS,
+      A == B ? tw : tw + A * B, bd, sc, pk, ok);
   __syncthreads();
   // 5. forward pass 2 into line q
   if (q < NF && t < B) fx_x_pass2_fwd<CLS>(p, t, R + (NF + q) * LS, R + q * LS);

@@ -2,7 +2,9 @@
 // length with a plan, both signs, four kinds of lines, against a direct
 // transform in long double.  The relative L2 error must not exceed that of a
 // mixed-radix FP64 transform (radices 4, 2, 3, 5, correctly rounded twiddles)
-// on the same lines.  Then the ends of the range: scaled lines give the same
+// on the same lines.  The products of six lines and their transform back are
+// held to the same bound against FP64 products of FP64 transforms.  Then the
+// ends of the range: scaled lines give the same
 // digits, zero and tiny lines zeros, lines with an infinity, a NaN or a
 // magnitude from 2^1009 NaN.
 #include <cmath>
@@ -20,54 +22,73 @@ using cd = std::complex<double>;
 using cl = std::complex<long double>;
 static const long double kTwoPi = 2.0L * 3.14159265358979323846264338327950288L;
 
-template <int CLS, bool BACKWARD>
-static void line_of_class(const FxPlan p, const std::vector<cd> &in, std::vector<cd> &out) {
-  const int A = BACKWARD ? p.A : p.B, B = BACKWARD ? p.B : p.A, L = A * B;
+// One line's transform on load(point), as a block's threads run it; INT: the
+// input is integers 2^k x.
+template <bool BACKWARD, bool INT, class Load>
+static FxScale transform(int L, Load load, int k, std::vector<fxc> &out) {
+  const FxPlan p = fx_plan(L);
+  const int A = BACKWARD ? p.A : p.B, B = BACKWARD ? p.B : p.A;
   std::vector<FxBound> bd(B);
   std::vector<fxc> S(L);
-  auto load = [&](int b, int a) {
-    fxc v;
-    const double re = in[b + B * a].real(), im = in[b + B * a].imag();
-    std::memcpy(&v.x, &re, 8);
-    std::memcpy(&v.y, &im, 8);
-    return v;
-  };
+  out.resize(L);
   FxScale sc{};
-  for (int pass = 0; pass < 2; ++pass) {
-    if (pass == 1) sc = fx_scale(B, [&](int t) { return bd[t]; });
-    for (int b = 0; b < B; ++b)
-      fx_radix<CLS>(A, [&](auto n) {
+  int shift = 0;
+  auto run = [&](auto cls) {
+    constexpr int CLS = decltype(cls)::value;
+    for (int pass = 0; pass < 2; ++pass) {
+      if (pass == 1) {
+        if (INT) sc = fx_scale_int(B, [&](int t) { return bd[t].s; }, k, true, shift);
+        else sc = fx_scale(B, [&](int t) { return bd[t]; });
+      }
+      for (int b = 0; b < B; ++b)
+        fx_radix<CLS>(A, [&](auto n) {
+          constexpr int N = decltype(n)::value;
+          fxc x[N];
+          for (int a = 0; a < N; ++a) x[a] = load(b + B * a);
+          if (pass == 0) {
+            if (INT) bd[b].s = fx_bound_int<N>(x);
+            else bd[b] = fx_bound<N>(x);
+            return;
+          }
+          const int left = std::max(shift, 0), right = std::max(-shift, 0);
+          for (int a = 0; a < N; ++a)
+            x[a] = INT ? fxc{fx_rescale(x[a].x, left, right), fx_rescale(x[a].y, left, right)}
+                       : fxc{fx_from_bits(x[a].x, sc), fx_from_bits(x[a].y, sc)};
+          fx_dft<N, BACKWARD>(x);
+          S[b] = fx_quarter(x[0]);
+          for (int a = 1; a < N; ++a) S[a * B + b] = fx_twiddle<BACKWARD>(x[a], fx_tw_entry(a * b, L));
+        });
+    }
+    for (int a = 0; a < A; ++a)
+      fx_radix<CLS>(B, [&](auto n) {
         constexpr int N = decltype(n)::value;
-        fxc x[N];
-        for (int a = 0; a < N; ++a) x[a] = load(b, a);
-        if (pass == 0) {
-          bd[b] = fx_bound<N>(x);
-          return;
-        }
-        for (int a = 0; a < N; ++a) x[a] = fxc{fx_from_bits(x[a].x, sc), fx_from_bits(x[a].y, sc)};
-        fx_dft<N, BACKWARD>(x);
-        S[b] = fx_quarter(x[0]);
-        for (int a = 1; a < N; ++a) S[a * B + b] = fx_twiddle<BACKWARD>(x[a], fx_tw_entry(a * b, L));
+        fxc y[N];
+        for (int b = 0; b < N; ++b) y[b] = S[a * B + b];
+        fx_dft<N, BACKWARD>(y);
+        for (int b = 0; b < N; ++b) out[a + A * b] = y[b];
       });
-  }
-  const double f = fx_factor(sc);
-  for (int a = 0; a < A; ++a)
-    fx_radix<CLS>(B, [&](auto n) {
-      constexpr int N = decltype(n)::value;
-      fxc y[N];
-      for (int b = 0; b < N; ++b) y[b] = S[a * B + b];
-      fx_dft<N, BACKWARD>(y);
-      for (int b = 0; b < N; ++b) out[a + A * b] = cd((double)y[b].x * f, (double)y[b].y * f);
-    });
+  };
+  if (p.cls == 0) run(std::integral_constant<int, 0>{});
+  else if (p.cls == 1) run(std::integral_constant<int, 1>{});
+  else run(std::integral_constant<int, 2>{});
+  return sc;
+}
+
+static fxc bits(cd z) {
+  fxc v;
+  const double re = z.real(), im = z.imag();
+  std::memcpy(&v.x, &re, 8);
+  std::memcpy(&v.y, &im, 8);
+  return v;
 }
 
 template <bool BACKWARD>
 static void fix_line(const std::vector<cd> &in, std::vector<cd> &out) {
-  const FxPlan p = fx_plan((int)in.size());
+  std::vector<fxc> n;
+  const FxScale sc = transform<BACKWARD, false>((int)in.size(), [&](int i) { return bits(in[i]); }, 0, n);
+  const double f = fx_factor(sc);
   out.resize(in.size());
-  if (p.cls == 0) line_of_class<0, BACKWARD>(p, in, out);
-  else if (p.cls == 1) line_of_class<1, BACKWARD>(p, in, out);
-  else line_of_class<2, BACKWARD>(p, in, out);
+  for (size_t i = 0; i < in.size(); ++i) out[i] = cd((double)n[i].x * f, (double)n[i].y * f);
 }
 
 static std::vector<cl> g_w;  // exp(2 pi i k / L)
@@ -113,6 +134,91 @@ static void fp64_line(const cd *x, int n, int stride, cd *o, int sign, int L) {
       o[k + 3 * m] = a2 - b2;
     }
   }
+}
+
+// The Lamb vector's line: six real lines from their spectra (two per complex
+// transform), u x omega, two products per transform back, against long double.
+// Returns the largest error over that of the same in FP64.
+static double product_ratio(int L, const double amp[6], double decay, double mean, std::mt19937_64 &gen) {
+  std::normal_distribution<double> nd;
+  const int H = L / 3;
+  long double ef[3] = {}, ed[3] = {};
+  for (int rep = 0; rep < 4; ++rep) {
+    std::vector<std::vector<cd>> f(6, std::vector<cd>(H));
+    for (int i = 0; i < 6; ++i)
+      for (int k = 0; k < H; ++k) {
+        f[i][k] = amp[i] * std::pow(1.0 + k, -decay) * cd(nd(gen), nd(gen));
+        if (k == 0) f[i][k] = f[i][k].real();
+      }
+    f[0][0] += mean;
+    std::vector<std::vector<long double>> ph(6, std::vector<long double>(L));
+    for (int i = 0; i < 6; ++i)
+      for (int x = 0; x < L; ++x) {
+        cl v = f[i][0].real();
+        for (int k = 1; k < H; ++k) v += 2.0L * std::real(cl(f[i][k]) * g_w[(size_t)k * x % L]);
+        ph[i][x] = v.real();
+      }
+    std::vector<fxc> n[3];
+    std::vector<cd> d[3];
+    FxScale sc[3];
+    for (int q = 0; q < 3; ++q) {
+      std::vector<cd> z(L);
+      for (int m = 0; m < L; ++m) {
+        cd a, b;
+        if (m < H) a = f[2 * q][m], b = f[2 * q + 1][m];
+        else if (m > L - H) a = std::conj(f[2 * q][L - m]), b = std::conj(f[2 * q + 1][L - m]);
+        z[m] = a + cd(0, 1) * b;
+      }
+      sc[q] = transform<true, false>(L, [&](int i) { return bits(z[i]); }, 0, n[q]);
+      d[q].resize(L);
+      fp64_line(z.data(), L, 1, d[q].data(), 1, L);
+    }
+    const FxProducts c = fx_products(fx_k(sc[0]), fx_k(sc[1]), fx_k(sc[2]), 1 << 20);
+    std::vector<fxc> p01(L), p2(L);
+    std::vector<cd> d01(L), d2(L);
+    for (int x = 0; x < L; ++x) {
+      const long long v[6] = {n[0][x].x << 1, n[0][x].y << 1, n[1][x].x << 1, n[1][x].y << 2, n[2][x].x << 2, n[2][x].y << 2};
+      int h[6], l[6];
+      for (int i = 0; i < 6; ++i) fx_split(v[i], h[i], l[i]);
+      auto mul = [&](int i, int j, int s) { return fx_shift_right(fx_product(h[i], l[i], h[j], l[j]), s); };
+      p01[x] = fxc{mul(1, 5, c.s02) - mul(2, 4, c.s12), mul(2, 3, c.s11) - mul(0, 5, c.s02)};
+      p2[x] = fxc{mul(0, 4, c.z02) - mul(1, 3, c.z01), 0};
+      const double u = d[0][x].real(), w1 = d[0][x].imag(), w = d[1][x].real(), ox = d[1][x].imag(), oy = d[2][x].real(),
+                   oz = d[2][x].imag();
+      const volatile double t[6] = {w1 * oz, w * oy, w * ox, u * oz, u * oy, w1 * ox};
+      d01[x] = cd(t[0] - t[1], t[2] - t[3]);
+      d2[x] = t[4] - t[5];
+    }
+    std::vector<fxc> o01, o2;
+    const double f01 = fx_factor(transform<false, true>(L, [&](int i) { return p01[i]; }, c.kxy, o01));
+    const double f2 = fx_factor(transform<false, true>(L, [&](int i) { return p2[i]; }, c.kz, o2));
+    std::vector<cd> q01(L), q2(L);
+    fp64_line(d01.data(), L, 1, q01.data(), -1, L);
+    fp64_line(d2.data(), L, 1, q2.data(), -1, L);
+    for (int m = 0; m < H; ++m)
+      for (int r = 0; r < 3; ++r) {
+        cl s = 0;
+        for (int x = 0; x < L; ++x) {
+          const long double lam = r == 0   ? ph[1][x] * ph[5][x] - ph[2][x] * ph[4][x]
+                                  : r == 1 ? ph[2][x] * ph[3][x] - ph[0][x] * ph[5][x]
+                                           : ph[0][x] * ph[4][x] - ph[1][x] * ph[3][x];
+          s += lam * std::conj(g_w[(size_t)m * x % L]);
+        }
+        const int mc = m ? L - m : 0;
+        const fxc zm = r < 2 ? o01[m] : o2[m], zc = r < 2 ? o01[mc] : o2[mc];
+        const cd qm = r < 2 ? q01[m] : q2[m], qc = r < 2 ? q01[mc] : q2[mc];
+        const double w = 0.5 * (r < 2 ? f01 : f2);
+        const cd a = r == 1 ? cd((double)(zm.y + zc.y) * w, (double)(zc.x - zm.x) * w)
+                            : cd((double)(zm.x + zc.x) * w, (double)(zm.y - zc.y) * w);
+        const cd b = r == 1 ? cd((qm.imag() + qc.imag()) * 0.5, (qc.real() - qm.real()) * 0.5)
+                            : cd((qm.real() + qc.real()) * 0.5, (qm.imag() - qc.imag()) * 0.5);
+        ef[r] += std::norm(cl(a) - s);
+        ed[r] += std::norm(cl(b) - s);
+      }
+  }
+  double worst = 0.0;
+  for (int r = 0; r < 3; ++r) worst = std::max(worst, (double)std::sqrt(ef[r] / ed[r]));
+  return worst;
 }
 
 int main() {
@@ -179,5 +285,16 @@ int main() {
     }
   }
   std::printf("%d lengths, largest error %.2f times that of FP64, %d failures\n", lengths, worst, bad);
+  // white fields; a channel's core (mean flow, vorticity 20 times the velocity
+  // fluctuations), two decays; next to the wall (shear, v and w small)
+  const double one[6] = {1, 1, 1, 1, 1, 1}, core[6] = {0.1, 0.05, 0.05, 2, 2, 2}, wall[6] = {0.1, 0.001, 1e-5, 50, 50, 80};
+  for (int L : {48, 192, 480, 576}) {
+    g_w.resize(L);
+    for (int k = 0; k < L; ++k) g_w[k] = cl(std::cos(kTwoPi * k / L), std::sin(kTwoPi * k / L));
+    const double r[4] = {product_ratio(L, one, 0.0, 0.0, gen), product_ratio(L, core, 1.0, 1.3, gen),
+                         product_ratio(L, core, 2.0, 1.3, gen), product_ratio(L, wall, 1.0, 1.3, gen)};
+    std::printf("products on lines of %d: error %.2f %.2f %.2f %.2f times that of FP64\n", L, r[0], r[1], r[2], r[3]);
+    for (double x : r) bad += !(x <= 1.0);
+  }
   return bad || lengths != 38 ? 1 : 0;
 }
