@@ -237,9 +237,9 @@ int owt_get_grid(const owt_handle *h, double *y) {
 int owt_statistics(owt_handle *h, double *out7ny) {
   return guard(h, [&] {
     if (!out7ny) throw OwtError(OWT_ERR_INVALID, "null buffer");
-    double *d = reinterpret_cast<double *>(h->tmpA);  // 7 NY doubles fit easily
+    double *d = reinterpret_cast<double *>(h->tmpA);  // stats_values() <= 2 NY M doubles
     launch_stats(h->u, h->ring_level(h->v_ring, 0), h->w, h->NY, h->NZ, h->NXH, d, h->st);
-    ++h->launches;
+    h->launches += 2;
     h->check_launch("statistics");
     ck(cudaMemcpyAsync(out7ny, d, 7 * (size_t)h->NY * sizeof(double), cudaMemcpyDeviceToHost, h->st), "D2H");
     h->sync_and_check();

@@ -893,56 +893,88 @@ void launch_lamb_mean_shift(double2 *lx_ring, double2 *lz_ring, const double2 *l
   k_lamb_mean_shift<<<1, 256, 0, st>>>(lx_ring, lz_ring, lx, lz, NY, M, step);
 }
 
-// Wall-normal statistics by Parseval, one block per y plane, fixed reduction
-// order (deterministic).  Physical field f = sum_{kx>0} 2 Re(f_k e^{..}) +
+// Wall-normal statistics by Parseval, in a fixed order of summation
+// (deterministic).  Physical field f = sum_{kx>0} 2 Re(f_k e^{..}) +
 // Re(sum_kz f(0,kz) e^{..}) with the Nyquist kz row dropped, so the x-z mean of
 // f g is sum_{kx>0} 2 Re(f conj g) + sum_kz Re(Hf conj Hg) over the kx = 0
 // column's Hermitian parts Hf(kz) = (f(kz) + conj f(-kz))/2.
-__global__ void k_stats(const double2 *u, const double2 *v, const double2 *w, int NY, int NZ, int NXH, double *out) {
-  const int j = blockIdx.x;
+//
+// Block (part, y) sums a part of plane y's modes, k_stats_final adds the parts.
+// Bound by FP64 issue: eight multiply-adds a mode (the weight 2 of kx > 0 once
+// per block instead of per mode).  The parts give every SM at least four
+// blocks: one block a plane and weights per mode took 94 us at 192x129x192,
+// this 59 (141 and 100 us a call with the read-back).
+constexpr int kStatsThreads = 256;
+int stats_parts(int NY, int M) {
+  return std::max(1, std::min((4 * 152 + NY - 1) / NY, M / (2 * kStatsThreads)));
+}
+__global__ void __launch_bounds__(kStatsThreads)
+    k_stats(const double2 *u, const double2 *v, const double2 *w, int NY, int NZ, int NXH, double *partial) {
+  const int part = blockIdx.x, parts = gridDim.x, j = blockIdx.y, t = threadIdx.x;
   const int M = NZ * NXH, NZH = NZ / 2;
   const double2 *pu = u + (size_t)j * M, *pv = v + (size_t)j * M, *pw = w + (size_t)j * M;
   double acc[4] = {0.0, 0.0, 0.0, 0.0};  // uu, vv, ww, uv
-  for (int m = threadIdx.x; m < M; m += blockDim.x) {
-    const int k = m / NXH, i = m - k * NXH;
-    if (k == NZH) continue;
-    double2 a = pu[m], b = pv[m], c = pw[m];
-    double wgt = 2.0;
-    if (i == 0) {
-      const int kp = (k == 0) ? 0 : NZ - k;
-      const double2 ap = pu[(size_t)kp * NXH], bp = pv[(size_t)kp * NXH], cp = pw[(size_t)kp * NXH];
-      a = make_double2(0.5 * (a.x + ap.x), 0.5 * (a.y - ap.y));
-      b = make_double2(0.5 * (b.x + bp.x), 0.5 * (b.y - bp.y));
-      c = make_double2(0.5 * (c.x + cp.x), 0.5 * (c.y - cp.y));
-      wgt = 1.0;
+  auto add = [&](double2 a, double2 b, double2 c) {
+    acc[0] = fma(a.x, a.x, fma(a.y, a.y, acc[0]));
+    acc[1] = fma(b.x, b.x, fma(b.y, b.y, acc[1]));
+    acc[2] = fma(c.x, c.x, fma(c.y, c.y, acc[2]));
+    acc[3] = fma(a.x, b.x, fma(a.y, b.y, acc[3]));
+  };
+  const int m1 = (int)((long long)M * (part + 1) / parts);
+#pragma unroll 4
+  for (int m = (int)((long long)M * part / parts) + t; m < m1; m += kStatsThreads) {
+    const int k = m / NXH;
+    if (k == NZH || m == k * NXH) continue;
+    add(pu[m], pv[m], pw[m]);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) acc[q] *= 2.0;
+  if (part == 0) {  // the kx = 0 column
+    for (int k = t; k < NZ; k += kStatsThreads) {
+      if (k == NZH) continue;
+      const size_t at = (size_t)k * NXH, ap = (size_t)(k == 0 ? 0 : NZ - k) * NXH;
+      auto half = [&](const double2 *f) { return make_double2(0.5 * (f[at].x + f[ap].x), 0.5 * (f[at].y - f[ap].y)); };
+      add(half(pu), half(pv), half(pw));
     }
-    acc[0] += wgt * (a.x * a.x + a.y * a.y);
-    acc[1] += wgt * (b.x * b.x + b.y * b.y);
-    acc[2] += wgt * (c.x * c.x + c.y * c.y);
-    acc[3] += wgt * (a.x * b.x + a.y * b.y);
   }
-  __shared__ double red[4][256];
-  for (int q = 0; q < 4; ++q) red[q][threadIdx.x] = acc[q];
+  __shared__ double red[4][kStatsThreads / 32];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_down_sync(0xffffffffu, acc[q], o);
+    if ((t & 31) == 0) red[q][t >> 5] = acc[q];
+  }
   __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st)
-      for (int q = 0; q < 4; ++q) red[q][threadIdx.x] += red[q][threadIdx.x + st];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    const double U = pu[0].x, V = pv[0].x, W = pw[0].x;
-    out[0 * NY + j] = U;
-    out[1 * NY + j] = V;
-    out[2 * NY + j] = W;
-    out[3 * NY + j] = sqrt(fmax(red[0][0] - U * U, 0.0));
-    out[4 * NY + j] = sqrt(fmax(red[1][0] - V * V, 0.0));
-    out[5 * NY + j] = sqrt(fmax(red[2][0] - W * W, 0.0));
-    out[6 * NY + j] = red[3][0] - U * V;
+  if (t < 4) {
+    double s = 0.0;
+    for (int i = 0; i < kStatsThreads / 32; ++i) s += red[t][i];
+    partial[((size_t)j * parts + part) * 4 + t] = s;
   }
 }
+__global__ void k_stats_final(const double2 *u, const double2 *v, const double2 *w, int NY, int M, int parts,
+                              const double *partial, double *out) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= NY) return;
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int p = 0; p < parts; ++p)
+    for (int q = 0; q < 4; ++q) s[q] += partial[((size_t)j * parts + p) * 4 + q];
+  const double U = u[(size_t)j * M].x, V = v[(size_t)j * M].x, W = w[(size_t)j * M].x;
+  out[0 * NY + j] = U;
+  out[1 * NY + j] = V;
+  out[2 * NY + j] = W;
+  out[3 * NY + j] = sqrt(fmax(s[0] - U * U, 0.0));
+  out[4 * NY + j] = sqrt(fmax(s[1] - V * V, 0.0));
+  out[5 * NY + j] = sqrt(fmax(s[2] - W * W, 0.0));
+  out[6 * NY + j] = s[3] - U * V;
+}
+// out: 7 NY values, then scratch; stats_values() in all
+size_t stats_values(int NY, int M) { return (7 + 4 * (size_t)stats_parts(NY, M)) * NY; }
 void launch_stats(const double2 *u, const double2 *v, const double2 *w, int NY, int NZ, int NXH, double *out,
                   cudaStream_t st) {
-  k_stats<<<NY, 256, 0, st>>>(u, v, w, NY, NZ, NXH, out);
+  const int M = NZ * NXH, parts = stats_parts(NY, M);
+  double *partial = out + 7 * (size_t)NY;
+  k_stats<<<dim3(parts, NY), kStatsThreads, 0, st>>>(u, v, w, NY, NZ, NXH, partial);
+  k_stats_final<<<(NY + 63) / 64, 64, 0, st>>>(u, v, w, NY, M, parts, partial, out);
 }
 
 // Reference layout [z][x][y] <-> device layout [y][z][x]: a transpose of an

@@ -235,6 +235,7 @@ void launch_transpose_real(const double *in, double *out, int rows, int cols, cu
 // bytes (a multiple of 16) from device-addressable host memory, both
 // addresses 16-byte aligned, copied by SM loads
 void launch_host_load(const void *src, void *dst, size_t bytes, cudaStream_t st);
+size_t stats_values(int NY, int M);  // doubles launch_stats writes at out (results and scratch)
 void launch_stats(const double2 *u, const double2 *v, const double2 *w, int NY, int NZ, int NXH, double *out,
                   cudaStream_t st);
 
