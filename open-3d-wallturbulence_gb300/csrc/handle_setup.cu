@@ -321,6 +321,7 @@ void owt_handle::setup(const owt_params &prm) {
   ck(lamb_prepare(xd), "transform kernel attributes");
   ck(phys_prepare(xd), "transform kernel attributes");
   ck(nl_prepare(NY), "nonlinear source attributes");
+  ck(dy2_prepare(NY), "DY2 kernel attributes");
   mean_smem = mean_prepare(NY, bg.n);
   zbuf = dalloc<unsigned char>(lamb_zbuf_bytes(xd, 0), owned);
   lbuf = dalloc<unsigned char>(lamb_lbuf_bytes(xd, 0), owned);

@@ -263,7 +263,7 @@ void owt_handle::recompute_dirty_q(cudaStream_t on) {
   a.NY = NY; a.M = M;
   a.m0 = 0; a.mcount = M;
   a.ab1 = b1.ab; a.piv1 = b1.piv; a.ab2 = b2.ab; a.piv2 = b2.piv;
-  a.b1_col = b1_col; a.b1_val = b1_val; a.b2_col = b2_col; a.b2_val = b2_val;
+  a.b1_val = b1_val; a.b2_val = b2_val;
   a.c21 = c21; a.c22 = c22;
   double2 *scr[3] = {tmpA, tmpB, tmpC};
   for (int sl = 0; sl < 3; ++sl) {
@@ -613,7 +613,7 @@ void owt_handle::step_host(const double *const *hist, const double *means, const
             a.NY = NY; a.M = M;
             a.m0 = k0[q] * NXH; a.mcount = (k1[q] - k0[q]) * NXH;
             a.ab1 = b1.ab; a.piv1 = b1.piv; a.ab2 = b2.ab; a.piv2 = b2.piv;
-            a.b1_col = b1_col; a.b1_val = b1_val; a.b2_col = b2_col; a.b2_val = b2_val;
+            a.b1_val = b1_val; a.b2_val = b2_val;
             a.c21 = c21; a.c22 = c22;
             double2 *scr[3] = {tmpA, tmpB, tmpC};
             for (int l = 0; l < 3; ++l) {

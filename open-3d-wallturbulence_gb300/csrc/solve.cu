@@ -781,39 +781,152 @@ void launch_dapply(const DApplyArgs &a, cudaStream_t st) {
 // DY2 f = c21 A1^-1 B1 f + c22 A2^-1 B2 f along y for every mode of up to
 // three fields (the DY2 v history after v levels were replaced), in one
 // launch: one thread per field (blockIdx.y), mode and real component (the
-// band systems are real), two band solves per thread with the B stencils
-// applied inside the right-hand sides.
+// band systems are real).  As the nonlinear source: one sweep up with both
+// stencils on the last five values and both eliminations two rows behind, one
+// sweep down with both solutions; the second system's forward-swept values
+// wait in `out`.  Bound by FP64 issue, 21 operations a node and component.
+// Three fields of a 128x129x128 channel in a host-state step: four launches of
+// 361 us over parts of the modes (one system a thread and sweep) -> one of
+// 350 us.
+//
+// Rows of B2 (setup_host.cpp): columns 0..2 in row 0, 0..4 in row 1, i-2..i+2
+// in between, and the mirror image at the top; B1 as in the nonlinear source.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_dy2(DY2Args a) {
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  if ((tid >> 1) >= a.mcount) return;
-  const int m = a.m0 + (tid >> 1), comp = tid & 1, f = blockIdx.y;
-  const int M = a.M, NY = a.NY;
-  auto E = [&](int j) { return 2 * ((size_t)j * M + m) + comp; };
-  const double *in = reinterpret_cast<const double *>(a.in[f]);
-  double *out = reinterpret_cast<double *>(a.out[f]);
-  double *scr = reinterpret_cast<double *>(a.scr[f]);
-  auto ys = [&](int p, double y) { scr[E(p)] = y; };
-  auto yl = [&](int p) -> double { return scr[E(p)]; };
-  auto stencil = [&](const int *bc, const double *bv, int p) -> double {
-    double acc = 0.0;
-#pragma unroll
-    for (int e = 0; e < 5; ++e) {
-      const double b = bv[p * 5 + e];
-      if (nonzero(b)) acc += b * in[E(bc[p * 5 + e])];
-    }
-    return acc;
+constexpr int kDY2Threads = 64;
+// per row: B1 (4), B2 (5), L1 (2), U1 (5, the reciprocal diagonal first), L2 (2), U2 (5), c21, c22
+constexpr int kDY2Row = 25;
+constexpr size_t dy2_smem_bytes(int NY) { return (size_t)NY * (kDY2Row * sizeof(double) + 2) + 8; }
+constexpr size_t kDY2Smem = 220 * 1024;  // larger tables are read from device memory
+
+template <bool SMEM>
+__global__ void __launch_bounds__(kDY2Threads) k_dy2(const __grid_constant__ DY2Args a) {
+  const int NY = a.NY, n = NY - 1;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double *tab = reinterpret_cast<double *>(smraw);
+  uint8_t *spiv = reinterpret_cast<uint8_t *>(tab + (size_t)NY * kDY2Row);  // of A1, then of A2
+  // entry q of row j: band rows (LAPACK layout, KV = 4) 5, 6 are L, 4 .. 0 U
+  auto entry = [&](int j, int q) -> double {
+    if (q < 4) return a.b1_val[j * 5 + q];
+    if (q < 9) return a.b2_val[j * 5 + q - 4];
+    if (q < 11) return a.ab1[(size_t)(q - 4) * NY + j];
+    if (q < 16) return a.ab1[(size_t)(15 - q) * NY + j];
+    if (q < 18) return a.ab2[(size_t)(q - 11) * NY + j];
+    if (q < 23) return a.ab2[(size_t)(22 - q) * NY + j];
+    return q == 23 ? a.c21[j] : a.c22[j];
   };
-  auto rhs1 = [&](int p) -> double { return stencil(a.b1_col, a.b1_val, p); };
-  auto out1 = [&](int c, double d) { out[E(c)] = a.c21[c] * d; };
-  band_solve<2, 2>(a.ab1, a.piv1, NY, 1, 0, rhs1, ys, yl, out1);
-  auto rhs2 = [&](int p) -> double { return stencil(a.b2_col, a.b2_val, p); };
-  auto out2 = [&](int c, double d) { out[E(c)] += a.c22[c] * d; };
-  band_solve<2, 2>(a.ab2, a.piv2, NY, 1, 0, rhs2, ys, yl, out2);
+  if (SMEM) {
+    for (int e = threadIdx.x; e < NY * kDY2Row; e += kDY2Threads) {
+      const int j = e / kDY2Row;
+      tab[e] = entry(j, e - j * kDY2Row);
+    }
+    for (int j = threadIdx.x; j < NY; j += kDY2Threads) {
+      spiv[j] = a.piv1[j];
+      spiv[NY + j] = a.piv2[j];
+    }
+    __syncthreads();
+  }
+  auto at = [&](int j, int q) { return SMEM ? tab[j * kDY2Row + q] : entry(j, q); };
+  const int tid = blockIdx.x * kDY2Threads + threadIdx.x;
+  if ((tid >> 1) >= a.mcount) return;
+  const size_t ld = 2 * (size_t)a.M, e0 = 2 * (size_t)a.m0 + tid;
+  const double *in = reinterpret_cast<const double *>(a.in[blockIdx.y]) + e0;
+  double *out = reinterpret_cast<double *>(a.out[blockIdx.y]) + e0;
+  double *scr = reinterpret_cast<double *>(a.scr[blockIdx.y]) + e0;
+  auto row = [&](int j) { return (size_t)(j < n ? (j > 0 ? j : 0) : n) * ld; };
+  double f[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, nx[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) nx[q] = in[row(q)];
+  auto push = [&](int j) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) f[q] = f[q + 1];
+    f[4] = nx[0];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) nx[q] = nx[q + 1];
+    nx[3] = in[row(j + 4)];
+  };
+  // sums of row r's entries from q0 with the values v0 ..
+  auto sum = [&](int r, int q0, auto... v) {
+    const double x[] = {v...};
+    double s = at(r, q0) * x[0];
+#pragma unroll
+    for (int i = 1; i < (int)sizeof...(v); ++i) s = fma(at(r, q0 + i), x[i], s);
+    return s;
+  };
+#pragma unroll
+  for (int j = 0; j < 5; ++j) push(j);
+  double w[2][3] = {{sum(0, 0, f[0], f[1], f[2], f[3]), sum(1, 0, f[0], f[2]), sum(2, 0, f[0], f[1], f[3], f[4])},
+                    {sum(0, 4, f[0], f[1], f[2]), sum(1, 4, f[0], f[1], f[2], f[3], f[4]),
+                     sum(2, 4, f[0], f[1], f[2], f[3], f[4])}};
+  double *y[2] = {scr, out};
+  auto eliminate = [&](int c, double next1, double next2) {
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int off = SMEM ? spiv[s * NY + c] : s ? a.piv2[c] : a.piv1[c];
+      if (off == 1) {
+        const double q = w[s][0]; w[s][0] = w[s][1]; w[s][1] = q;
+      } else if (off == 2) {
+        const double q = w[s][0]; w[s][0] = w[s][2]; w[s][2] = q;
+      }
+      const double v = w[s][0];
+      y[s][(size_t)c * ld] = v;
+      w[s][0] = fma(-at(c, s ? 16 : 9), v, w[s][1]);
+      w[s][1] = fma(-at(c, s ? 17 : 10), v, w[s][2]);
+      w[s][2] = s ? next2 : next1;
+    }
+  };
+#pragma unroll 2
+  for (int j = 5; j <= n; ++j) {
+    push(j);
+    eliminate(j - 5, sum(j - 2, 0, f[0], f[1], f[3], f[4]), sum(j - 2, 4, f[0], f[1], f[2], f[3], f[4]));
+  }
+  eliminate(n - 4, sum(n - 1, 0, f[2], f[4]), sum(n - 1, 4, f[0], f[1], f[2], f[3], f[4]));
+  eliminate(n - 3, sum(n, 0, f[1], f[2], f[3], f[4]), sum(n, 4, f[2], f[3], f[4]));
+  eliminate(n - 2, 0.0, 0.0);
+  eliminate(n - 1, 0.0, 0.0);
+  y[0][(size_t)n * ld] = w[0][0];
+  y[1][(size_t)n * ld] = w[1][0];
+  double u[2][5], ny[2][4];
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+#pragma unroll
+    for (int q = 0; q < 5; ++q) u[s][q] = y[s][row(n - q)];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) ny[s][q] = y[s][row(n - 5 - q)];
+  }
+#pragma unroll 2
+  for (int c = n; c >= 0; --c) {
+    double d[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int q0 = s ? 18 : 11;
+      d[s] = u[s][0] * at(c, q0);
+      u[s][0] = fma(-at(c, q0 + 1), d[s], u[s][1]);
+      u[s][1] = fma(-at(c, q0 + 2), d[s], u[s][2]);
+      u[s][2] = u[s][3];
+      u[s][3] = u[s][4];
+      const double u3 = at(c, q0 + 3), u4 = at(c, q0 + 4);
+      if (nonzero(u3) || nonzero(u4)) {  // only beside the row interchanges
+        u[s][2] = fma(-u3, d[s], u[s][2]);
+        u[s][3] = fma(-u4, d[s], u[s][3]);
+      }
+      u[s][4] = ny[s][0];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) ny[s][q] = ny[s][q + 1];
+      ny[s][3] = y[s][row(c - 9)];
+    }
+    out[(size_t)c * ld] = fma(at(c, 24), d[1], __dmul_rn(at(c, 23), d[0]));
+  }
 }
 
+cudaError_t dy2_prepare(int NY) {
+  const size_t b = dy2_smem_bytes(NY);
+  return b <= kDY2Smem ? raise_smem_limit(k_dy2<true>, b) : cudaSuccess;
+}
 void launch_dy2(const DY2Args &a, cudaStream_t st) {
-  k_dy2<<<dim3((unsigned)((2 * (long long)a.mcount + 127) / 128), a.nf), 128, 0, st>>>(a);
+  const dim3 g((unsigned)((2 * (long long)a.mcount + kDY2Threads - 1) / kDY2Threads), a.nf);
+  const size_t b = dy2_smem_bytes(a.NY);
+  if (b <= kDY2Smem) k_dy2<true><<<g, kDY2Threads, b, st>>>(a);
+  else k_dy2<false><<<g, kDY2Threads, 0, st>>>(a);
 }
 
 // Elementwise helpers --------------------------------------------------------

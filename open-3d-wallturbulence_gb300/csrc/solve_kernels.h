@@ -114,7 +114,7 @@ struct DY2Args {
   const double2 *in[3];
   double2 *out[3], *scr[3];  // scr: one field of scratch each
   const double *ab1, *ab2; const uint8_t *piv1, *piv2;
-  const int *b1_col, *b2_col; const double *b1_val, *b2_val;
+  const double *b1_val, *b2_val;
   const double *c21, *c22;
 };
 
@@ -219,6 +219,7 @@ void launch_mean(const MeanArgs &a, bool smem, cudaStream_t st);
 bool mean_prepare(int NY, int n_g);
 void launch_nl(const NLArgs &a, cudaStream_t st);
 void launch_dapply(const DApplyArgs &a, cudaStream_t st);
+cudaError_t dy2_prepare(int NY);  // its shared memory, before any launch
 void launch_dy2(const DY2Args &a, cudaStream_t st);
 void launch_combine_y(double2 *out, const double2 *A, const double *ca, const double2 *B, const double *cb, int NY,
                       int M, cudaStream_t st);
