@@ -279,7 +279,8 @@ int owt_state_restore(owt_handle *h);
  *   the whole fields.
  * OWT_OPT_HOST_CHUNKS: owt_time_integration_host pipelines its uploads with
  *   the mode kernel over this many chunks of Fourier modes (1 .. 8; 0 = the
- *   default, 2) when the mode kernel in use maps threads by quads.
+ *   default: 2, or 1 for channels whose mode kernel has too few blocks to be
+ *   shared out) when the mode kernel in use maps threads by quads.
  * OWT_INFO_SPARSE_SOLVE: 1 if the interior-sparse v-system solve is active.
  * OWT_INFO_PATTERN_VIOLATIONS: modes whose factors fell outside the sparse
  *   pattern at setup (any such mode selects the full-band solve).

@@ -539,7 +539,11 @@ void owt_handle::step_host(const double *const *hist, const double *means, const
   ck(cudaStreamSynchronize(st), "host step");
   const int variant = forced_variant >= 0 ? forced_variant : modes_variant;
   const bool quad = modes_sparse() && !sparse_v6 && modes_variant_is_quad(variant);
-  const int want = host_chunks > 0 ? host_chunks : HostStep::kDefaultChunks;
+  // By default no chunk smaller than twice what is resident at once: a part of
+  // the modes of a small channel takes the mode kernel as long as all of them
+  // (0.96 against 1.02 ms for half of 128x129x128).
+  const int waves = 2 * str_groups(Uq) / (2 * 7 * 152);
+  const int want = host_chunks > 0 ? host_chunks : std::min(HostStep::kDefaultChunks, std::max(waves, 1));
   const int nchunk = quad ? std::min(std::min(want, HostStep::kChunks), NZH + 1) : 1;
   // means first (the mean-mode kernel starts with the step)
   for (int w = 0; w < OWT_NUM_MEANS; ++w)
