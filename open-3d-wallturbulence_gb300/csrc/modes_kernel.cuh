@@ -196,7 +196,7 @@ __device__ __forceinline__ void mode_body(const ModeArgs &a, const int tid) {
           double *uo = reinterpret_cast<double *>(a.u_out), *wo = reinterpret_cast<double *>(a.w_out);
           double *oxo = reinterpret_cast<double *>(a.ox_out), *ozo = reinterpret_cast<double *>(a.oz_out);
           uo[e + comp] = fma(sax, dvo, -(saz * go));
-          wo[e + comp] = fma(sax, go, saz * dvo);
+          wo[e + comp] = fma(saz, dvo, sax * go);
           oxo[e + comp] = fma(-skz, xo, fma(saz, qo, sax * dgo));
           ozo[e + comp] = fma(skx, xo, fma(-sax, qo, saz * dgo));
         }

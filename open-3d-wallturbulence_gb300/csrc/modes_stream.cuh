@@ -572,7 +572,7 @@ __device__ __forceinline__ void str_v(const ModeArgs &a, const StrLane &L, int w
     }
     if (horiz) {
       uo[e] = fma(sax, dvo, -(saz * go));
-      wo[e] = fma(sax, go, saz * dvo);
+      wo[e] = fma(saz, dvo, sax * go);
       oxo[e] = fma(-skz, xo, fma(saz, qo, sax * dgo));
       ozo[e] = fma(skx, xo, fma(-sax, qo, saz * dgo));
     }

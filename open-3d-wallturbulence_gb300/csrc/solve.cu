@@ -692,7 +692,7 @@ __device__ __forceinline__ void nl_body(const NLArgs &a, const int tid) {
 #pragma unroll 4
   for (int c = n; c >= 0; --c) {
     const double d = u[0] * up(c, 0);
-    hv[(size_t)c * ld] = fma(-c11(c), d, -__dmul_rn(k2, nl[0]));
+    hv[(size_t)c * ld] = fma(-k2, nl[0], -__dmul_rn(c11(c), d));
     u[0] = fma(-up(c, 1), d, u[1]);
     u[1] = fma(-up(c, 2), d, u[2]);
     u[2] = u[3];
