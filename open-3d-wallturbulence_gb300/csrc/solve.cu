@@ -1010,7 +1010,9 @@ void launch_lamb_mean_shift(double2 *lx_ring, double2 *lz_ring, const double2 *l
 // (deterministic).  Physical field f = sum_{kx>0} 2 Re(f_k e^{..}) +
 // Re(sum_kz f(0,kz) e^{..}) with the Nyquist kz row dropped, so the x-z mean of
 // f g is sum_{kx>0} 2 Re(f conj g) + sum_kz Re(Hf conj Hg) over the kx = 0
-// column's Hermitian parts Hf(kz) = (f(kz) + conj f(-kz))/2.
+// column's Hermitian parts Hf(kz) = (f(kz) + conj f(-kz))/2.  The fluctuations'
+// sums leave the mean modes out: subtracted afterwards, the squared means
+// cancel most of the sum's digits.
 //
 // Block (part, y) sums a part of plane y's modes, k_stats_final adds the parts.
 // Bound by FP64 issue: eight multiply-adds a mode (the weight 2 of kx > 0 once
@@ -1042,10 +1044,10 @@ __global__ void __launch_bounds__(kStatsThreads)
   }
 #pragma unroll
   for (int q = 0; q < 4; ++q) acc[q] *= 2.0;
-  if (part == 0) {  // the kx = 0 column
-    for (int k = t; k < NZ; k += kStatsThreads) {
+  if (part == 0) {  // the kx = 0 column, without the means
+    for (int k = 1 + t; k < NZ; k += kStatsThreads) {
       if (k == NZH) continue;
-      const size_t at = (size_t)k * NXH, ap = (size_t)(k == 0 ? 0 : NZ - k) * NXH;
+      const size_t at = (size_t)k * NXH, ap = (size_t)(NZ - k) * NXH;
       auto half = [&](const double2 *f) { return make_double2(0.5 * (f[at].x + f[ap].x), 0.5 * (f[at].y - f[ap].y)); };
       add(half(pu), half(pv), half(pw));
     }
@@ -1075,10 +1077,11 @@ __global__ void k_stats_final(const double2 *u, const double2 *v, const double2 
   out[0 * NY + j] = U;
   out[1 * NY + j] = V;
   out[2 * NY + j] = W;
-  out[3 * NY + j] = sqrt(fmax(s[0] - U * U, 0.0));
-  out[4 * NY + j] = sqrt(fmax(s[1] - V * V, 0.0));
-  out[5 * NY + j] = sqrt(fmax(s[2] - W * W, 0.0));
-  out[6 * NY + j] = s[3] - U * V;
+  // (U - U: 0, or NaN for a mean that is not finite)
+  out[3 * NY + j] = sqrt(fmax(s[0] + (U - U), 0.0));
+  out[4 * NY + j] = sqrt(fmax(s[1] + (V - V), 0.0));
+  out[5 * NY + j] = sqrt(fmax(s[2] + (W - W), 0.0));
+  out[6 * NY + j] = s[3] + (U - U) + (V - V);
 }
 // out: 7 NY values, then scratch; stats_values() in all
 size_t stats_values(int NY, int M) { return (7 + 4 * (size_t)stats_parts(NY, M)) * NY; }
