@@ -228,7 +228,7 @@ struct AdjXformKernels {
   void (*zback)(AdjXformArgs), (*xlamb)(AdjXformArgs), (*zfwd)(AdjXformArgs);
   int tx, xlines, zthreads, xthreads;
   size_t zsmem, xsmem;
-  bool persistent;  // the x pass runs the resident blocks
+  bool persistent;  // the x pass runs the resident blocks, a group a pair of lines
 };
 static FxAdjKernels fx_adj_kernels(int L) {
   switch (fx_plan(L).cls) {
@@ -251,7 +251,7 @@ static AdjXformKernels adj_kernels(const XformDims &d, bool stockham) {
   }
   if (fx.ok) {
     k.xlamb = fx.xlamb;
-    k.xlines = fx.xlines; k.xthreads = fx.xthreads; k.xsmem = fx.xsmem;
+    k.xthreads = fx.xthreads; k.xsmem = fx.xsmem;
     k.persistent = true;
   }
   return k;
@@ -274,7 +274,7 @@ void launch_adj_lamb(const AdjXformArgs &a, cudaStream_t st) {
   const int gx = (d.NXH + k.tx - 1) / k.tx;
   k.zback<<<dim3(gx, d.NY, 9), k.zthreads, k.zsmem, st>>>(a);
   size_t grid = ((size_t)d.NY * d.NZ2 + k.xlines - 1) / k.xlines;
-  if (k.persistent) grid = std::min(grid, (size_t)resident_blocks(k.xlamb, k.xthreads, k.xsmem));
+  if (k.persistent) grid = std::min(fx_groups(d, 2), resident_blocks(k.xlamb, k.xthreads, k.xsmem));
   k.xlamb<<<(unsigned)grid, k.xthreads, k.xsmem, st>>>(a);
   k.zfwd<<<dim3(gx, d.NY, 6), k.zthreads, k.zsmem, st>>>(a);
 }

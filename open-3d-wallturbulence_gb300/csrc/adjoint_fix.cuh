@@ -8,12 +8,12 @@
 
 namespace owt {
 
-// (y, z) lines per x group (5 backward and 3 forward lines each) and resident
-// blocks asked of the register allocator, by plan class.
+// Resident blocks asked of the register allocator for an x group of one pair of
+// (y, z) lines (9 backward and 6 forward packed lines), by plan class.
 template <int CLS> struct FxAdjCfg;
-template <> struct FxAdjCfg<0> { static constexpr int P = 2, XB = 5; };
-template <> struct FxAdjCfg<1> { static constexpr int P = 1, XB = 5; };
-template <> struct FxAdjCfg<2> { static constexpr int P = 1, XB = 3; };
+template <> struct FxAdjCfg<0> { static constexpr int XB = 5; };
+template <> struct FxAdjCfg<1> { static constexpr int XB = 3; };
+template <> struct FxAdjCfg<2> { static constexpr int XB = 2; };
 
 template <int CLS>
 __global__ void __launch_bounds__(FxCfg<CLS>::TX *FxCfg<CLS>::T, FxCfg<CLS>::ZB)
@@ -64,82 +64,72 @@ __global__ void __launch_bounds__(FxCfg<CLS>::TX *FxCfg<CLS>::T, FxCfg<CLS>::ZB)
 
 template <int CLS>
 constexpr size_t fx_adj_xsmem(int A, int B) {
-  constexpr int P = FxAdjCfg<CLS>::P;
-  return 6 * P * (size_t)fx_xline(A, B) * sizeof(fxc) + (size_t)fx_xtables(A, B) * sizeof(FxTw) +
-         5 * P * ((size_t)FxCfg<CLS>::T * sizeof(FxBound) + sizeof(FxScale));
+  return 9 * (size_t)fx_xline(A, B) * sizeof(fxc) + (size_t)fx_xtables(A, B) * sizeof(FxTw) +
+         9 * ((size_t)FxCfg<CLS>::T * sizeof(FxBound) + sizeof(FxScale));
 }
 
-// Persistent; per group of P (y, z) lines: 5P packed backward lines (u,v)
-// (w,ox) (oy,oz) (lbx,lby) (lbz,0), products, 3P packed forward lines.
+// Persistent; per pair of (y, z) lines: 9 packed backward lines (u v w ox oy oz
+// lbx lby lbz, one field on both lines, as the step's x pass), products,
+// 6 packed forward lines.  In place: a line's pass reads all it needs before a
+// barrier.
 template <int CLS>
-__global__ void __launch_bounds__(5 * FxAdjCfg<CLS>::P *FxCfg<CLS>::T, FxAdjCfg<CLS>::XB)
+__global__ void __launch_bounds__(9 * FxCfg<CLS>::T, FxAdjCfg<CLS>::XB)
     k_xlamb_adj_fx(const __grid_constant__ AdjXformArgs a) {
-  constexpr int P = FxAdjCfg<CLS>::P, NF = 3 * P;
   extern __shared__ __align__(16) unsigned char smraw[];
   const XformDims d = a.d;
   const FxPlan p = a.fpx;
   const int A = p.A, B = p.B, LS = fx_xline(A, B), ntw = fx_xtables(A, B);
   fxc *R = reinterpret_cast<fxc *>(smraw);
-  FxTw *tw = reinterpret_cast<FxTw *>(R + 6 * P * LS);
+  FxTw *tw = reinterpret_cast<FxTw *>(R + 9 * LS);
   FxBound *bd = reinterpret_cast<FxBound *>(tw + ntw);
-  FxScale *sc = reinterpret_cast<FxScale *>(bd + 5 * P * FxCfg<CLS>::T);
+  FxScale *sc = reinterpret_cast<FxScale *>(bd + 9 * FxCfg<CLS>::T);
   double2 *D = reinterpret_cast<double2 *>(R);
   for (int k = threadIdx.x; k < ntw; k += blockDim.x) tw[k] = a.fxx[k];
   const int q = threadIdx.x / p.T, t = threadIdx.x - q * p.T;
-  const size_t nlines = (size_t)d.NY * d.NZ2, fstride = nlines * d.NXH;
-  const int ngroups = (int)((nlines + P - 1) / P);
+  const size_t fstride = (size_t)d.NY * d.NZ2 * d.NXH;
+  const int ngroups = fx_groups(d, 2);
   for (int g = blockIdx.x; g < ngroups; g += gridDim.x) {
     __syncthreads();  // the last group's spectra are read (the first: the table is written)
-    const size_t line0 = (size_t)g * P;
-    // 1. backward transforms
-    {
-      const int pair = q / P, l = q - pair * P;
-      const bool have = line0 + l < nlines;
-      const double2 *Af = a.zbuf + (size_t)(2 * pair) * fstride + (line0 + l) * d.NXH;
-      fx_x_pass1<CLS, true>(
-          p, t < B, q, t,
-          [&](auto upper, int s) {
-            return fx_bits(fx_hermitian<decltype(upper)::value>(Af, fstride, have, s, d.NXH, d.NX2, pair < 4));
-          },
-          R + q * LS, tw, bd, sc);
-    }
+    const FxPair pr = fx_pair(d, (unsigned)g);
+    // 1. backward transforms: line q is field q
+    const double2 *Af = a.zbuf + (size_t)q * fstride + pr.line * d.NXH;
+    fx_x_pass1<CLS, true>(
+        p, t < B, q, t,
+        [&](auto upper, int s) {
+          return fx_bits(fx_hermitian<decltype(upper)::value>(Af, pr.have, pr.have_b, s, d.NXH, d.NX2));
+        },
+        R + q * LS, tw, bd, sc);
     __syncthreads();
     fx_x_pass2_back<CLS>(p, t < A, t, R + q * LS, sc + q);
     __syncthreads();
-    // 2. u_bar = om x lb, om_bar = lb x u, packed (ub,vb) (wb,oxb) (oyb,ozb), in place
-    for (int idx = threadIdx.x; idx < P * A * B; idx += blockDim.x) {
-      const int l = idx / (A * B), x = idx - l * (A * B);
-      const double2 uv = D[(0 * P + l) * LS + x], wox = D[(1 * P + l) * LS + x], oyz = D[(2 * P + l) * LS + x];
-      const double2 bxy = D[(3 * P + l) * LS + x], bz0 = D[(4 * P + l) * LS + x];
-      const double u = uv.x, v = uv.y, w = wox.x, ox = wox.y, oy = oyz.x, oz = oyz.y;
-      const double bx = bxy.x, by = bxy.y, bz = bz0.x;
-      D[(0 * P + l) * LS + x] = make_double2(oy * bz - oz * by, oz * bx - ox * bz);
-      D[(1 * P + l) * LS + x] = make_double2(ox * by - oy * bx, by * w - bz * v);
-      D[(2 * P + l) * LS + x] = make_double2(bz * u - bx * w, bx * v - by * u);
+    // 2. u_bar = om x lb, om_bar = lb x u into lines 0..5, in place
+    for (int x = threadIdx.x; x < A * B; x += blockDim.x) {
+      const double2 u = D[x], v = D[LS + x], w = D[2 * LS + x], ox = D[3 * LS + x], oy = D[4 * LS + x],
+                    oz = D[5 * LS + x], bx = D[6 * LS + x], by = D[7 * LS + x], bz = D[8 * LS + x];
+      D[x] = make_double2(oy.x * bz.x - oz.x * by.x, oy.y * bz.y - oz.y * by.y);
+      D[LS + x] = make_double2(oz.x * bx.x - ox.x * bz.x, oz.y * bx.y - ox.y * bz.y);
+      D[2 * LS + x] = make_double2(ox.x * by.x - oy.x * bx.x, ox.y * by.y - oy.y * bx.y);
+      D[3 * LS + x] = make_double2(by.x * w.x - bz.x * v.x, by.y * w.y - bz.y * v.y);
+      D[4 * LS + x] = make_double2(bz.x * u.x - bx.x * w.x, bz.y * u.y - bx.y * w.y);
+      D[5 * LS + x] = make_double2(bx.x * v.x - by.x * u.x, bx.y * v.y - by.y * u.y);
     }
     __syncthreads();
     // 3. forward transforms
     fx_x_pass1<CLS, false>(
-        p, q < NF && t < A, q, t, [&](auto, int s) { return fx_bits(D[q * LS + s]); }, R + (NF + (q < NF ? q : 0)) * LS,
+        p, q < 6 && t < A, q, t, [&](auto, int s) { return fx_bits(D[q * LS + s]); }, R + q * LS,
         A == B ? tw : tw + A * B, bd, sc);
     __syncthreads();
-    if (q < NF && t < B) fx_x_pass2_fwd<CLS>(p, t, R + (NF + q) * LS, R + q * LS);
+    fx_x_pass2_fwd<CLS, true>(p, q < 6 && t < B, t, R + q * LS, R + q * LS);
     __syncthreads();
     // 4. unpack the real-pair spectra, keep kx < NXH, weight 1 (kx = 0) or 2
-    for (int idx = threadIdx.x; idx < P * d.NXH; idx += blockDim.x) {
-      const int l = idx / d.NXH, km = idx - l * d.NXH;
-      const size_t line = line0 + l;
-      if (line >= nlines) continue;
+    for (int idx = threadIdx.x; idx < 6 * d.NXH; idx += blockDim.x) {
+      const int f = idx / d.NXH, km = idx - f * d.NXH;
       const int mc = (km == 0) ? 0 : d.NX2 - km;
-#pragma unroll
-      for (int pair = 0; pair < 3; ++pair) {
-        const double w = (km == 0 ? 0.5 : 1.0) * fx_factor(sc[pair * P + l]);
-        const fxc zm = R[(pair * P + l) * LS + km], zc = R[(pair * P + l) * LS + mc];
-        a.lbuf[(size_t)(2 * pair) * fstride + line * d.NXH + km] =
-            make_double2(__ll2double_rn(zm.x + zc.x) * w, __ll2double_rn(zm.y - zc.y) * w);
-        a.lbuf[(size_t)(2 * pair + 1) * fstride + line * d.NXH + km] =
-            make_double2(__ll2double_rn(zm.y + zc.y) * w, __ll2double_rn(zc.x - zm.x) * w);
-      }
+      const double w = (km == 0 ? 0.5 : 1.0) * fx_factor(sc[f]);
+      const fxc zm = R[f * LS + km], zc = R[f * LS + mc];
+      double2 *o = a.lbuf + (size_t)f * fstride + pr.line * d.NXH + km;
+      o[0] = make_double2(__ll2double_rn(zm.x + zc.x) * w, __ll2double_rn(zm.y - zc.y) * w);
+      if (pr.have_b) o[d.NXH] = make_double2(__ll2double_rn(zm.y + zc.y) * w, __ll2double_rn(zc.x - zm.x) * w);
     }
   }
 }
@@ -156,8 +146,7 @@ FxAdjKernels fx_adj_kernels_of_class(int L) {
   k.tx = FxCfg<CLS>::TX;
   k.zthreads = FxCfg<CLS>::TX * p.T;
   k.zsmem = fx_zsmem<CLS>(L);
-  k.xlines = FxAdjCfg<CLS>::P;
-  k.xthreads = 5 * FxAdjCfg<CLS>::P * p.T;
+  k.xthreads = 9 * p.T;
   k.xsmem = fx_adj_xsmem<CLS>(p.A, p.B);
   return k;
 }

@@ -52,7 +52,7 @@ struct AdjXformArgs {
 struct FxAdjKernels {
   bool ok = false;
   void (*zback)(AdjXformArgs) = nullptr, (*xlamb)(AdjXformArgs) = nullptr, (*zfwd)(AdjXformArgs) = nullptr;
-  int tx = 0, zthreads = 0, xthreads = 0, xlines = 0;
+  int tx = 0, zthreads = 0, xthreads = 0;  // an x group: one pair of lines
   size_t zsmem = 0, xsmem = 0;
 };
 FxAdjKernels fx_adj_kernels0(int L);

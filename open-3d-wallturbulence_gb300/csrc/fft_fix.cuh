@@ -384,11 +384,14 @@ __device__ __forceinline__ double fx_to_double(long long n, FxOut o) {
 #endif
 
 // ---------------------------------------------------------------------------
-// Products of two lines in physical space and the transform back, all in
-// integers.  A line's integers after a transform are 2^k x with k = e - 2 and
-// at most 61 bits; the product of u and o (of lines with k_u, k_o) is
-// fx_product(u << 1, o << 2) = u o 2^-61, rounded, 2^(k_u + k_o - 61) times the
-// real product.
+// Products of lines in physical space and the transform back, all in integers.
+// A packed line holds one field on two neighbouring (y, z) lines: its integers
+// after a transform are 2^k x with k = e - 2 and at most 62 bits.  Each field
+// is shifted left to its own largest value, below 2^62; the high 64 bits of
+// u o are then 2^(k_u + k_o - 64) times the real product, below 2^60.  (Two
+// fields in one line would share a scale: w beside o_x, hundreds of times
+// larger, lost its low bits, and the products' error rose to 1.45 times that
+// of FP64 where o_x has a mean.)
 // ---------------------------------------------------------------------------
 OWT_HD long long fx_product(int ah, int al, int bh, int bl) {  // words of fx_split
   const long long cr = fx_wide(al, bh) + (fx_wide(ah, bl) + 0x80000000ll);
@@ -397,31 +400,64 @@ OWT_HD long long fx_product(int ah, int al, int bh, int bl) {  // words of fx_sp
 OWT_HD long long fx_shift_right(long long x, int d) {  // rounded, 0 <= d <= 62
   return (x + ((1ll << d) >> 1)) >> d;
 }
+// |high word| of a value or of the larger component, for a line's largest
+OWT_HD unsigned fx_mag(long long v) {
+  const int hi = fx_hi(v);
+  return (unsigned)(hi ^ (hi >> 31));
+}
+OWT_HD unsigned fx_mag(fxc v) {  // (an OR has the same highest bit as the maximum)
+  return fx_mag(v.x) | fx_mag(v.y);
+}
+OWT_HD int fx_bits_of(unsigned v) {  // position of the highest set bit, from 1; 0 for 0
+#ifdef __CUDA_ARCH__
+  return 32 - __clz((int)v);
+#else
+  return v ? 32 - __builtin_clz(v) : 0;
+#endif
+}
 // k of a line after its transform; a line of zeros does not limit the scale
 // of the products it enters.
 OWT_HD int fx_k(const FxScale &s) { return s.rsh == 4096 ? 1 << 14 : s.e - 2; }
-// Right shifts of the six products of a (y, z) line for k of the (u, v),
-// (w, ox) and (oy, oz) lines, and the scales of (lx, ly) and of lz.
-struct FxProducts {
-  int s02, s12, s11;  // lx = v oz - w oy, ly = w ox - u oz
-  int z02, z01;       // lz = u oy - v ox
-  int kxy, kz;
-};
 OWT_HD int fx_min(int a, int b) { return a < b ? a : b; }
-// kz_other: the lz scale of the line that shares lz's transform
-OWT_HD int fx_kz(int k0, int k1, int k2) { return fx_min(k0 + k2, k0 + k1) - 61; }
-OWT_HD FxProducts fx_products(int k0, int k1, int k2, int kz_other) {
+// Left shifts of the fields u, v, w, ox, oy, oz, right shifts of the products
+// and the scales k of lx = v oz - w oy, ly = w ox - u oz, lz = u oy - v ox.
+struct FxProducts {
+  int s[6];
+  int v_oz, w_oy, w_ox, u_oz, u_oy, v_ox;
+  int k[3];
+};
+// k, mag: the six lines' scales and largest magnitudes (fx_mag)
+OWT_HD FxProducts fx_products(const int (&k)[6], const unsigned (&mag)[6]) {
   FxProducts p;
-  const int c02 = k0 + k2, c12 = k1 + k2, c11 = 2 * k1, c01 = k0 + k1;
-  const int c = fx_min(c02, fx_min(c12, c11)), z = fx_min(fx_min(c02, c01), kz_other + 61);
-  p.s02 = fx_min(c02 - c, 62);
-  p.s12 = fx_min(c12 - c, 62);
-  p.s11 = fx_min(c11 - c, 62);
-  p.z02 = fx_min(c02 - z, 62);
-  p.z01 = fx_min(c01 - z, 62);
-  p.kxy = c - 61;
-  p.kz = z - 61;
+  int n[6];
+  for (int f = 0; f < 6; ++f) {
+    p.s[f] = 30 - fx_bits_of(mag[f]);
+    n[f] = k[f] + p.s[f];
+  }
+  const int cx = fx_min(n[1] + n[5], n[2] + n[4]);
+  const int cy = fx_min(n[2] + n[3], n[0] + n[5]);
+  const int cz = fx_min(n[0] + n[4], n[1] + n[3]);
+  p.v_oz = fx_min(n[1] + n[5] - cx, 62);
+  p.w_oy = fx_min(n[2] + n[4] - cx, 62);
+  p.w_ox = fx_min(n[2] + n[3] - cy, 62);
+  p.u_oz = fx_min(n[0] + n[5] - cy, 62);
+  p.u_oy = fx_min(n[0] + n[4] - cz, 62);
+  p.v_ox = fx_min(n[1] + n[3] - cz, 62);
+  p.k[0] = cx - 64;
+  p.k[1] = cy - 64;
+  p.k[2] = cz - 64;
   return p;
+}
+// The Lamb vector at one point: f the six fields in, l out.
+OWT_HD void fx_lamb(const long long (&f)[6], const FxProducts &p, long long (&l)[3]) {
+  int h[6], w[6];
+  for (int i = 0; i < 6; ++i) fx_split(f[i] << p.s[i], h[i], w[i]);
+  l[0] = fx_shift_right(fx_product(h[1], w[1], h[5], w[5]), p.v_oz) -
+         fx_shift_right(fx_product(h[2], w[2], h[4], w[4]), p.w_oy);
+  l[1] = fx_shift_right(fx_product(h[2], w[2], h[3], w[3]), p.w_ox) -
+         fx_shift_right(fx_product(h[0], w[0], h[5], w[5]), p.u_oz);
+  l[2] = fx_shift_right(fx_product(h[0], w[0], h[4], w[4]), p.u_oy) -
+         fx_shift_right(fx_product(h[1], w[1], h[3], w[3]), p.v_ox);
 }
 // Bound of a thread's integers (below 2^62) in units of 2^38.
 template <int N>

@@ -241,8 +241,9 @@ struct owt_handle {
     cudaStream_t up = nullptr, tx = nullptr, aux = nullptr, down = nullptr;
     // chunks of Fourier modes the uploads and the mode kernel pipeline over:
     // at most kChunks; unless set, kDefaultChunks where the mode kernel has
-    // enough blocks, else one (two measured fastest at 384x257x384, 6% ahead of one and of four; with eight the DY2 v
-    // re-derivations compete with the mode kernel, 25% slower)
+    // enough blocks, else one (two measured fastest at 384x257x384, 6% ahead
+    // of one and of four; with eight the DY2 v re-derivations compete with the
+    // mode kernel, 25% slower)
     static constexpr int kChunks = 8, kDefaultChunks = 2;
     double2 *stage[12] = {}, *dstage[2] = {nullptr, nullptr};
     // pinned host staging of the six friction values in and out, so that

@@ -268,9 +268,14 @@ struct FxXformKernels {
   void (*zback)(XformArgs) = nullptr, (*xlamb)(XformArgs) = nullptr, (*zfwd)(XformArgs) = nullptr;
   void (*zback_b)(BatchTable<XformArgs>) = nullptr, (*xlamb_b)(BatchTable<XformArgs>) = nullptr,
       (*zfwd_b)(BatchTable<XformArgs>) = nullptr;
-  int tx = 0, zthreads = 0, xthreads = 0, xlines = 0;  // kx columns per z block, (y, z) lines per x group
+  int tx = 0, zthreads = 0, xthreads = 0, xlines = 0;  // kx columns per z block, (y, z) lines per x group (fx_groups)
   size_t zsmem = 0, xsmem = 0;
 };
+// Groups of the fixed-point x pass: `lines` (y, z) lines (even) in pairs of
+// z-neighbours, the last pair of a plane one line where NZ2 is odd.
+__host__ __device__ inline int fx_groups(const XformDims &d, int lines) {
+  return (d.NY * ((d.NZ2 + 1) / 2) + lines / 2 - 1) / (lines / 2);
+}
 FxXformKernels fx_xform_kernels0(int L);  // by class of the plan
 FxXformKernels fx_xform_kernels1(int L);
 FxXformKernels fx_xform_kernels2(int L);

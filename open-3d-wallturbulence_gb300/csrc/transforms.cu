@@ -345,6 +345,10 @@ struct XformKernels {
   int zthreads, xthreads;
   size_t zsmem, xsmem;
   int xgrid;  // x-pass blocks at most (0: one block per group of P lines)
+  bool pairs = false;  // groups of the fixed-point kernels (fx_groups)
+  int xgroups(const XformDims &d) const {
+    return pairs ? fx_groups(d, P) : (int)(((size_t)d.NY * d.NZ2 + P - 1) / P);
+  }
 };
 static FxXformKernels fx_kernels(int L) {
   switch (fx_plan(L).cls) {
@@ -407,6 +411,7 @@ static XformKernels<T> kernels(const XformDims &d, bool stockham = false) {
       k.xthreads = fx.xthreads;
       k.xsmem = fx.xsmem;
       k.P = fx.xlines;
+      k.pairs = true;
       k.xgrid = resident_blocks(fx.xlamb, fx.xthreads, fx.xsmem);
     }
   }
@@ -423,9 +428,8 @@ static void lamb_part_t(const XformArgs &a, int part, cudaStream_t st) {
   if (part == 0) {
     k.zback<<<dim3(gx, d.NY, 6), k.zthreads, k.zsmem, st>>>(a);
   } else if (part == 1) {
-    const size_t nl = (size_t)d.NY * d.NZ2;
-    size_t grid = (nl + k.P - 1) / k.P;
-    if (k.xgrid > 0 && grid > (size_t)k.xgrid) grid = k.xgrid;
+    int grid = k.xgroups(d);
+    if (k.xgrid > 0 && grid > k.xgrid) grid = k.xgrid;
     k.xlamb<<<(unsigned)grid, k.xthreads, k.xsmem, st>>>(a);
   } else if (part == 2) {
     k.zfwd<<<dim3(gx, d.NY, 3), k.zthreads, k.zsmem, st>>>(a);
@@ -482,7 +486,7 @@ static int lamb_blocks_t(const XformDims &d, int part, bool stockham) {
   const int gx = (d.NXH + k.tx - 1) / k.tx;
   if (part == 0) return gx * d.NY * 6;
   if (part == 2) return gx * d.NY * 3;
-  if (part == 1) return (int)(((size_t)d.NY * d.NZ2 + k.P - 1) / k.P);
+  if (part == 1) return k.xgroups(d);
   return ((d.NZ * d.NXH + 255) / 256) * d.NY;
 }
 int lamb_batch_blocks(const XformDims &d, int precision, int part, bool stockham) {

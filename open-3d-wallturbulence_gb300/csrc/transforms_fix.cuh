@@ -16,7 +16,8 @@
 //  k_xlamb_fx : persistent; per group of P (y, z) lines: 3P packed backward
 //               lines, products in shared memory (integers too), 3P/2 packed
 //               forward lines, the real-pair unpack; the next group's input
-//               is prefetched into L2.
+//               is prefetched into L2.  A packed line holds one field on two
+//               z-neighbours of a plane, so that a field has its own scale.
 //  k_zfwd_fx  : as k_zback_fx, forward.
 //
 // Measured at 384x257x384 (lines of 576 points), FP64 kernels -> these:
@@ -172,22 +173,35 @@ __device__ __forceinline__ void zfwd_fx_body(const XformArgs &a, const int bx, c
 // ---------------------------------------------------------------------------
 // x pass
 // ---------------------------------------------------------------------------
-// Point m = t + N2 r of the packed line of two real lines' spectra A, B
-// (hermitian_pair of owt_device.cuh): UPPER (r in the upper third) takes the
+// Point m = t + N2 r of the packed line of two real lines' spectra A and
+// B = A + NXH (hermitian_pair of owt_device.cuh): UPPER (r in the upper third) takes the
 // conjugate half, the padding slot 2 NX2/3 included as zero.  have, have_b:
 // the lines exist (else zeros).
 template <bool UPPER>
-__device__ __forceinline__ double2 fx_hermitian(const double2 *__restrict__ A, size_t fstride, bool have, int m, int NXH,
-                                                int NX2, bool have_b = true) {
+__device__ __forceinline__ double2 fx_hermitian(const double2 *__restrict__ A, bool have, bool have_b, int m, int NXH,
+                                                int NX2) {
   const int mp = UPPER ? NX2 - m : m;
   double2 x = make_double2(0.0, 0.0), y = x;
   if (have && mp < NXH) {
     x = __ldg(A + mp);
-    if (have_b) y = __ldg(A + fstride + mp);
+    if (have_b) y = __ldg(A + NXH + mp);
   }
   if (UPPER) return make_double2(x.x + y.y, y.x - x.y);
   if (m == 0) x.y = y.y = 0.0;
   return make_double2(x.x - y.y, x.y + y.x);
+}
+
+// Pairs of z-neighbours are numbered plane by plane (the last of a plane with
+// an odd number of lines holds one line); groups of the x pass are PAIRS
+// consecutive pairs.
+struct FxPair {
+  bool have, have_b;
+  size_t line;  // the first line, y NZ2 + z
+};
+__device__ __forceinline__ FxPair fx_pair(const XformDims &d, unsigned pair) {
+  const unsigned half = (unsigned)(d.NZ2 + 1) / 2, j = pair / half, z = 2 * (pair - j * half);
+  const bool have = j < (unsigned)d.NY;
+  return FxPair{have, have && (int)z + 1 < d.NZ2, (size_t)j * d.NZ2 + z};
 }
 
 // Shared memory: 3P lines of LS values (transposes with odd row stride, or
@@ -201,7 +215,7 @@ template <int CLS>
 constexpr size_t fx_xsmem(int A, int B) {
   constexpr int P = FxCfg<CLS>::P;
   return 3 * P * (size_t)fx_xline(A, B) * sizeof(fxc) + (size_t)fx_xtables(A, B) * sizeof(FxTw) +
-         3 * P * ((size_t)FxCfg<CLS>::T * sizeof(FxBound) + sizeof(FxScale));
+         3 * P * ((size_t)FxCfg<CLS>::T * sizeof(FxBound) + sizeof(FxScale) + sizeof(unsigned));
 }
 
 // Pass 1 of line q's transform on input in(r, s) (s = t + N2 r), its
@@ -250,9 +264,11 @@ __device__ __forceinline__ void fx_x_pass1(const FxPlan p, bool act, int q, int 
 }
 
 // Backward pass 2 of line q: point t + A r, in place (R: the line), as FP64 or
-// (INT) as integers of scale fx_k(*sc).
+// (INT) as integers of scale fx_k(*sc) with the highest bit of fx_mag into mag
+// (zero on entry).
 template <int CLS, bool INT = false>
-__device__ __forceinline__ void fx_x_pass2_back(const FxPlan p, bool act, int t, fxc *R, const FxScale *sc) {
+__device__ __forceinline__ void fx_x_pass2_back(const FxPlan p, bool act, int t, fxc *R, const FxScale *sc,
+                                                unsigned *mag = nullptr) {
   const int A = p.A;
   fx_radix<CLS>(p.B, [&](auto n) {
     constexpr int N = decltype(n)::value, RS = fx_row(N);
@@ -261,6 +277,11 @@ __device__ __forceinline__ void fx_x_pass2_back(const FxPlan p, bool act, int t,
     if (act) {
       fx_for<0, N>([&](auto rc) { y[decltype(rc)::value] = R[t * RS + decltype(rc)::value]; });
       fx_dft<N, true>(y);
+      if constexpr (INT) {
+        unsigned m = 0;
+        fx_for<0, N>([&](auto rc) { m |= fx_mag(y[decltype(rc)::value]); });
+        atomicOr(mag, m);
+      }
     }
     __syncthreads();
     if (!act) return;
@@ -278,15 +299,22 @@ __device__ __forceinline__ void fx_x_pass2_back(const FxPlan p, bool act, int t,
 }
 
 // Forward pass 2: spectrum slot t + B r, integers, from the transposes at R
-// into the line at out (the middle third is not read).  No barrier.
-template <int CLS>
-__device__ __forceinline__ void fx_x_pass2_fwd(const FxPlan p, int t, const fxc *R, fxc *out) {
+// into the line at out (the middle third is not read).  IN_PLACE: out is R,
+// all threads call it (act: the thread has a transform); else no barrier.
+template <int CLS, bool IN_PLACE = false>
+__device__ __forceinline__ void fx_x_pass2_fwd(const FxPlan p, bool act, int t, const fxc *R, fxc *out) {
   const int B = p.B;
+  if (!IN_PLACE && !act) return;
   fx_radix<CLS>(p.A, [&](auto n) {
     constexpr int N = decltype(n)::value, RS = fx_row(N);
     fxc y[N];
-    fx_for<0, N>([&](auto rc) { y[decltype(rc)::value] = R[t * RS + decltype(rc)::value]; });
-    fx_dft<N, false>(y);
+    if constexpr (IN_PLACE) fx_for<0, N>([&](auto rc) { y[decltype(rc)::value] = fxc{0, 0}; });
+    if (act) {
+      fx_for<0, N>([&](auto rc) { y[decltype(rc)::value] = R[t * RS + decltype(rc)::value]; });
+      fx_dft<N, false>(y);
+    }
+    if constexpr (IN_PLACE) __syncthreads();
+    if (!act) return;
     fx_for<0, N>([&](auto rc) {
       constexpr int r = decltype(rc)::value;
       if constexpr (N % 3 != 0 || r < N / 3 || r >= 2 * N / 3) out[t + B * r] = y[r];
@@ -295,84 +323,65 @@ __device__ __forceinline__ void fx_x_pass2_fwd(const FxPlan p, int t, const fxc 
 }
 
 template <int CLS>
-__device__ __forceinline__ void xlamb_fx_group(const XformArgs &a, const size_t line0, fxc *R, const FxTw *tw,
-                                               FxBound *bd, FxScale *sc) {
-  constexpr int P = FxCfg<CLS>::P, NF = P + P / 2;
+__device__ __forceinline__ void xlamb_fx_group(const XformArgs &a, const unsigned pair0, fxc *R, const FxTw *tw,
+                                               FxBound *bd, FxScale *sc, unsigned *mag) {
+  constexpr int P = FxCfg<CLS>::P, H = P / 2, NF = 3 * H;
   const XformDims d = a.d;
   const FxPlan p = a.fpx;
   const int A = p.A, B = p.B, LS = fx_xline(A, B);
   const int q = threadIdx.x / p.T, t = threadIdx.x - q * p.T;
-  const size_t nlines = (size_t)d.NY * d.NZ2, fstride = nlines * d.NXH;
-  // 1. backward pass 1: packed line q = pair P + l holds fields (2 pair, 2 pair + 1)
+  const size_t fstride = (size_t)d.NY * d.NZ2 * d.NXH;
+  // 1. backward pass 1: packed line q = H f + h holds pair h of field f
+  if (t == 0) mag[q] = 0u;
   {
-    const int pair = q / P, l = q - pair * P;
-    const bool have = line0 + l < nlines;
-    const double2 *Af = reinterpret_cast<const double2 *>(a.zbuf) + (size_t)(2 * pair) * fstride + (line0 + l) * d.NXH;
+    const int f = q / H;
+    const FxPair pr = fx_pair(d, pair0 + (q - f * H));
+    const double2 *Af = reinterpret_cast<const double2 *>(a.zbuf) + (size_t)f * fstride + pr.line * d.NXH;
     fx_x_pass1<CLS, true>(
         p, t < B, q, t,
         [&](auto upper, int s) {
-          return fx_bits(fx_hermitian<decltype(upper)::value>(Af, fstride, have, s, d.NXH, d.NX2));
+          return fx_bits(fx_hermitian<decltype(upper)::value>(Af, pr.have, pr.have_b, s, d.NXH, d.NX2));
         },
         R + q * LS, tw, bd, sc);
   }
   __syncthreads();
   // 2. backward pass 2
-  fx_x_pass2_back<CLS, true>(p, t < A, t, R + q * LS, sc + q);
+  fx_x_pass2_back<CLS, true>(p, t < A, t, R + q * LS, sc + q, mag + q);
   __syncthreads();
-  // 3. lamb = u x omega in integers, packed as (lx + i ly) in line l and
-  // (lz_l + i lz_l+1) in line P + l/2, in place: one thread owns point xx of
-  // every line
-  int pk = 0;
+  // 3. lamb = u x omega in integers, component c of pair h into line H c + h,
+  // in place: one thread owns point xx of every line
+  int pk = 0;  // scale and finiteness of this thread's forward line
   bool ok = true;
-  {
-    FxProducts pr[P];
+#pragma unroll 1
+  for (int h = 0; h < H; ++h) {
+    int k[6];
+    unsigned mg[6];
+    bool fin = true;
 #pragma unroll
-    for (int l = 0; l < P; l += 2) {
-      int k[2][3];
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int i = 0; i < 3; ++i) k[h][i] = fx_k(sc[i * P + l + h]);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) pr[l + h] = fx_products(k[h][0], k[h][1], k[h][2], fx_kz(k[1 - h][0], k[1 - h][1], k[1 - h][2]));
+    for (int f = 0; f < 6; ++f) {
+      k[f] = fx_k(sc[f * H + h]);
+      fin = fin && sc[f * H + h].finite;
+      mg[f] = mag[f * H + h];
     }
-    // scale and finiteness of this thread's forward line
+    const FxProducts pr = fx_products(k, mg);
 #pragma unroll
-    for (int l = 0; l < P; ++l) {
-      const bool f = sc[l].finite && sc[P + l].finite && sc[2 * P + l].finite;
-      if (q == l) {
-        pk = pr[l].kxy;
-        ok = f;
+    for (int c = 0; c < 3; ++c)
+      if (q == c * H + h) {
+        pk = pr.k[c];
+        ok = fin;
       }
-      if (q == P + l / 2) {
-        pk = pr[l].kz;
-        ok = ok && f;
-      }
-    }
     for (int xx = threadIdx.x; xx < A * B; xx += blockDim.x) {
+      long long f0[6], f1[6], l0[3], l1[3];
 #pragma unroll
-      for (int l = 0; l < P; l += 2) {
-        long long lz[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const fxc uv = R[(l + h) * LS + xx], wox = R[(P + l + h) * LS + xx], oyz = R[(2 * P + l + h) * LS + xx];
-          const FxProducts &c = pr[l + h];
-          int uh, ul, vh, vl, wh, wl, xh, xl, yh, yl, zh, zl;
-          fx_split(uv.x << 1, uh, ul);
-          fx_split(uv.y << 1, vh, vl);
-          fx_split(wox.x << 1, wh, wl);
-          fx_split(wox.y << 2, xh, xl);
-          fx_split(oyz.x << 2, yh, yl);
-          fx_split(oyz.y << 2, zh, zl);
-          const long long lx = fx_shift_right(fx_product(vh, vl, zh, zl), c.s02) -
-                               fx_shift_right(fx_product(wh, wl, yh, yl), c.s12);
-          const long long ly = fx_shift_right(fx_product(wh, wl, xh, xl), c.s11) -
-                               fx_shift_right(fx_product(uh, ul, zh, zl), c.s02);
-          lz[h] = fx_shift_right(fx_product(uh, ul, yh, yl), c.z02) - fx_shift_right(fx_product(vh, vl, xh, xl), c.z01);
-          R[(l + h) * LS + xx] = fxc{lx, ly};
-        }
-        R[(P + l / 2) * LS + xx] = fxc{lz[0], lz[1]};
+      for (int f = 0; f < 6; ++f) {
+        const fxc v = R[(f * H + h) * LS + xx];
+        f0[f] = v.x;
+        f1[f] = v.y;
       }
+      fx_lamb(f0, pr, l0);
+      fx_lamb(f1, pr, l1);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) R[(c * H + h) * LS + xx] = fxc{l0[c], l1[c]};
     }
   }
   __syncthreads();
@@ -382,72 +391,73 @@ __device__ __forceinline__ void xlamb_fx_group(const XformArgs &a, const size_t 
       A == B ? tw : tw + A * B, bd, sc, pk, ok);
   __syncthreads();
   // 5. forward pass 2 into line q
-  if (q < NF && t < B) fx_x_pass2_fwd<CLS>(p, t, R + (NF + q) * LS, R + q * LS);
+  fx_x_pass2_fwd<CLS>(p, q < NF && t < B, t, R + (NF + q) * LS, R + q * LS);
   __syncthreads();
   // 6. unpack the real-pair spectra, keep kx < NXH, scale by 1/NX2:
   // Xa = (Z[m] + conj Z[-m]) / 2 ; Xb = (Z[m] - conj Z[-m]) / (2i)
   double2 *lb = reinterpret_cast<double2 *>(a.lbuf);
   const double half = 0.5 * a.inv_nx2;
-  for (int idx = threadIdx.x; idx < P * d.NXH; idx += blockDim.x) {
-    const int l = idx / d.NXH, km = idx - l * d.NXH;
-    const size_t line = line0 + l;
-    if (line >= nlines) continue;
+  for (int idx = threadIdx.x; idx < H * d.NXH; idx += blockDim.x) {
+    const int h = idx / d.NXH, km = idx - h * d.NXH;
+    const FxPair pr = fx_pair(d, pair0 + h);
+    if (!pr.have) continue;
     const int mc = (km == 0) ? 0 : d.NX2 - km;
-    {
-      const double w = half * fx_factor(sc[l]);
-      const fxc zm = R[l * LS + km], zc = R[l * LS + mc];
-      lb[line * d.NXH + km] =
-          make_double2(__dmul_rn(__ll2double_rn(zm.x + zc.x), w), __dmul_rn(__ll2double_rn(zm.y - zc.y), w));
-      lb[fstride + line * d.NXH + km] =
-          make_double2(__dmul_rn(__ll2double_rn(zm.y + zc.y), w), __dmul_rn(__ll2double_rn(zc.x - zm.x), w));
-    }
-    {
-      const double w = half * fx_factor(sc[P + l / 2]);
-      const fxc zm = R[(P + l / 2) * LS + km], zc = R[(P + l / 2) * LS + mc];
-      const long long vx = (l & 1) ? zm.y + zc.y : zm.x + zc.x, vy = (l & 1) ? zc.x - zm.x : zm.y - zc.y;
-      lb[2 * fstride + line * d.NXH + km] =
-          make_double2(__dmul_rn(__ll2double_rn(vx), w), __dmul_rn(__ll2double_rn(vy), w));
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double w = half * fx_factor(sc[c * H + h]);
+      const fxc zm = R[(c * H + h) * LS + km], zc = R[(c * H + h) * LS + mc];
+      double2 *o = lb + (size_t)c * fstride + pr.line * d.NXH + km;
+      o[0] = make_double2(__dmul_rn(__ll2double_rn(zm.x + zc.x), w), __dmul_rn(__ll2double_rn(zm.y - zc.y), w));
+      if (pr.have_b)
+        o[d.NXH] = make_double2(__dmul_rn(__ll2double_rn(zm.y + zc.y), w), __dmul_rn(__ll2double_rn(zc.x - zm.x), w));
     }
   }
 }
 
-// Fetch the input lines line0 .. line0 + P - 1 of the six fields into L2.
-template <int P>
-__device__ __forceinline__ void fx_prefetch_lines(const XformArgs &a, size_t line0) {
-  const size_t nlines = (size_t)a.d.NY * a.d.NZ2, fstride = nlines * a.d.NXH;
-  const int nl = nlines - line0 < (size_t)P ? (int)(nlines - line0) : P;
+// Fetch the input lines of the pairs pair0 .. pair0 + PAIRS - 1 of the six
+// fields into L2 (consecutive in memory: a plane's last line is followed by the
+// next plane's first).
+template <int PAIRS>
+__device__ __forceinline__ void fx_prefetch_lines(const XformArgs &a, unsigned pair0) {
+  const size_t fstride = (size_t)a.d.NY * a.d.NZ2 * a.d.NXH;
+  const FxPair first = fx_pair(a.d, pair0);
+  FxPair last = fx_pair(a.d, pair0 + PAIRS - 1);
+  if (!last.have) last = first;
+  const int nl = first.have ? (int)(last.line - first.line) + (last.have_b ? 2 : 1) : 0;
   const int per = (nl * a.d.NXH + 7) / 8;  // 128-byte lines per field
   for (int idx = threadIdx.x; idx < 6 * per; idx += blockDim.x) {
     const int f = idx / per, o = idx - f * per;
-    const double2 *src = reinterpret_cast<const double2 *>(a.zbuf) + (size_t)f * fstride + line0 * a.d.NXH + 8 * o;
+    const double2 *src =
+        reinterpret_cast<const double2 *>(a.zbuf) + (size_t)f * fstride + first.line * a.d.NXH + 8 * o;
     asm volatile("prefetch.global.L2 [%0];" ::"l"(src));
   }
 }
 
-// The groups g0, g0 + step, ... < ngroups; args(g, line0) gives the arguments
-// and first line of group g (several channels, all of one plan, in the batch).
+// The groups g0, g0 + step, ... < ngroups; args(g, pair0) gives the arguments
+// and first pair of group g (several channels, all of one plan, in the batch).
 template <int CLS, class Args>
 __device__ __forceinline__ void xlamb_fx_run(int g0, int step, int ngroups, Args args) {
   constexpr int P = FxCfg<CLS>::P;
   extern __shared__ __align__(16) unsigned char smraw[];
-  size_t line0;
-  const XformArgs &a0 = args(g0 < ngroups ? g0 : 0, line0);
+  unsigned pair0;
+  const XformArgs &a0 = args(g0 < ngroups ? g0 : 0, pair0);
   const int A = a0.fpx.A, B = a0.fpx.B;
   fxc *R = reinterpret_cast<fxc *>(smraw);
   FxTw *tw = reinterpret_cast<FxTw *>(R + 3 * P * fx_xline(A, B));
   const int ntw = fx_xtables(A, B);
   FxBound *bd = reinterpret_cast<FxBound *>(tw + ntw);
   FxScale *sc = reinterpret_cast<FxScale *>(bd + 3 * P * FxCfg<CLS>::T);
+  unsigned *mag = reinterpret_cast<unsigned *>(sc + 3 * P);
   for (int k = threadIdx.x; k < ntw; k += blockDim.x) tw[k] = a0.fxx[k];
   for (int g = g0; g < ngroups; g += step) {
     __syncthreads();  // the last group's spectra are read (the first: the table is written)
-    const XformArgs &ag = args(g, line0);
+    const XformArgs &ag = args(g, pair0);
     if (g + step < ngroups) {
-      size_t nline0;
-      const XformArgs &an = args(g + step, nline0);
-      fx_prefetch_lines<P>(an, nline0);
+      unsigned npair0;
+      const XformArgs &an = args(g + step, npair0);
+      fx_prefetch_lines<P / 2>(an, npair0);
     }
-    xlamb_fx_group<CLS>(ag, line0, R, tw, bd, sc);
+    xlamb_fx_group<CLS>(ag, pair0, R, tw, bd, sc, mag);
   }
 }
 
@@ -465,10 +475,9 @@ template <int CLS>
 __global__ void __launch_bounds__(3 * FxCfg<CLS>::P *FxCfg<CLS>::T, FxCfg<CLS>::XB)
     k_xlamb_fx(const __grid_constant__ XformArgs a) {
   constexpr int P = FxCfg<CLS>::P;
-  const int ngroups = (int)(((size_t)a.d.NY * a.d.NZ2 + P - 1) / P);
   const XformArgs *pa = &a;
-  xlamb_fx_run<CLS>(blockIdx.x, gridDim.x, ngroups, [pa](int g, size_t &line0) -> const XformArgs & {
-    line0 = (size_t)g * P;
+  xlamb_fx_run<CLS>(blockIdx.x, gridDim.x, fx_groups(a.d, P), [pa](int g, unsigned &pair0) -> const XformArgs & {
+    pair0 = (unsigned)g * (P / 2);
     return *pa;
   });
 }
@@ -493,9 +502,9 @@ __global__ void __launch_bounds__(FxCfg<CLS>::TX *FxCfg<CLS>::T, FxCfg<CLS>::ZB)
 template <int CLS>
 __global__ void __launch_bounds__(3 * FxCfg<CLS>::P *FxCfg<CLS>::T, FxCfg<CLS>::XB)
     k_xlamb_fx_batch(const __grid_constant__ BatchTable<XformArgs> t) {
-  xlamb_fx_run<CLS>(blockIdx.x, gridDim.x, t.start[t.n], [&](int g, size_t &line0) -> const XformArgs & {
+  xlamb_fx_run<CLS>(blockIdx.x, gridDim.x, t.start[t.n], [&](int g, unsigned &pair0) -> const XformArgs & {
     const int c = batch_channel(t.start, t.n, g);
-    line0 = (size_t)(g - t.start[c]) * FxCfg<CLS>::P;
+    pair0 = (unsigned)(g - t.start[c]) * (FxCfg<CLS>::P / 2);
     return t.a[c];
   });
 }
