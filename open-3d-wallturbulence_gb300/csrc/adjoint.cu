@@ -20,7 +20,7 @@
 //               with u_p, om_p the step's physical fields recomputed from its
 //               spectral fields (the recompute tape).
 //  k_adj_mean   solve_mean^T + solve_friction_force^T (one block).
-//  k_adj_modes  mode kernel^T: solve_horizontal^T, then transposed solves of
+//  k_adj_modes  mode kernel^T (adjoint_modes.cu): solve_horizontal^T, then transposed solves of
 //               the augmented v- and omega_y-systems on the forward factors,
 //               and the source assembly^T into the three history levels.  The
 //               transposed v solve also yields d objective / d v_w from the
@@ -359,165 +359,6 @@ __global__ void k_adj_mean(AdjMeanArgs a) {
 }
 
 void launch_adj_mean(const AdjMeanArgs &a, cudaStream_t st) { k_adj_mean<<<1, 32, 0, st>>>(a); }
-
-// ---------------------------------------------------------------------------
-// Mode kernel adjoint, two threads per real component of a mode (one per system).
-// ---------------------------------------------------------------------------
-// VMODE: the v-system's transposed solve over the full band (0) or inside
-// the interior masks the setup check admitted (1: VMasks, 2: VMasks6).
-// Blocks of two warps serve 16 modes (both real components): warp 0 the
-// v-system's part (its inputs from solve_horizontal^T, the transposed v
-// solve, the v, DY2 v and Hv histories), warp 1 the omega_y-system's (its
-// inputs, the transposed omega_y solve, the g and Hg histories).  The two
-// parts read and write disjoint data, so they need no synchronisation, and
-// each value comes from the same operations as in one thread doing both.
-template <int KLV, int KUV, int KLG, int KUG, int VMODE>
-__global__ void __launch_bounds__(64) k_adj_modes(AdjModeArgs a) {
-  const int role = threadIdx.x >> 5;  // 0: v-system, 1: omega_y-system
-  const int tid = blockIdx.x * 32 + (threadIdx.x & 31);
-  const int m = tid >> 1, comp = tid & 1;
-  if (m >= a.M) return;
-  const int M = a.M, NY = a.NY;
-  const int k = m / a.NXH, i = m - k * a.NXH;
-  const int kabs = (k <= a.NZH) ? k : a.NZ - k;
-  const int u = kabs * a.NXH + i;
-  const double kx = a.kx[i], kz = a.kz[k];
-  const double k2 = kx * kx + kz * kz;
-  const bool horiz = !(k2 < 1.e-8);
-  const double ik2 = horiz ? 1.0 / k2 : 0.0;
-  const double ax = kx * ik2, az = kz * ik2;
-  const double icg = a.inv_cg[u], nu = a.nu, idt = a.inv_dt;
-  const double al0 = 3.0, al1 = -1.5, al2 = 1.0 / 3.0, be0 = 3.0, be1 = -3.0, be2 = 1.0;
-  auto E = [&](int j) { return 2 * ((size_t)j * M + m) + comp; };
-  auto D = [](double2 *p) { return reinterpret_cast<double *>(p); };
-  auto cmp = [&](double2 v) { return comp ? v.y : v.x; };
-  // level 1 += c0 s, level 2 += c1 s, level 0 = c2 s
-  auto upd = [&](double2 *const *f, int j, double s, double c0, double c1, double c2) {
-    const size_t e = E(j);
-    D(f[1])[e] += c0 * s;
-    D(f[2])[e] += c1 * s;
-    D(f[0])[e] = c2 * s;
-  };
-
-  // 1. solve_horizontal^T and the adjoints of the solves' outputs per node:
-  //    v, D1 v (through DY1 v = c11 d1, DY2 v = c21 d1 + c22 d2), g, D1 g
-  //    (each warp the part its system reads)
-  for (int j = 0; j < NY; ++j) {
-    const bool in = j != 0 && j != NY - 1;
-    const size_t at = (size_t)j * M + m;
-    const double c11 = a.c11[j], c21 = a.c21[j], c22 = a.c22[j];
-    const size_t e = E(j);
-    if (role == 0) {
-      double2 vt = a.v[0][at], qt = a.q[0][at];
-      const double2 vf = a.vb[at];
-      vt.x += vf.x; vt.y += vf.y;
-      double2 dv = make_double2(0.0, 0.0);
-      if (horiz) {
-        const double2 ub = a.ub[at], wb = a.wb[at], oxb = a.oxb[at], ozb = a.ozb[at];
-        // adjoints of u = i ax DY1v - i az g, w = i ax g + i az DY1v,
-        // om_x = i/k2 (kx DY1g + kz DY2v) - i kz v, om_z = i/k2 (kz DY1g - kx DY2v) + i kx v
-        dv = make_double2(ax * ub.y + az * wb.y, -ax * ub.x - az * wb.x);
-        qt.x += az * oxb.y - ax * ozb.y;
-        qt.y += -az * oxb.x + ax * ozb.x;
-        vt.x += -kz * oxb.y + kx * ozb.y;
-        vt.y += kz * oxb.x - kx * ozb.x;
-      }
-      const double v_ = cmp(vt), q_ = cmp(qt), dv_ = cmp(dv);
-      D(a.xv0)[e] = v_;
-      D(a.xv1)[e] = a.inv_h * (c11 * dv_ + c21 * q_);
-      D(a.xv2)[e] = a.inv_h2 * c22 * q_;
-    } else {
-      double2 gt = a.g[0][at];
-      const double2 gf = a.gb[at];
-      gt.x += gf.x; gt.y += gf.y;
-      double2 dg = make_double2(0.0, 0.0);
-      if (horiz) {
-        const double2 ub = a.ub[at], wb = a.wb[at], oxb = a.oxb[at], ozb = a.ozb[at];
-        gt.x += -az * ub.y + ax * wb.y;
-        gt.y += az * ub.x - ax * wb.x;
-        dg = make_double2(ax * oxb.y + az * ozb.y, -ax * oxb.x - az * ozb.x);
-      }
-      const double g_ = cmp(gt), dg_ = cmp(dg);
-      D(a.xg0)[e] = a.inv_h * (c11 * dg_ + (in ? nu * c21 * icg * g_ : 0.0));
-      D(a.xg1)[e] = in ? a.inv_h2 * nu * c22 * icg * g_ : 0.0;
-      D(a.sgb)[e] = in ? icg * g_ : 0.0;
-    }
-  }
-
-  // 2. v-system^T: the source adjoint is scattered through the rows' rhs
-  //    tables, then feeds Hv, v, DY2 v of the three levels; the two wall
-  //    rows give the wall-velocity gradient
-  if (role == 0) {
-    for (int j = 0; j < NY; ++j) D(a.svb)[E(j)] = 0.0;
-    auto rhs = [&](int c) -> double {
-      int t, jn;
-      vcol_split(c, NY, t, jn);
-      if (t == 0) return D(a.xv0)[E(jn)];
-      if (t == 1) return D(a.xv1)[E(jn)];
-      if (t == 2) return D(a.xv2)[E(jn)];
-      return 0.0;
-    };
-    auto ys = [&](int p, double y) { D(a.yv)[E(p)] = y; };
-    auto yl = [&](int p) -> double { return D(a.yv)[E(p)]; };
-    auto out = [&](int p, double z) {
-      const double r = z * a.rs_v[(size_t)p * a.U + u];
-      const int tag = a.rhs_node_v[p];
-      if (tag == kRhsTable) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const double b = a.rbv_val[p * 4 + q];
-          if (nonzero(b)) D(a.svb)[E(a.rbv_col[p * 4 + q])] += b * r;
-        }
-      } else if (tag == kRhsWallBottom) {
-        D(a.grad)[2 * (size_t)m + comp] += r;
-      } else if (tag == kRhsWallTop) {
-        D(a.grad)[2 * ((size_t)M + m) + comp] += r;
-      }
-    };
-    if constexpr (VMODE == 1)
-      band_solve_t_masked<KLV, KUV, 4, 2, VMasks>(a.ab_v, a.piv_v, a.n_v, a.U, u, rhs, ys, yl, out);
-    else if constexpr (VMODE == 2)
-      band_solve_t_masked<KLV, KUV, 4, 2, VMasks6>(a.ab_v, a.piv_v, a.n_v, a.U, u, rhs, ys, yl, out);
-    else
-      band_solve_t<KLV, KUV>(a.ab_v, a.piv_v, a.n_v, a.U, u, rhs, ys, yl, out);
-    // source_v = sum beta Hv_l - k^2/dt sum alpha v_l + sum alpha q_l / dt on
-    // nodes 2..NY-3; the tables reference no other node, so svb is zero there
-    for (int j = 0; j < NY; ++j) {
-      const double r = D(a.svb)[E(j)];
-      upd(a.hv, j, r, be0, be1, be2);
-      upd(a.v, j, -k2 * idt * r, al0, al1, al2);
-      upd(a.q, j, idt * r, al0, al1, al2);
-    }
-  }
-
-  // 3. omega_y-system^T: source adjoint scattered through the B rows
-  else {
-    auto rhs = [&](int c) -> double { return (c & 1) ? D(a.xg1)[E(c >> 1)] : D(a.xg0)[E(c >> 1)]; };
-    auto ys = [&](int p, double y) { D(a.yg)[E(p)] = y; };
-    auto yl = [&](int p) -> double { return D(a.yg)[E(p)]; };
-    auto out = [&](int p, double z) {
-      const double r = z * icg * a.rs_g[(size_t)p * a.U + u];
-#pragma unroll
-      for (int e = 0; e < 5; ++e) {
-        const double b = a.rb_val[p * 5 + e];
-        if (nonzero(b)) D(a.sgb)[E(a.rb_col[p * 5 + e])] += b * r;
-      }
-    };
-    band_solve_t<KLG, KUG>(a.ab_g, a.piv_g, a.n_g, a.U, u, rhs, ys, yl, out);
-    for (int j = 0; j < NY; ++j) {
-      const double s = D(a.sgb)[E(j)];
-      upd(a.hg, j, s, be0, be1, be2);
-      upd(a.g, j, idt * s, al0, al1, al2);
-    }
-  }
-}
-
-void launch_adj_modes(const AdjModeArgs &a, int vmode, cudaStream_t st) {
-  const int grid = (2 * a.M + 31) / 32;  // 16 modes (32 real components) a block of two warps
-  if (vmode == 1) k_adj_modes<kVKL, kVKU, 6, 6, 1><<<grid, 64, 0, st>>>(a);
-  else if (vmode == 2) k_adj_modes<kVKL, kVKU, 6, 6, 2><<<grid, 64, 0, st>>>(a);
-  else k_adj_modes<kVKL, kVKU, 6, 6, 0><<<grid, 64, 0, st>>>(a);
-}
 
 // ---------------------------------------------------------------------------
 __global__ void k_objective_add(const double *fx_ring, const long long *step, double weight, double *acc) {

@@ -74,25 +74,28 @@ struct AdjMeanArgs {
 
 // Adjoint of the mode kernel (both implicit solves and solve_horizontal).
 struct AdjModeArgs {
-  int NY, NZ, NXH, NZH, M, U;
+  int NY, NZ, NXH, NZH, M, U, u0, u1;  // u0, u1: 0, U
   double inv_dt, nu, inv_h, inv_h2;
   const double *kx, *kz, *c11, *c21, *c22, *inv_cg;
   const double *ab_v; const uint8_t *piv_v; int n_v; const int *rhs_node_v; const double *rs_v;
-  const int *rbv_col; const double *rbv_val;  // v-system rhs tables [n_v][4]
-  const double *ab_g; const uint8_t *piv_g; int n_g; const int *rb_col; const double *rb_val; const double *rs_g;
+  const double *ab_g; const uint8_t *piv_g; int n_g; const double *rs_gi;
+  // the right-hand sides' rows by their last node, as ModeArgs; the packed
+  // streams of the factors and the row scales in the rows' order
+  const int *vptr, *gptr;
+  const StrRow *vrows, *grows;
+  StrBuffers str;
   const double2 *ub, *vb, *wb, *oxb, *gb, *ozb;  // adjoint fields from the Lamb vector
   double2 *v[3], *g[3], *hv[3], *hg[3], *q[3];   // adjoint histories [NY][M]
   double2 *grad;          // [2][M] accumulated d objective / d v_w (bottom, top)
-  double2 *yv, *yg;       // scratch [n_v][M], [n_g][M]
-  double2 *xv0, *xv1, *xv2, *xg0, *xg1, *sgb, *svb;  // scratch [NY][M]
+  double2 *yv, *yg, *sgb;  // scratch rows [n_v], [n_g], [NY] of max(M, str_scratch_values(U)) values
 };
 
 void launch_adj_nl(const AdjNLArgs &a, cudaStream_t st);
 cudaError_t adj_lamb_prepare(const XformDims &d);
 void launch_adj_lamb(const AdjXformArgs &a, cudaStream_t st);  // three launches
 void launch_adj_mean(const AdjMeanArgs &a, cudaStream_t st);
-// vmode: 0 full band, 1 / 2 the v-system's transposed solve inside the
-// eighth- / sixth-order interior masks (only where the setup check passed)
+// vmode: 0 full band, 1 / 2 on the packed streams of the eighth- / sixth-order
+// interior masks (only where the setup check passed)
 void launch_adj_modes(const AdjModeArgs &a, int vmode, cudaStream_t st);
 void launch_objective_add(const double *fx_ring, const long long *step, double weight, double *acc,
                           cudaStream_t st);

@@ -73,8 +73,10 @@ void owt_handle::adj_alloc() {
   const XformDims xd{NY, NZ, NXH, NZH, NX2, NZ2};
   adj.zbuf = dalloc<double2>(adj_zbuf_values(xd), owned);
   adj.lbuf = dalloc<double2>(adj_lbuf_values(xd), owned);
-  adj.yv = dalloc<double2>((size_t)bv.n * M, owned);
-  adj.yg = dalloc<double2>((size_t)bg.n * M, owned);
+  const size_t row = std::max((size_t)M, str_scratch_values(Uq));
+  adj.yv = dalloc<double2>((size_t)bv.n * row, owned);
+  adj.yg = dalloc<double2>((size_t)bg.n * row, owned);
+  adj.sgb = dalloc<double2>((size_t)NY * row, owned);
   adj.mscr = dalloc<double2>(2 * (3 * (size_t)NY + bg.n), owned);
   adj.grad = dalloc<double2>(2 * (size_t)M, owned);
   ck(adj_lamb_prepare(xd), "adjoint transform kernel attributes");
@@ -122,20 +124,18 @@ void owt_handle::adjoint_step(const double2 *tp, double wgt) {
   ck(cudaEventRecord(ev_join, st2), "join");
 
   AdjModeArgs mo{};
-  mo.NY = NY; mo.NZ = NZ; mo.NXH = NXH; mo.NZH = NZH; mo.M = M; mo.U = Uq;
+  mo.NY = NY; mo.NZ = NZ; mo.NXH = NXH; mo.NZH = NZH; mo.M = M; mo.U = Uq; mo.u0 = 0; mo.u1 = Uq;
   mo.inv_dt = 1.0 / p.dt; mo.nu = p.nu; mo.inv_h = 1.0 / grid.ds; mo.inv_h2 = 1.0 / (grid.ds * grid.ds);
   mo.kx = kx; mo.kz = kz; mo.c11 = c11; mo.c21 = c21; mo.c22 = c22; mo.inv_cg = inv_cg;
   mo.ab_v = bv.ab; mo.piv_v = bv.piv; mo.n_v = bv.n; mo.rhs_node_v = rhs_node_v; mo.rs_v = bv.rscale;
-  mo.rbv_col = rbv_col; mo.rbv_val = rbv_val;
-  mo.ab_g = bg.ab; mo.piv_g = bg.piv; mo.n_g = bg.n; mo.rb_col = rb_col; mo.rb_val = rb_val; mo.rs_g = bg.rscale;
+  mo.ab_g = bg.ab; mo.piv_g = bg.piv; mo.n_g = bg.n; mo.rs_gi = rs_gi;
+  mo.vptr = vptr; mo.gptr = gptr; mo.vrows = vrows; mo.grows = grows; mo.str = str;
   mo.ub = adj.fb[0]; mo.vb = adj.fb[1]; mo.wb = adj.fb[2]; mo.oxb = adj.fb[3]; mo.gb = adj.fb[4]; mo.ozb = adj.fb[5];
   for (int l = 0; l < 3; ++l) {
     mo.v[l] = adj.hist[0][l]; mo.g[l] = adj.hist[1][l]; mo.hv[l] = adj.hist[2][l];
     mo.hg[l] = adj.hist[3][l]; mo.q[l] = adj.hist[4][l];
   }
-  mo.grad = adj.grad; mo.yv = adj.yv; mo.yg = adj.yg;
-  mo.xv0 = adj.xs[0]; mo.xv1 = adj.xs[1]; mo.xv2 = adj.xs[2]; mo.xg0 = adj.xs[3]; mo.xg1 = adj.xs[4];
-  mo.sgb = adj.xs[5]; mo.svb = adj.xs[6];
+  mo.grad = adj.grad; mo.yv = adj.yv; mo.yg = adj.yg; mo.sgb = adj.sgb;
   launch_adj_modes(mo, force_dense ? 0 : sparse_v ? 1 : sparse_v6 ? 2 : 0, st);
   ck(cudaStreamWaitEvent(st, ev_join, 0), "join wait");
   launches += 6;
@@ -152,6 +152,7 @@ void owt_handle::drag_backward(double gJ, double *grad_bottom, double *grad_top)
   if (adj.nsteps == 0 || adj.version != state_version)
     throw OwtError(OWT_ERR_STATE, "owt_drag_forward must come first, with no change of state or wall velocity since");
   adj_alloc();
+  build_streams();
   if (adj.tape_len < adj.interval) {
     if (adj.tape) free_owned(adj.tape);
     adj.tape = nullptr;

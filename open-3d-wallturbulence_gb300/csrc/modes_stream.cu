@@ -7,6 +7,14 @@
 namespace owt {
 
 namespace {
+// rs[p] of the listed rows, in their order
+__global__ void k_str_row_scales(double *__restrict__ out, const double *__restrict__ rs, const StrRow *__restrict__ rows,
+                                 int U) {
+  const double *src = rs + (size_t)rows[blockIdx.y].p * U;
+  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < U; u += gridDim.x * blockDim.x)
+    out[(size_t)blockIdx.y * U + u] = src[u];
+}
+
 struct Variant {
   const char *name;
   void (*kernel)(ModeArgs), (*sixth)(ModeArgs);

@@ -135,14 +135,6 @@ __global__ void k_str_pack(const double *__restrict__ ab, const uint8_t *__restr
   }
 }
 
-// rs[p] of the listed rows, in their order
-__global__ void k_str_row_scales(double *__restrict__ out, const double *__restrict__ rs, const StrRow *__restrict__ rows,
-                                 int U) {
-  const double *src = rs + (size_t)rows[blockIdx.y].p * U;
-  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < U; u += gridDim.x * blockDim.x)
-    out[(size_t)blockIdx.y * U + u] = src[u];
-}
-
 __device__ __forceinline__ void str_copy16(void *smem, const void *g) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(g));
@@ -187,6 +179,20 @@ struct StrFeed {
     const double *p = ring + get * SLOT;
     get = get == kStrSlots - 1 ? 0 : get + 1;
     return p;
+  }
+};
+
+// The same for the transposed solves, which read a sweep's stream from its end:
+// units in descending order.
+template <int SLOT>
+struct StrFeedBack : StrFeed<SLOT> {
+  using Base = StrFeed<SLOT>;
+  __device__ __forceinline__ StrFeedBack(const double *end, double *r, int ln) : Base(end, r, ln) {}
+  template <int SIZE>
+  __device__ __forceinline__ void fetch() {
+    this->next -= SIZE;
+    Base::template fetch<SIZE>();
+    this->next -= SIZE;
   }
 };
 
@@ -371,7 +377,8 @@ struct StrLane {
   int m, comp, u, lane;
   bool active;
 };
-__device__ __forceinline__ StrLane str_lane(const ModeArgs &a, int warp, int lane) {
+template <class Args>
+__device__ __forceinline__ StrLane str_lane(const Args &a, int warp, int lane) {
   StrLane l;
   l.lane = lane;
   l.comp = lane & 1;
