@@ -37,52 +37,147 @@
 namespace owt {
 
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_adj_nl(AdjNLArgs a) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= a.M) return;
-  const int M = a.M, NY = a.NY;
+// One thread per real component of a mode, as the nonlinear source (solve.cu):
+// one sweep up with U^T, one down with L^T, B_1^T on the last seven solved rows
+// and the outputs.  Bound by FP64 issue (18 operations a node and component);
+// the operator tables of a block are in shared memory, what a row reads from
+// memory is fetched four rows ahead.  128x129x128, one thread a mode, the solve
+// and B_1^T through memory -> here: 0.404 -> 0.215 ms.
+constexpr int kANLThreads = 64, kANLThreadsLarge = 256;
+// per row: U's column from the diagonal (5), L (2), c11, B_1's column (7 rows)
+constexpr int kANLRow = 15;
+constexpr size_t adj_nl_smem(int NY) { return (size_t)NY * (kANLRow * sizeof(double) + 1) + 8; }
+constexpr size_t kANLSmem = 220 * 1024;  // larger tables are read from device memory
+
+template <bool SMEM>
+__global__ void __launch_bounds__(kANLThreadsLarge) k_adj_nl(const __grid_constant__ AdjNLArgs a) {
+  const int M = a.M, NY = a.NY, n = NY - 1, tid = blockIdx.x * blockDim.x + threadIdx.x;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double *tab = reinterpret_cast<double *>(smraw);
+  uint8_t *spiv = reinterpret_cast<uint8_t *>(tab + (size_t)NY * kANLRow);
+  auto b1t = [&](int j, int r) {  // B_1(j + r, j)
+    double b = 0.0;
+    for (int e = 0; e < 8; ++e)
+      if (a.b1t_col[j * 8 + e] == j + r && nonzero(a.b1t_val[j * 8 + e])) b = a.b1t_val[j * 8 + e];
+    return b;
+  };
+  auto band = [&](int row, int j) { return a.ab1[(size_t)row * NY + j]; };  // LAPACK layout, KV = 4
+  if (SMEM) {
+    for (int e = threadIdx.x; e < NY * kANLRow; e += blockDim.x) {
+      const int j = e / kANLRow, q = e - j * kANLRow;
+      tab[e] = q < 5 ? band(4 - q, j) : q < 7 ? band(q, j) : q == 7 ? a.c11[j] : b1t(j, q - 11);
+    }
+    for (int j = threadIdx.x; j < NY; j += blockDim.x) spiv[j] = a.piv1[j];
+    __syncthreads();
+  }
+  auto up = [&](int j, int t) { return SMEM ? tab[j * kANLRow + t] : band(4 - t, j); };
+  auto lo = [&](int j, int t) { return SMEM ? tab[j * kANLRow + 4 + t] : band(4 + t, j); };
+  auto c11 = [&](int j) { return SMEM ? tab[j * kANLRow + 7] : a.c11[j]; };
+  auto bt = [&](int j, int r) { return SMEM ? tab[j * kANLRow + 11 + r] : b1t(j, r); };
+  auto piv = [&](int j) { return SMEM ? (int)spiv[j] : (int)a.piv1[j]; };
+  const int m = tid >> 1, comp = tid & 1;
+  if (m >= M) return;
   const int k = m / a.NXH, i = m - k * a.NXH;
   const double kx = a.kx[i], kz = a.kz[k];
-  const double k2 = kx * kx + kz * kz;
-  // w = A_1^-T (c11 .* Hv_bar)
-  auto rhs = [&](int p) -> double2 {
-    const double2 h = a.hvb[(size_t)p * M + m];
-    const double c = a.c11[p];
-    return make_double2(c * h.x, c * h.y);
-  };
-  auto ys = [&](int p, double2 y) { a.ys[(size_t)p * M + m] = y; };
-  auto yl = [&](int p) -> double2 { return a.ys[(size_t)p * M + m]; };
-  auto out = [&](int c, double2 x) { a.ws[(size_t)c * M + m] = x; };
-  band_solve_t<2, 2>(a.ab1, a.piv1, NY, 1, 0, rhs, ys, yl, out);
-  for (int j = 0; j < NY; ++j) {
-    // q = B_1^T w  (so that the adjoint of f = i kx lx + i kz lz is -q)
-    double2 q = make_double2(0.0, 0.0);
+  const double k2 = fma(kx, kx, kz * kz);
+  const double sgn = comp ? 1.0 : -1.0;  // component c of z gives component 1 - c of -+ i z
+  const double skx = sgn * kx, skz = sgn * kz;
+  const size_t ld = 2 * (size_t)M;
+  const double *hv = reinterpret_cast<const double *>(a.hvb) + tid, *hg = reinterpret_cast<const double *>(a.hgb) + tid;
+  double *y = reinterpret_cast<double *>(a.ys) + tid;
+  double *lx = reinterpret_cast<double *>(a.lxb) + 2 * (size_t)m + 1 - comp;
+  double *lz = reinterpret_cast<double *>(a.lzb) + 2 * (size_t)m + 1 - comp;
+  double *ly = reinterpret_cast<double *>(a.lyb) + tid;
+  auto at = [&](int j) { return (size_t)(j < n ? (j > 0 ? j : 0) : n) * ld; };
+  {
+    // U^T y = c11 Hv_bar
+    double h[4] = {0.0, 0.0, 0.0, 0.0}, nx[4];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const double b = a.b1t_val[j * 8 + e];
-      if (nonzero(b)) {
-        const double2 x = a.ws[(size_t)a.b1t_col[j * 8 + e] * M + m];
-        q.x += b * x.x;
-        q.y += b * x.y;
+    for (int q = 0; q < 4; ++q) nx[q] = hv[at(q)];
+#pragma unroll 4
+    for (int c = 0; c <= n; ++c) {
+      double acc = c11(c) * nx[0];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) nx[q] = nx[q + 1];
+      nx[3] = hv[at(c + 4)];
+#pragma unroll
+      for (int t = 1; t <= 4; ++t) fms(acc, up(c, t), h[t - 1]);
+      acc *= up(c, 0);
+      y[(size_t)c * ld] = acc;
+#pragma unroll
+      for (int t = 3; t > 0; --t) h[t] = h[t - 1];
+      h[0] = acc;
+    }
+  }
+  // L^T and the interchanges: b0 .. b2 the entries c .. c + 2, of which c + 2 is
+  // final after column c; w: the last seven final rows, c + 2 .. c + 8; node
+  // c + 5 goes out
+  double b0 = 0.0, b1 = 0.0, b2 = 0.0, w[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, ny[4], ng[4], nv[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    ny[q] = y[at(n - q)];
+    ng[q] = hg[at(n - q)];
+    nv[q] = hv[at(n - q)];
+  }
+#pragma unroll 4
+  for (int c = n; c >= -5; --c) {
+    b2 = b1;
+    b1 = b0;
+    b0 = 0.0;
+    if (c >= 0) {
+      b0 = ny[0];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) ny[q] = ny[q + 1];
+      ny[3] = y[at(c - 4)];
+      fms(b0, lo(c, 1), b1);
+      fms(b0, lo(c, 2), b2);
+      const int off = piv(c);
+      if (off == 1) {
+        const double q = b0; b0 = b1; b1 = q;
+      } else if (off == 2) {
+        const double q = b0; b0 = b2; b2 = q;
       }
     }
-    const size_t at = (size_t)j * M + m;
-    const double2 hg = a.hgb[at], hv = a.hvb[at];
+#pragma unroll
+    for (int q = 6; q > 0; --q) w[q] = w[q - 1];
+    w[0] = b2;
+    const int j = c + 5;
+    if (j > n) continue;
+    // q = B_1^T w, so that the adjoint of f = i kx lx + i kz lz is -q; the rows
+    // further than two off reach only the nodes at the walls
+    double q = 0.0;
+    if (j <= 3) q = bt(j, -3) * w[0];
+    q = fma(bt(j, -2), w[1], q);
+    q = fma(bt(j, -1), w[2], q);
+    if (j == 0 || j == n) q = fma(bt(j, 0), w[3], q);
+    q = fma(bt(j, 1), w[4], q);
+    q = fma(bt(j, 2), w[5], q);
+    if (j >= n - 3) q = fma(bt(j, 3), w[6], q);
     // lx_bar = -i kz Hg_bar + i kx q ; ly_bar = -k^2 Hv_bar ; lz_bar = i kx Hg_bar + i kz q
-    double2 bx = make_double2(kz * hg.y - kx * q.y, -kz * hg.x + kx * q.x);
-    double2 bz = make_double2(-kx * hg.y - kz * q.y, kx * hg.x + kz * q.x);
+    double bx = fma(skz, ng[0], -(skx * q)), bz = -fma(skx, ng[0], skz * q);
     if (m == 0) {
-      bx.x += a.lxmb[j].x; bx.y += a.lxmb[j].y;
-      bz.x += a.lzmb[j].x; bz.y += a.lzmb[j].y;
+      bx += reinterpret_cast<const double *>(a.lxmb)[2 * j + 1 - comp];
+      bz += reinterpret_cast<const double *>(a.lzmb)[2 * j + 1 - comp];
     }
-    a.lxb[at] = bx;
-    a.lyb[at] = make_double2(-k2 * hv.x, -k2 * hv.y);
-    a.lzb[at] = bz;
+    const size_t o = (size_t)j * ld;
+    lx[o] = bx;
+    ly[o] = -k2 * nv[0];
+    lz[o] = bz;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      ng[r] = ng[r + 1];
+      nv[r] = nv[r + 1];
+    }
+    ng[3] = hg[at(j - 4)];
+    nv[3] = hv[at(j - 4)];
   }
 }
 
 void launch_adj_nl(const AdjNLArgs &a, cudaStream_t st) {
-  k_adj_nl<<<(a.M + 127) / 128, 128, 0, st>>>(a);
+  const int bs = 2 * a.M >= 152 * 4 * kANLThreadsLarge ? kANLThreadsLarge : kANLThreads, gs = (2 * a.M + bs - 1) / bs;
+  const size_t b = adj_nl_smem(a.NY);
+  if (b <= kANLSmem) k_adj_nl<true><<<gs, bs, b, st>>>(a);
+  else k_adj_nl<false><<<gs, bs, 0, st>>>(a);
 }
 
 // ---------------------------------------------------------------------------
@@ -280,85 +375,110 @@ void launch_adj_lamb(const AdjXformArgs &a, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
-// Mean mode.  Thread 0: U (with fx), thread 1: W (with fz).  Forward:
+// Mean mode: U (with fx) and W (with fz).  Forward:
 //   s_j = sum_l beta_l (L_l,j + f_l) + sum_l alpha_l U_l,j / dt   (interior j)
 //   U = solve(s) by the omega_y-system of mode (0, 0), dU = c11 d1
 //   f = -nu/Ly (dU_NY-1 - dU_0).re ;  u(0,0) = U ;  om_z(0,0) = -dU
 //   (W: om_x(0,0) = +dW)
-// ---------------------------------------------------------------------------
-__global__ void k_adj_mean(AdjMeanArgs a) {
-  const int t = threadIdx.x;
-  if (t >= 2) return;
-  const int NY = a.NY, n = a.n_g, M = a.M;
+//
+// One block: the solves are a serial chain, one lane per real component of each
+// profile; the factors of mode (0, 0) (strided by the number of unique modes in
+// memory) and the vectors are in shared memory, everything else is spread over
+// the block.  128x129x128, two threads on device memory -> here: 1.36 -> 0.26 ms.
+constexpr int kAMNThreads = 256, kAMNBand = 19;  // band rows of the factors
+size_t adj_mean_smem(int NY, int n) {
+  return 2 * (size_t)(NY + n) * sizeof(double2) + (size_t)kAMNBand * n * sizeof(double) + n;
+}
+constexpr size_t kAMNSmem = 200 * 1024;  // larger factors are read from device memory
+
+template <bool SMEM>
+__global__ void __launch_bounds__(kAMNThreads) k_adj_mean(const __grid_constant__ AdjMeanArgs a) {
+  const int t = threadIdx.x, NY = a.NY, n = a.n_g, M = a.M;
   const double icg = a.inv_cg0, nu = a.nu;
-  double2 *sc = a.scratch + (size_t)t * (3 * NY + n);
-  double2 *ubar = sc, *dbar = sc + NY, *sb = sc + 2 * NY, *yy = sc + 3 * NY;
-  double2 *X0 = t == 0 ? a.Ub[0] : a.Wb[0];
-  double2 *X1 = t == 0 ? a.Ub[1] : a.Wb[1];
-  double2 *X2 = t == 0 ? a.Ub[2] : a.Wb[2];
-  double2 *L0 = t == 0 ? a.Lxb[0] : a.Lzb[0];
-  double2 *L1 = t == 0 ? a.Lxb[1] : a.Lzb[1];
-  double2 *L2 = t == 0 ? a.Lxb[2] : a.Lzb[2];
-  double *F0 = t == 0 ? a.fxb[0] : a.fzb[0];
-  double *F1 = t == 0 ? a.fxb[1] : a.fzb[1];
-  double *F2 = t == 0 ? a.fxb[2] : a.fzb[2];
-  const double2 *fld = t == 0 ? a.ub : a.wb;
-  for (int j = 0; j < NY; ++j) {
-    const double2 x = X0[j], y = fld[(size_t)j * M];
-    ubar[j] = make_double2(x.x + y.x, x.y + y.y);
-    const double2 o = t == 0 ? a.ozb[(size_t)j * M] : a.oxb[(size_t)j * M];
-    dbar[j] = t == 0 ? make_double2(-o.x, -o.y) : o;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double2 *sb = SMEM ? reinterpret_cast<double2 *>(smraw) : a.scratch;  // [2][NY] source adjoints
+  double2 *yy = sb + 2 * NY;                                            // [2][n]
+  const double *ab = a.ab_g;
+  const uint8_t *piv = a.piv_g;
+  const int U = SMEM ? 1 : a.U;
+  if (SMEM) {
+    double *sab = reinterpret_cast<double *>(yy + 2 * n);
+    uint8_t *spv = reinterpret_cast<uint8_t *>(sab + (size_t)kAMNBand * n);
+    for (int e = t; e < kAMNBand * n; e += blockDim.x) sab[e] = a.ab_g[(size_t)e * a.U];
+    for (int e = t; e < n; e += blockDim.x) spv[e] = a.piv_g[(size_t)e * a.U];
+    ab = sab;
+    piv = spv;
   }
-  const double fbar = *F0 + (t == 0 ? a.weight : 0.0);
-  dbar[NY - 1].x += -nu / a.Ly * fbar;
-  dbar[0].x += nu / a.Ly * fbar;
-  for (int j = 0; j < NY; ++j) {
+  for (int e = t; e < 2 * NY; e += blockDim.x) {
+    const int q = e / NY, j = e - q * NY;
+    const double2 x = q == 0 ? a.Ub[0][j] : a.Wb[0][j], f = (q == 0 ? a.ub : a.wb)[(size_t)j * M];
+    const double2 ubar = make_double2(x.x + f.x, x.y + f.y);
+    const double2 o = (q == 0 ? a.ozb : a.oxb)[(size_t)j * M];
+    double2 dbar = q == 0 ? make_double2(-o.x, -o.y) : o;
+    const double fbar = q == 0 ? *a.fxb[0] + a.weight : *a.fzb[0];
+    if (j == NY - 1) dbar.x += -nu / a.Ly * fbar;
+    if (j == 0) dbar.x += nu / a.Ly * fbar;
     const bool in = j != 0 && j != NY - 1;
-    sb[j] = in ? make_double2(icg * ubar[j].x, icg * ubar[j].y) : make_double2(0.0, 0.0);
+    const double w1 = in ? nu * a.c21[j] * icg : 0.0, w2 = in ? a.inv_h2 * nu * a.c22[j] * icg : 0.0, c1 = a.c11[j];
+    sb[e] = in ? make_double2(icg * ubar.x, icg * ubar.y) : make_double2(0.0, 0.0);
+    yy[q * n + 2 * j] = make_double2(a.inv_h * (c1 * dbar.x + w1 * ubar.x), a.inv_h * (c1 * dbar.y + w1 * ubar.y));
+    yy[q * n + 2 * j + 1] = make_double2(w2 * ubar.x, w2 * ubar.y);
   }
-  auto rhs = [&](int c) -> double2 {
-    const int jn = c >> 1;
-    const bool in = jn != 0 && jn != NY - 1;
-    if (c & 1) {
-      const double w = in ? a.inv_h2 * nu * a.c22[jn] * icg : 0.0;
-      return make_double2(w * ubar[jn].x, w * ubar[jn].y);
-    }
-    const double w = in ? nu * a.c21[jn] * icg : 0.0, c1 = a.c11[jn];
-    return make_double2(a.inv_h * (c1 * dbar[jn].x + w * ubar[jn].x), a.inv_h * (c1 * dbar[jn].y + w * ubar[jn].y));
-  };
-  auto ys = [&](int p, double2 y) { yy[p] = y; };
-  auto yl = [&](int p) -> double2 { return yy[p]; };
-  auto out = [&](int p, double2 z) {
-    const double s = icg * a.rs_g[(size_t)p * a.U];
-    for (int e = 0; e < 5; ++e) {
-      const double b = a.rb_val[p * 5 + e];
-      if (nonzero(b)) {
-        double2 &d = sb[a.rb_col[p * 5 + e]];
-        d.x += b * s * z.x;
-        d.y += b * s * z.y;
-      }
-    }
-  };
-  band_solve_t<6, 6>(a.ab_g, a.piv_g, n, a.U, 0, rhs, ys, yl, out);
+  __syncthreads();
+  if (t < 4) {
+    double *y = reinterpret_cast<double *>(yy + (t >> 1) * n) + (t & 1);
+    band_solve_t<6, 6>(
+        ab, piv, n, U, 0, [&](int c) { return y[2 * c]; }, [&](int p, double v) { y[2 * p] = v; },
+        [&](int p) { return y[2 * p]; }, [&](int p, double z) { y[2 * p] = z; });
+  }
+  __syncthreads();
+  // the rows' sources node by node: those whose last node is j .. j + 4
   const double al0 = 3.0, al1 = -1.5, al2 = 1.0 / 3.0, be0 = 3.0, be1 = -3.0, be2 = 1.0;
-  double fsum = 0.0;
-  for (int j = 0; j < NY; ++j) {
-    const double2 s = sb[j];
-    fsum += s.x;
-    L1[j].x += be0 * s.x; L1[j].y += be0 * s.y;
-    L2[j].x += be1 * s.x; L2[j].y += be1 * s.y;
-    L0[j] = make_double2(be2 * s.x, be2 * s.y);
-    const double q0 = al0 * a.inv_dt, q1 = al1 * a.inv_dt, q2 = al2 * a.inv_dt;
-    X1[j].x += q0 * s.x; X1[j].y += q0 * s.y;
-    X2[j].x += q1 * s.x; X2[j].y += q1 * s.y;
-    X0[j] = make_double2(q2 * s.x, q2 * s.y);
+  const double q0 = al0 * a.inv_dt, q1 = al1 * a.inv_dt, q2 = al2 * a.inv_dt;
+  for (int e = t; e < 2 * NY; e += blockDim.x) {
+    const int q = e / NY, j = e - q * NY;
+    double2 s = sb[e];
+    for (int l = min(j + 4, NY - 1); l >= j; --l)
+      for (int r = a.gptr[l + 1] - 1; r >= a.gptr[l]; --r) {
+        const StrRow &row = a.grows[r];
+        const double w = row.w[4 - (l - j)] * (icg * a.rs_g[(size_t)row.p * a.U]);
+        const double2 z = yy[q * n + row.p];
+        s.x = fma(w, z.x, s.x);
+        s.y = fma(w, z.y, s.y);
+      }
+    sb[e] = s;
+    double2 *const *X = q == 0 ? a.Ub : a.Wb, *const *L = q == 0 ? a.Lxb : a.Lzb;
+    L[1][j].x += be0 * s.x; L[1][j].y += be0 * s.y;
+    L[2][j].x += be1 * s.x; L[2][j].y += be1 * s.y;
+    L[0][j] = make_double2(be2 * s.x, be2 * s.y);
+    X[1][j].x += q0 * s.x; X[1][j].y += q0 * s.y;
+    X[2][j].x += q1 * s.x; X[2][j].y += q1 * s.y;
+    X[0][j] = make_double2(q2 * s.x, q2 * s.y);
   }
-  *F1 += be0 * fsum;
-  *F2 += be1 * fsum;
-  *F0 = be2 * fsum;
+  __syncthreads();
+  if (t < 2) {
+    double fsum = 0.0;
+    for (int j = 0; j < NY; ++j) fsum += sb[t * NY + j].x;
+    double *const *F = t == 0 ? a.fxb : a.fzb;
+    *F[1] += be0 * fsum;
+    *F[2] += be1 * fsum;
+    *F[0] = be2 * fsum;
+  }
 }
 
-void launch_adj_mean(const AdjMeanArgs &a, cudaStream_t st) { k_adj_mean<<<1, 32, 0, st>>>(a); }
+void launch_adj_mean(const AdjMeanArgs &a, cudaStream_t st) {
+  const size_t b = adj_mean_smem(a.NY, a.n_g);
+  if (b <= kAMNSmem) k_adj_mean<true><<<1, kAMNThreads, b, st>>>(a);
+  else k_adj_mean<false><<<1, kAMNThreads, 0, st>>>(a);
+}
+
+cudaError_t adj_prepare(int NY, int n_g) {
+  cudaError_t e = cudaSuccess;
+  if (adj_nl_smem(NY) <= kANLSmem) e = raise_smem_limit(k_adj_nl<true>, adj_nl_smem(NY));
+  if (e == cudaSuccess && adj_mean_smem(NY, n_g) <= kAMNSmem)
+    e = raise_smem_limit(k_adj_mean<true>, adj_mean_smem(NY, n_g));
+  return e;
+}
 
 // ---------------------------------------------------------------------------
 __global__ void k_objective_add(const double *fx_ring, const long long *step, double weight, double *acc) {

@@ -26,7 +26,7 @@ struct AdjNLArgs {
   double2 *lxb, *lyb, *lzb;      // out: adjoint of the Lamb vector [NY][M]
   const double *ab1; const uint8_t *piv1;    // band LU of A_1 (one system)
   const int *b1t_col; const double *b1t_val;  // B_1 transposed, (row, val) x 8 per column
-  double2 *ys, *ws;              // scratch [NY][M]
+  double2 *ys;                   // scratch [NY][M]
 };
 
 // Adjoint of the Lamb vector: inputs are the step's six spectral fields and
@@ -65,11 +65,12 @@ struct AdjMeanArgs {
   double inv_dt, nu, Ly, inv_cg0, inv_h, inv_h2;
   double weight;          // d objective / d fx of this step
   const double *c11, *c21, *c22;
-  const double *ab_g; const uint8_t *piv_g; const int *rb_col; const double *rb_val; const double *rs_g;
+  const double *ab_g; const uint8_t *piv_g; const double *rs_g;
+  const int *gptr; const StrRow *grows;  // the right-hand sides' rows by their last node
   const double2 *ub, *wb, *oxb, *ozb;   // adjoint fields; the mean mode is column 0
   double2 *Ub[3], *Wb[3], *Lxb[3], *Lzb[3];  // [NY] each
   double *fxb[3], *fzb[3];
-  double2 *scratch;       // 2 (3 NY + n_g)
+  double2 *scratch;       // 2 (NY + n_g), where the kernel does not keep it in shared memory
 };
 
 // Adjoint of the mode kernel (both implicit solves and solve_horizontal).
@@ -90,6 +91,7 @@ struct AdjModeArgs {
   double2 *yv, *yg, *sgb;  // scratch rows [n_v], [n_g], [NY] of max(M, str_scratch_values(U)) values
 };
 
+cudaError_t adj_prepare(int NY, int n_g);
 void launch_adj_nl(const AdjNLArgs &a, cudaStream_t st);
 cudaError_t adj_lamb_prepare(const XformDims &d);
 void launch_adj_lamb(const AdjXformArgs &a, cudaStream_t st);  // three launches

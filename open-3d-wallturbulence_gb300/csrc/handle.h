@@ -270,7 +270,7 @@ struct owt_handle {
     double2 *hist[5][3] = {};  // adjoints of the v, omega_y, Hv, Hg, DY2 v histories
     double2 *mean[4][3] = {};  // U, W, mean lx, mean lz
     double *fric[2][3] = {};   // fx, fz
-    double2 *lb[3] = {}, *fb[6] = {}, *xs[2] = {};
+    double2 *lb[3] = {}, *fb[6] = {}, *ys = nullptr;
     double2 *zbuf = nullptr, *lbuf = nullptr, *yv = nullptr, *yg = nullptr, *sgb = nullptr, *mscr = nullptr;
     double2 *grad = nullptr;
     double *fric_block = nullptr;

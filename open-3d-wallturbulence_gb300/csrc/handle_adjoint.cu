@@ -69,7 +69,7 @@ void owt_handle::adj_alloc() {
     for (int l = 0; l < 3; ++l) adj.fric[q][l] = adj.fric_block + 3 * q + l;
   for (auto &p3 : adj.lb) p3 = dalloc<double2>(fs, owned);
   for (auto &p3 : adj.fb) p3 = dalloc<double2>(fs, owned);
-  for (auto &p3 : adj.xs) p3 = dalloc<double2>(fs, owned);
+  adj.ys = dalloc<double2>(fs, owned);
   const XformDims xd{NY, NZ, NXH, NZH, NX2, NZ2};
   adj.zbuf = dalloc<double2>(adj_zbuf_values(xd), owned);
   adj.lbuf = dalloc<double2>(adj_lbuf_values(xd), owned);
@@ -77,9 +77,10 @@ void owt_handle::adj_alloc() {
   adj.yv = dalloc<double2>((size_t)bv.n * row, owned);
   adj.yg = dalloc<double2>((size_t)bg.n * row, owned);
   adj.sgb = dalloc<double2>((size_t)NY * row, owned);
-  adj.mscr = dalloc<double2>(2 * (3 * (size_t)NY + bg.n), owned);
+  adj.mscr = dalloc<double2>(2 * ((size_t)NY + bg.n), owned);
   adj.grad = dalloc<double2>(2 * (size_t)M, owned);
   ck(adj_lamb_prepare(xd), "adjoint transform kernel attributes");
+  ck(adj_prepare(NY, bg.n), "adjoint kernel attributes");
   adj.ready = true;
 }
 
@@ -89,7 +90,7 @@ void owt_handle::adjoint_step(const double2 *tp, double wgt) {
   na.hvb = adj.hist[2][0]; na.hgb = adj.hist[3][0]; na.lxmb = adj.mean[2][0]; na.lzmb = adj.mean[3][0];
   na.lxb = adj.lb[0]; na.lyb = adj.lb[1]; na.lzb = adj.lb[2];
   na.ab1 = b1.ab; na.piv1 = b1.piv; na.b1t_col = b1t_col; na.b1t_val = b1t_val;
-  na.ys = adj.xs[0]; na.ws = adj.xs[1];
+  na.ys = adj.ys;
   launch_adj_nl(na, st);
 
   AdjXformArgs xa{};
@@ -108,7 +109,7 @@ void owt_handle::adjoint_step(const double2 *tp, double wgt) {
   ma.inv_dt = 1.0 / p.dt; ma.nu = p.nu; ma.Ly = Ly; ma.inv_cg0 = inv_cg0;
   ma.inv_h = 1.0 / grid.ds; ma.inv_h2 = 1.0 / (grid.ds * grid.ds); ma.weight = wgt;
   ma.c11 = c11; ma.c21 = c21; ma.c22 = c22;
-  ma.ab_g = bg.ab; ma.piv_g = bg.piv; ma.rb_col = rb_col; ma.rb_val = rb_val; ma.rs_g = bg.rscale;
+  ma.ab_g = bg.ab; ma.piv_g = bg.piv; ma.rs_g = bg.rscale; ma.gptr = gptr; ma.grows = grows;
   ma.ub = adj.fb[0]; ma.wb = adj.fb[2]; ma.oxb = adj.fb[3]; ma.ozb = adj.fb[5];
   for (int l = 0; l < 3; ++l) {
     ma.Ub[l] = adj.mean[0][l]; ma.Wb[l] = adj.mean[1][l]; ma.Lxb[l] = adj.mean[2][l]; ma.Lzb[l] = adj.mean[3][l];
