@@ -285,9 +285,9 @@ int owt_state_restore(owt_handle *h);
  * OWT_INFO_PATTERN_VIOLATIONS: modes whose factors fell outside the sparse
  *   pattern at setup (any such mode selects the full-band solve).
  * OWT_INFO_DEVICE_BYTES: device memory held by the handle.
- * Autotuning: owt_create times every variant of the mode kernel (thread
- * mapping, block shape, register budget; bitwise-identical results) and keeps
- * the fastest.  OWT_INFO_MODES_VARIANT is the variant in use,
+ * Autotuning: before a handle's first own step every variant of the mode
+ * kernel (thread mapping, block shape, register budget; bitwise-identical
+ * results) is timed and the fastest kept.  OWT_INFO_MODES_VARIANT is the variant in use,
  * OWT_INFO_MODES_VARIANTS their number, OWT_OPT_MODES_VARIANT forces one
  * (-1 returns to the tuned choice), owt_tuning_report() lists the timings. */
 #define OWT_OPT_FORCE_DENSE_BANDS 1

@@ -1,7 +1,10 @@
 // The Lamb vector's adjoint (adjoint.cu) with fixed-point line transforms, for
 // the line lengths with a plan: the same three kernels, data layouts, weights
 // and products as the FP64 ones, on the passes of transforms_fix.cuh.  One
-// translation unit per plan class (adjoint_fix0.cu, ...).
+// translation unit per plan class (adjoint_fix0.cu, ...).  The x pass has the
+// integer work of the forward one and its FP64 pipe half busy with conversions
+// and products: 128x129x128, FP64 kernel -> this, 2.06 -> 0.74 ms (0.93 with
+// two fields in a packed line and one line a group).
 #pragma once
 #include "adjoint_kernels.h"
 #include "transforms_fix.cuh"

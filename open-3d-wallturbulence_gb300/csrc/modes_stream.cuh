@@ -25,7 +25,7 @@
 // FP64 pipe 95% busy, bound by it), 320x160x320 7.5 -> 5.6, 128x129x128
 // 1.81 -> 1.0, 64x97x48 1.38 -> 0.73, 32x65x32 0.62 -> 0.49 (a warp's own FP64
 // instructions 0.53 of the 128x129x128 time; the fullest SMs have four of the
-// 514 blocks there, the average 3.4), the 64-channel ensemble 4.79 -> 3.82.  A
+// 514 blocks there, the average 3.4), the 64-channel ensemble 4.79 -> 3.76.  A
 // cp.async ring over the band storage without packing gave 1.50 at
 // 128x129x128: 16 instructions for each FP64 one, against 9.5 here.
 //

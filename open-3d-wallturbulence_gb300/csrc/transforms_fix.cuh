@@ -21,16 +21,16 @@
 //  k_zfwd_fx  : as k_zback_fx, forward.
 //
 // Measured at 384x257x384 (lines of 576 points), FP64 kernels -> these:
-// z backward 10.74 -> 1.65 ms, x pass 27.99 -> 7.21 ms, z forward
-// 5.27 -> 0.96 ms; at 128x129x128 0.496 -> 0.095, 1.189 -> 0.388 and
-// 0.255 -> 0.061 ms.  The z passes are bound by integer issue at half of the
-// DRAM rate, the x pass by latency (about 1.4 instructions a clock whatever the
-// number of resident blocks; a fifth of the stalls are its barriers, an eighth
-// instruction fetch).  In the x pass FP64 products of converted values took
-// 7.85 and 0.42 ms: a conversion is an FP64 instruction, and the FP64 pipe was
-// 43% busy.  Block shapes were measured over the classes (three blocks an SM
-// instead of two for the x pass of class 2: 12.2 -> 7.9 ms with the zero thirds
-// left out; z blocks of 4 or 16 columns 5 to 25% slower).
+// z backward 10.74 -> 1.65 ms, x pass 27.99 -> 6.92 ms, z forward
+// 5.27 -> 0.96 ms; at 128x129x128 0.496 -> 0.095, 1.189 -> 0.400 and
+// 0.255 -> 0.060 ms.  The z passes are bound by integer issue at half of the
+// DRAM rate, the x pass by latency (about 1.6 instructions a clock whatever the
+// number of resident blocks; a fifth of the stalls are its barriers).  In the
+// x pass FP64 products of converted values took 7.85 and 0.42 ms: a conversion
+// is an FP64 instruction, and the FP64 pipe was 43% busy.  Block shapes were
+// measured over the classes (three blocks an SM instead of two for the x pass
+// of class 2: 12.2 -> 7.9 ms with the zero thirds left out; z blocks of 4 or 16
+// columns 5 to 25% slower).
 #pragma once
 #include <cuda_runtime.h>
 
