@@ -165,8 +165,9 @@ int owt_call(owt_handle *h, int routine);
 int owt_synchronize(owt_handle *h);
 
 /* Copy a spectral field (enum owt_field) between host [z][x][y] complex128
- * and the device.  A pinned (page-locked), 16-byte aligned host array is
- * written by the GPU's own stores at the host link's rate. */
+ * and the device.  A 16-byte aligned host array that lies as a whole in one
+ * page-locked allocation or registration is written by the GPU's own stores at
+ * the host link's rate; any other one is staged. */
 int owt_get_field(owt_handle *h, int field, double *host);
 int owt_set_field(owt_handle *h, int field, const double *host);
 

@@ -3,6 +3,7 @@
 // the reference routines run one at a time, init_fields, and the layout
 // transposes of host <-> device copies.
 #include "handle.h"
+#include "host_view.h"
 
 using namespace owt;
 
@@ -386,17 +387,10 @@ void owt_handle::to_device(const double *host, double2 *dst) {
   check_launch("layout transpose");
 }
 
-// The device address of a host array the kernels can read and write directly
-// (pinned or registered memory, 16-byte aligned), or null.
-static double2 *device_view(const double *p) {
-  if (reinterpret_cast<uintptr_t>(p) % 16 != 0) return nullptr;
-  cudaPointerAttributes at{};
-  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
-  return static_cast<double2 *>(at.devicePointer);
+// A field in host memory as kernels address it, or null where they may not
+// access the whole of it.
+static double2 *host_field(const double *p, size_t fs, bool write) {
+  return static_cast<double2 *>(host_view(host_range(p), reinterpret_cast<uintptr_t>(p), fs * sizeof(double2), write));
 }
 
 // Pinned arrays are written by the transpose itself over the host link (a field
@@ -404,7 +398,7 @@ static double2 *device_view(const double *p) {
 // times ran at a tenth of the link's rate, 4 to 25 ms); others go through the
 // staging buffer.
 void owt_handle::to_host(const double2 *src, double *host) {
-  double2 *direct = device_view(host);
+  double2 *direct = host_field(host, fs, true);
   launch_transpose(src, direct ? direct : stage, NY, M, st);  // [NY][M] -> [M][NY]
   ++launches;
   check_launch("layout transpose");
@@ -562,7 +556,7 @@ void owt_handle::step_host(const double *const *hist, const double *means, const
   double2 *rings[4] = {v_ring, g_ring, hv_ring, hg_ring};
   const size_t row = (size_t)NXH * NY;  // complex values of one kz row, reference layout
   const double2 *hdev[12];
-  for (int i = 0; i < 12; ++i) hdev[i] = device_view(hist[i]);
+  for (int i = 0; i < 12; ++i) hdev[i] = host_field(hist[i], fs, false);
   // row blocks [k0, k1) of chunk j: |kz| in [a, b) for kz <= NZH, and the
   // negative partners NZ - |kz| for 1 <= |kz| < NZH
   auto blocks = [&](int j, int (&k0)[2], int (&k1)[2]) {
@@ -653,7 +647,7 @@ void owt_handle::step_host(const double *const *hist, const double *means, const
   double *outs[2] = {v_out, g_out};
   double2 *src[2] = {v_ring + (size_t)hn * fs, g_ring + (size_t)hn * fs};
   for (int b = 0; b < 2; ++b) {
-    double2 *direct = device_view(outs[b]);
+    double2 *direct = host_field(outs[b], fs, true);
     launch_transpose(src[b], direct ? direct : hs.dstage[b], NY, M, hs.down);  // [NY][M] -> [M][NY]
     ++launches;
     if (!direct)
