@@ -157,6 +157,7 @@ void owt_handle::drag_backward(double gJ, double *grad_bottom, double *grad_top)
   if (adj.tape_len < adj.interval) {
     if (adj.tape) free_owned(adj.tape);
     adj.tape = nullptr;
+    adj.tape_len = 0;  // none while the new one may not fit
     adj.tape = dalloc<double2>(6 * fs * (size_t)adj.interval, owned);
     adj.tape_len = adj.interval;
   }
