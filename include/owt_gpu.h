@@ -282,6 +282,12 @@ int owt_state_restore(owt_handle *h);
  *   the mode kernel over this many chunks of Fourier modes (1 .. 8; 0 = the
  *   default: 2, or 1 for channels whose mode kernel has too few blocks to be
  *   shared out) when the mode kernel in use maps threads by quads.
+ * OWT_OPT_STREAM_BYTES: device memory the mode kernel's packed copy of the
+ *   factors may take, in bytes (-1, the default: what the device has).  Where
+ *   it does not fit, the kernel reads the factors themselves: slower, with the
+ *   same results.  The copy is also given back when another allocation of the
+ *   handle fails, and made again before the next step; not while the handle
+ *   steps in a batch that uses it.
  * OWT_INFO_SPARSE_SOLVE: 1 if the interior-sparse v-system solve is active.
  * OWT_INFO_PATTERN_VIOLATIONS: modes whose factors fell outside the sparse
  *   pattern at setup (any such mode selects the full-band solve).
@@ -296,6 +302,7 @@ int owt_state_restore(owt_handle *h);
 #define OWT_OPT_FFT_STOCKHAM 3
 #define OWT_OPT_MEAN_SPLIT 4
 #define OWT_OPT_HOST_CHUNKS 5
+#define OWT_OPT_STREAM_BYTES 6
 #define OWT_INFO_SPARSE_SOLVE 1
 #define OWT_INFO_PATTERN_VIOLATIONS 2
 #define OWT_INFO_DEVICE_BYTES 3

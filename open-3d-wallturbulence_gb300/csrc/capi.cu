@@ -262,6 +262,11 @@ int owt_set_option(owt_handle *h, int option, int64_t value) {
     } else if (option == OWT_OPT_MODES_VARIANT) {
       if (value < -1 || value >= modes_variant_count()) throw OwtError(OWT_ERR_INVALID, "no such variant");
       h->forced_variant = (int)value;
+    } else if (option == OWT_OPT_STREAM_BYTES) {
+      if (value < -1) throw OwtError(OWT_ERR_INVALID, "the limit must be a number of bytes, or -1");
+      h->str_limit = value;
+      h->release_streams();
+      h->str_denied = h->tuned = false;
     } else {
       throw OwtError(OWT_ERR_INVALID, "unknown option");
     }
@@ -277,7 +282,7 @@ int owt_get_info(const owt_handle *h, int what, int64_t *value) {
     case OWT_INFO_SPARSE_SOLVE: *value = ((h->sparse_v || h->sparse_v6) && !h->force_dense) ? 1 : 0; return OWT_OK;
     case OWT_INFO_PATTERN_VIOLATIONS: *value = h->pattern_violations; return OWT_OK;
     case OWT_INFO_DEVICE_BYTES: *value = (int64_t)h->device_bytes; return OWT_OK;
-    case OWT_INFO_MODES_VARIANT: *value = h->forced_variant >= 0 ? h->forced_variant : h->modes_variant; return OWT_OK;
+    case OWT_INFO_MODES_VARIANT: *value = h->forced_variant >= 0 && !h->str_denied ? h->forced_variant : h->variant(); return OWT_OK;
     case OWT_INFO_MODES_VARIANTS: *value = modes_variant_count(); return OWT_OK;
     default: return OWT_ERR_INVALID;
   }

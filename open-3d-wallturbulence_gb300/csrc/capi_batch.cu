@@ -205,6 +205,8 @@ struct owt_batch {
   // Time every variant of the batched mode kernel on the channels' current
   // state, then put back what the trials overwrote (the v, omega_y and DY2 v
   // rings and the horizontal fields) and keep the fastest.
+  // The channels' factor streams come after the copies: where they do not all
+  // fit, the variants on the band storage are timed alone.
   void autotune() {
     if (by_size(true).empty()) {
       tuning = "full-band solve (no variants)";
@@ -223,7 +225,14 @@ struct owt_batch {
       for (size_t i = 0; i < hs.size(); ++i) {
         owt_handle *h = hs[i];
         const size_t fs = h->fs;
-        ck(cudaMalloc(&snap[i], 13 * fs * sizeof(double2)), "tuning snapshot");
+        cudaError_t e = cudaMalloc(&snap[i], 13 * fs * sizeof(double2));
+        if (e == cudaErrorMemoryAllocation) {  // streams of the channels' own steps
+          bool any = false;
+          for (owt_handle *r : hs) any = r->release_streams() || any;
+          cudaGetLastError();
+          if (any) e = cudaMalloc(&snap[i], 13 * fs * sizeof(double2));
+        }
+        ck(e, "tuning snapshot");
         double2 *o = snap[i];
         for (double2 *ring : {h->v_ring, h->g_ring, h->q_ring}) {
           ck(cudaMemcpyAsync(o, ring, 3 * fs * sizeof(double2), cudaMemcpyDeviceToDevice, st), "snapshot");
@@ -234,10 +243,13 @@ struct owt_batch {
           o += fs;
         }
       }
+      bool streams = true;
+      for (int i : by_size(true)) streams = streams && hs[i]->build_streams();
+      for (owt_handle *h : hs) ck(cudaStreamSynchronize(h->st), "factor streams");
       ck(cudaEventCreate(&e0), "event");
       ck(cudaEventCreate(&e1), "event");
       float best = 1e30f;
-      for (int v = 0; v < modes_variant_count(); ++v) {
+      for (int v = 0; v < (streams ? modes_variant_count() : modes_band_count()); ++v) {
         build_modes(v, true);
         launch_modes_all(st);  // warm-up
         ck(cudaEventRecord(e0, st), "event");
@@ -274,6 +286,8 @@ struct owt_batch {
       throw;
     }
     cleanup();
+    if (modes_variant >= modes_band_count())
+      for (int i : by_size(true)) hs[i]->str_kept = true;
     tuning += std::string(" -> ") + modes_variant_name(modes_variant);
   }
 };
@@ -296,7 +310,6 @@ int owt_batch_create(owt_handle *const *handles, int count, owt_batch **out) {
         if (handles[r] == h) throw OwtError(OWT_ERR_INVALID, "a handle appears twice in the batch");
       ck(cudaStreamSynchronize(h->st), "batch");
       h->recompute_dirty_q();
-      if (h->sparse_v) h->build_streams();
       ck(cudaStreamSynchronize(h->st), "batch");
       b->hs.push_back(h);
     }

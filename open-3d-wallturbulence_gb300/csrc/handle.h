@@ -35,6 +35,10 @@ namespace owt {
 extern thread_local std::string g_create_error;
 // While set, device allocations of dalloc are counted here.
 extern thread_local size_t *g_alloc_counter;
+// The handle whose entry point the thread is in (guard), or null.
+extern thread_local owt_handle *g_handle;
+// Give back what that handle holds only to be faster; false: nothing to give.
+bool release_for_allocation();
 
 struct CudaError : std::runtime_error {
   using std::runtime_error::runtime_error;
@@ -52,13 +56,17 @@ template <typename T>
 T *dalloc(size_t n, std::vector<void *> &owned) {
   void *p = nullptr;
   if (n == 0) n = 1;
-  if (g_alloc_counter) *g_alloc_counter += n * sizeof(T);
   cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+  if (e == cudaErrorMemoryAllocation && release_for_allocation()) {
+    cudaGetLastError();
+    e = cudaMalloc(&p, n * sizeof(T));
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     throw OwtError(OWT_ERR_NOMEM, std::string("cudaMalloc of ") + std::to_string(n * sizeof(T)) +
                                       " bytes failed: " + cudaGetErrorString(e));
   }
+  if (g_alloc_counter) *g_alloc_counter += n * sizeof(T);
   owned.push_back(p);
   return static_cast<T *>(p);
 }
@@ -125,10 +133,20 @@ struct owt_handle {
   double *rbv_val = nullptr;
   int *vptr = nullptr, *gptr = nullptr;  // right-hand sides by last node (StrRow)
   owt::StrRow *vrows = nullptr, *grows = nullptr;
-  // packed factor streams, built before the handle's first own step
+  // Packed factor streams (modes_stream.cuh), a second copy of the factors
+  // that makes the mode kernel faster.  Built before a step where they fit the
+  // device and their limit; released when another allocation of the handle
+  // fails, and built again before the next step.  Without them the mode kernel
+  // reads the band storage (the sixth-order and the adjoint solves the full
+  // band), with the same results.
   owt::StrBuffers str;
+  size_t str_bytes = 0;
+  int64_t str_limit = -1;   // bytes they may take (-1: any number)
+  bool str_denied = false;  // they did not fit: not tried again
+  bool str_kept = false;    // a batch holds their addresses: never released
   int n_vrows = 0, n_grows = 0;
-  void build_streams();
+  bool build_streams();     // whether the handle has them
+  bool release_streams();
   double *rb_val = nullptr, *b1_val = nullptr, *b2_val = nullptr;
   // scratch
   double2 *sg = nullptr, *dg = nullptr, *yv = nullptr, *yg = nullptr, *sv = nullptr;
@@ -188,6 +206,8 @@ struct owt_handle {
   int host_chunks = 0;       // owt_time_integration_host: chunks of modes (0: the default)
   bool mean_smem = false;    // staged mean-mode solve in shared memory
   int modes_variant = 0;     // chosen by the autotuner
+  int band_variant = 0;      // the fastest of those that need no streams
+  int variant() const;       // the one a step runs
   int forced_variant = -1;   // testing aid: run this variant instead
   std::string tuning;        // autotuner report
 
@@ -310,6 +330,11 @@ namespace owt {
 template <typename F>
 int guard(owt_handle *h, F &&f) {
   if (!h) return OWT_ERR_INVALID;
+  struct Within {
+    owt_handle *before = g_handle;
+    explicit Within(owt_handle *now) { g_handle = now; }
+    ~Within() { g_handle = before; }
+  } within(h);
   try {
     f();
     h->err.clear();

@@ -137,7 +137,7 @@ void owt_handle::adjoint_step(const double2 *tp, double wgt) {
     mo.hg[l] = adj.hist[3][l]; mo.q[l] = adj.hist[4][l];
   }
   mo.grad = adj.grad; mo.yv = adj.yv; mo.yg = adj.yg; mo.sgb = adj.sgb;
-  launch_adj_modes(mo, force_dense ? 0 : sparse_v ? 1 : sparse_v6 ? 2 : 0, st);
+  launch_adj_modes(mo, force_dense || !str.vf ? 0 : sparse_v ? 1 : sparse_v6 ? 2 : 0, st);
   ck(cudaStreamWaitEvent(st, ev_join, 0), "join wait");
   launches += 6;
   check_launch("adjoint step");
@@ -153,7 +153,6 @@ void owt_handle::drag_backward(double gJ, double *grad_bottom, double *grad_top)
   if (adj.nsteps == 0 || adj.version != state_version)
     throw OwtError(OWT_ERR_STATE, "owt_drag_forward must come first, with no change of state or wall velocity since");
   adj_alloc();
-  build_streams();
   if (adj.tape_len < adj.interval) {
     if (adj.tape) free_owned(adj.tape);
     adj.tape = nullptr;

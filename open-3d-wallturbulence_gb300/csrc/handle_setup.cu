@@ -8,6 +8,8 @@ using namespace owt;
 
 namespace owt {
 thread_local size_t *g_alloc_counter = nullptr;
+thread_local owt_handle *g_handle = nullptr;
+bool release_for_allocation() { return g_handle && g_handle->release_streams(); }
 }  // namespace owt
 
 owt_handle::~owt_handle() {

@@ -99,12 +99,11 @@ void owt_handle::step_finish() {
 }
 
 void owt_handle::stage_modes() {
-  if (sparse_v6 && !force_dense) {
+  if (sparse_v6 && !force_dense && str.vf) {
     launch_modes_sixth(mode_args(), st);
     return;
   }
-  launch_modes(mode_args(), bv.kl, bv.ku, bg.kl, bg.ku, modes_sparse(),
-               forced_variant >= 0 ? forced_variant : modes_variant, st);
+  launch_modes(mode_args(), bv.kl, bv.ku, bg.kl, bg.ku, modes_sparse(), variant(), st);
 }
 
 ModeArgs owt_handle::mode_args() const {
@@ -177,32 +176,62 @@ void owt_handle::run_steps(int64_t n) {
   check_launch("time step");
 }
 
-// The factors of the stream mapping (a handle stepped only inside a batch never
-// needs them).
-void owt_handle::build_streams() {
-  if (str.vf || !(sparse_v || sparse_v6)) return;
+bool owt_handle::build_streams() {
+  if (str.vf) return true;
+  if (str_denied || !(sparse_v || sparse_v6)) return false;
   const StrSizes z = str_sizes(bv.n, bg.n, sparse_v6);
   const size_t g = (size_t)str_groups(Uq);
-  g_alloc_counter = &device_bytes;
-  struct Reset { ~Reset() { g_alloc_counter = nullptr; } } reset_counter;
   StrBuffers b;
-  b.vf = dalloc<double>(z.vf * g, owned);
-  b.vb = dalloc<double>(z.vb * g, owned);
-  b.gf = dalloc<double>(z.gf * g, owned);
-  b.gb = dalloc<double>(z.gb * g, owned);
-  b.vrs = dalloc<double>((size_t)n_vrows * Uq, owned);
-  b.grs = dalloc<double>((size_t)n_grows * Uq, owned);
+  const std::pair<double **, size_t> parts[] = {{&b.vf, z.vf * g}, {&b.vb, z.vb * g}, {&b.gf, z.gf * g}, {&b.gb, z.gb * g},
+                                                {&b.vrs, (size_t)n_vrows * Uq}, {&b.grs, (size_t)n_grows * Uq}};
+  std::vector<void *> got;
+  size_t bytes = 0;
+  try {
+    for (const auto &q : parts) {
+      bytes += q.second * sizeof(double);
+      if (str_limit >= 0 && bytes > (size_t)str_limit) throw OwtError(OWT_ERR_NOMEM, "factor streams beyond their limit");
+      *q.first = dalloc<double>(q.second, got);
+    }
+  } catch (const OwtError &) {
+    for (void *q : got) cudaFree(q);
+    str_denied = true;
+    return false;
+  }
+  owned.insert(owned.end(), got.begin(), got.end());
+  device_bytes += bytes;
+  str = b;
+  str_bytes = bytes;
+  drop_graph();  // of the kernels that do without
   launch_str_pack(mode_args(), sparse_v6, b, n_vrows, n_grows, st);
   launches += 4;
   check_launch("factor streams");
-  str = b;
+  return true;
+}
+
+bool owt_handle::release_streams() {
+  if (!str.vf || str_kept) return false;
+  ck(cudaStreamSynchronize(st), "factor streams");
+  drop_graph();  // it holds their addresses
+  for (double *q : {str.vf, str.vb, str.gf, str.gb, str.vrs, str.grs}) free_owned(q);
+  device_bytes -= str_bytes;
+  str = StrBuffers{};
+  str_bytes = 0;
+  return true;
+}
+
+int owt_handle::variant() const {
+  const int v = forced_variant >= 0 ? forced_variant : modes_variant;
+  return str.vf || v < modes_band_count() ? v : band_variant;
 }
 
 void owt_handle::ensure_tuned() {
-  if (tuned) return;
-  build_streams();
+  if (tuned) {
+    build_streams();
+    return;
+  }
   tuned = true;
   if (!initialized) {
+    build_streams();
     autotune_modes();
     return;
   }
@@ -210,6 +239,7 @@ void owt_handle::ensure_tuned() {
   double2 *snap = nullptr;
   ck(cudaMalloc(&snap, 13 * fs * sizeof(double2)), "tuning snapshot");
   try {
+    build_streams();  // (after the snapshot, which the trials cannot do without)
     double2 *o = snap;
     for (double2 *ring : {v_ring, g_ring, q_ring}) { d2d(o, ring, 3 * fs * sizeof(double2)); o += 3 * fs; }
     for (double2 *f : {u, w, ox, oz}) { d2d(o, f, fs * sizeof(double2)); o += fs; }
@@ -227,15 +257,18 @@ void owt_handle::ensure_tuned() {
 }
 
 void owt_handle::autotune_modes() {
-  modes_variant = 0;
+  modes_variant = band_variant = 0;
   tuning.clear();
-  if (sparse_v6) { tuning = "sixth-order masked solve (one variant)"; return; }
+  if (sparse_v6) {
+    tuning = str.vf ? "sixth-order masked solve (one variant)" : "full-band solve (no memory for the sixth-order masked one)";
+    return;
+  }
   if (!sparse_v) { tuning = "full-band solve (no variants)"; return; }
   cudaEvent_t e0, e1;
   ck(cudaEventCreate(&e0), "event");
   ck(cudaEventCreate(&e1), "event");
   float best = 1e30f;
-  for (int v = 0; v < modes_variant_count(); ++v) {
+  for (int v = 0; v < (str.vf ? modes_variant_count() : modes_band_count()); ++v) {
     forced_variant = v;
     stage_modes();  // warm-up
     ck(cudaEventRecord(e0, st), "event");
@@ -249,7 +282,11 @@ void owt_handle::autotune_modes() {
     char buf[96];
     std::snprintf(buf, sizeof(buf), "%s%s=%.3fms", tuning.empty() ? "" : " ", modes_variant_name(v), ms);
     tuning += buf;
-    if (ms < best) { best = ms; modes_variant = v; }
+    if (ms < best) {
+      best = ms;
+      modes_variant = v;
+      if (v < modes_band_count()) band_variant = v;
+    }
   }
   forced_variant = -1;
   cudaEventDestroy(e0);
@@ -531,8 +568,8 @@ void owt_handle::step_host(const double *const *hist, const double *means, const
   host_step_prepare();
   ensure_tuned();
   ck(cudaStreamSynchronize(st), "host step");
-  const int variant = forced_variant >= 0 ? forced_variant : modes_variant;
-  const bool quad = modes_sparse() && !sparse_v6 && modes_variant_is_quad(variant);
+  const int var = variant();
+  const bool quad = modes_sparse() && !sparse_v6 && modes_variant_is_quad(var);
   // By default no chunk smaller than twice what is resident at once: a part of
   // the modes of a small channel takes the mode kernel as long as all of them
   // (0.96 against 1.02 ms for half of 128x129x128).
@@ -635,7 +672,7 @@ void owt_handle::step_host(const double *const *hist, const double *means, const
       ModeArgs a = mode_args();
       a.u0 = ((NZH + 1) * j / nchunk) * NXH;
       a.u1 = ((NZH + 1) * (j + 1) / nchunk) * NXH;
-      launch_modes(a, bv.kl, bv.ku, bg.kl, bg.ku, true, variant, st);
+      launch_modes(a, bv.kl, bv.ku, bg.kl, bg.ku, true, var, st);
     }
     ++launches;
   }

@@ -309,6 +309,7 @@ bool band_supported(int kl, int ku) {
 // (separate translation units so they compile in parallel); this dispatches by
 // index, in that order.
 int modes_variant_count() { return modes_pair_count() + modes_quad_count() + modes_stream_count(); }
+int modes_band_count() { return modes_pair_count() + modes_quad_count(); }
 // variants whose launches can be limited to a range of unique modes
 bool modes_variant_is_quad(int v) { return v >= modes_pair_count(); }
 const char *modes_variant_name(int v) {

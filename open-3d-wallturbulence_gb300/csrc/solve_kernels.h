@@ -210,6 +210,7 @@ void launch_modes_sixth(const ModeArgs &a, cudaStream_t st);  // masked solve wi
 // dst[p U + u] = scale[u] src[p U + u], p < n
 void launch_scale_by_mode(double *dst, const double *src, const double *scale, int n, int U, cudaStream_t st);
 int modes_variant_count();  // pair, quad and stream mappings
+int modes_band_count();     // of them those on the band storage, the first ones
 bool modes_variant_is_quad(int v);
 const char *modes_variant_name(int v);
 void launch_check_pattern(int which, const double *ab, const uint8_t *piv, int n, int U, int *bad,

@@ -239,6 +239,11 @@ class GpuSolver:
         over (0: the library's default; OWT_OPT_HOST_CHUNKS)."""
         self._chk(self.L.owt_set_option(self.h, 5, int(n)))
 
+    def limit_stream_bytes(self, n):
+        """Device memory the mode kernel's packed copy of the factors may take
+        (-1: any; OWT_OPT_STREAM_BYTES); without it steps are slower."""
+        self._chk(self.L.owt_set_option(self.h, 6, int(n)))
+
     def force_modes_variant(self, v):
         """Run mode-kernel variant v (-1: the autotuned one)."""
         self._chk(self.L.owt_set_option(self.h, 2, int(v)))
