@@ -1078,10 +1078,11 @@ __global__ void k_stats_final(const double2 *u, const double2 *v, const double2 
   out[0 * NY + j] = U;
   out[1 * NY + j] = V;
   out[2 * NY + j] = W;
+  // sums of squares, so nothing to clamp: a clamp would turn NaN into 0
   // (U - U: 0, or NaN for a mean that is not finite)
-  out[3 * NY + j] = sqrt(fmax(s[0] + (U - U), 0.0));
-  out[4 * NY + j] = sqrt(fmax(s[1] + (V - V), 0.0));
-  out[5 * NY + j] = sqrt(fmax(s[2] + (W - W), 0.0));
+  out[3 * NY + j] = sqrt(s[0] + (U - U));
+  out[4 * NY + j] = sqrt(s[1] + (V - V));
+  out[5 * NY + j] = sqrt(s[2] + (W - W));
   out[6 * NY + j] = s[3] + (U - U) + (V - V);
 }
 // out: 7 NY values, then scratch; stats_values() in all
