@@ -243,24 +243,10 @@ void owt_handle::setup(const owt_params &prm) {
   rbv_val = upload(tv.rbv_val, owned, st);
   rb_col = upload(tg.rb_col, owned, st);
   rb_val = upload(tg.rb_val, owned, st);
-  // B1 / B2 rows as (col, val) x 5
   auto brows = [&](int which, int *&dcol, double *&dval) {
-    std::vector<int> cols((size_t)NY * 5, 0);
-    std::vector<double> vals((size_t)NY * 5, 0.0);
-    for (int j = 0; j < NY; ++j) {
-      int e = 0;
-      for (int c = 0; c < NY; ++c) {
-        const double b = sten.b(which, j, c);
-        if (b != 0.0) {
-          if (e >= 5) throw std::logic_error("stencil row wider than 5");
-          // the nonlinear-source kernel applies B1 with four taps per row
-          if (which == 0 && e >= 4) throw std::logic_error("first-derivative stencil row wider than 4");
-          cols[(size_t)j * 5 + e] = c;
-          vals[(size_t)j * 5 + e] = b;
-          ++e;
-        }
-      }
-    }
+    std::vector<int> cols;
+    std::vector<double> vals;
+    stencil_rows(sten, which, cols, vals);
     dcol = upload(cols, owned, st);
     dval = upload(vals, owned, st);
   };

@@ -163,6 +163,32 @@ Stencils make_stencils(int N, double h, int order) {
   return st;
 }
 
+void stencil_rows(const Stencils &st, int which, std::vector<int> &cols, std::vector<double> &vals) {
+  const int N = st.N;
+  cols.assign((size_t)N * 5, 0);
+  vals.assign((size_t)N * 5, 0.0);
+  for (int j = 0; j < N; ++j) {
+    const int side = j < N - 1 - j ? j : N - 1 - j;  // rows from the nearer wall
+    std::vector<int> at;                             // columns in increasing order
+    if (which == 0) {
+      if (side == 0) at = j == 0 ? std::vector<int>{0, 1, 2, 3} : std::vector<int>{N - 4, N - 3, N - 2, N - 1};
+      else if (side == 1) at = {j - 1, j + 1};
+      else at = {j - 2, j - 1, j + 1, j + 2};
+    } else {
+      if (side == 0) at = j == 0 ? std::vector<int>{0, 1, 2} : std::vector<int>{N - 3, N - 2, N - 1};
+      else if (side == 1) at = j == 1 ? std::vector<int>{0, 1, 2, 3, 4} : std::vector<int>{N - 5, N - 4, N - 3, N - 2, N - 1};
+      else at = {j - 2, j - 1, j, j + 1, j + 2};
+    }
+    for (int c = 0; c < N; ++c)
+      if (st.b(which, j, c) != 0.0 && std::find(at.begin(), at.end(), c) == at.end())
+        throw std::logic_error("a derivative's stencil row has a coefficient where the kernels read none");
+    for (size_t e = 0; e < at.size(); ++e) {
+      cols[(size_t)j * 5 + e] = at[e];
+      vals[(size_t)j * 5 + e] = st.b(which, j, at[e]);
+    }
+  }
+}
+
 namespace {
 
 struct Eq {

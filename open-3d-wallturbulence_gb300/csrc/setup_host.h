@@ -132,6 +132,12 @@ Grid make_grid(int N, double alpha);
 // Compact-FD stencils; order 8 (the reference's interior schemes) or 6
 // (sixth-order tridiagonal interior schemes for D1-D3, same boundary rows).
 Stencils make_stencils(int N, double h, int order = 8);
+// The rows of B_1 (which = 0) or B_2 (1) as the kernels read them, (column,
+// value) x 5 per row: entry e of a row is always the coefficient of the same
+// node, whatever its value -- for B_1 columns 0..3 in row 0, 0 and 2 in row 1,
+// i -+ 2 and i -+ 1 in between, for B_2 0..2, 0..4 and i - 2 .. i + 2, and the
+// mirror image at the top.  Throws for a coefficient at any other node.
+void stencil_rows(const Stencils &st, int which, std::vector<int> &cols, std::vector<double> &vals);
 BandTemplate build_v_system(const Grid &g, const Stencils &st, double nu);
 BandTemplate build_g_system(const Grid &g, const Stencils &st, double nu);
 // Band LU (no per-mode scalars) of A_1, shared by every mode for DY1 f; the
