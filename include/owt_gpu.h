@@ -271,7 +271,14 @@ int owt_state_restore(owt_handle *h);
  *   where register-transform kernels exist for the line length (the two
  *   agree to FP32 rounding; this exists to compare them), and the FP64
  *   transforms their FP64 Stockham kernels instead of the fixed-point ones
- *   (they agree to FP64 rounding).
+ *   (lines of up to 576 points that split into two of the factors 2 .. 6, 8 .. 10,
+ *   12, 15, 16, 18, 20, 24; the two agree to FP64 rounding).  The fixed-point
+ *   ones carry 61 bits below a line's largest magnitude and a narrower range of
+ *   exponents than FP64: a line whose largest magnitude is below 2^-895
+ *   (4e-270) counts as zero, one with a magnitude from 2^1009 (5e303), an
+ *   infinity or a NaN becomes NaN throughout, and a line of the Lamb vector
+ *   whose magnitudes are below about 2^-960 (1e-289) becomes zero.  Set the
+ *   option for fields beyond that.
  * OWT_OPT_MEAN_SPLIT: mixed precision only; 1 (the default) = the FP32
  *   transforms carry the fluctuations, and the mean-flow terms of the Lamb
  *   vector (mean velocity x fluctuating vorticity and back) are formed mode

@@ -224,8 +224,9 @@ class GpuSolver:
         self._chk(self.L.owt_set_option(self.h, 1, 1 if on else 0))
 
     def use_stockham_fft(self, on=True):
-        """FP32 transforms through the shared-memory Stockham kernels instead of
-        the register-transform ones (OWT_OPT_FFT_STOCKHAM), for comparisons."""
+        """Transforms through the shared-memory Stockham kernels instead of the
+        register-transform (FP32) and fixed-point (FP64) ones, for comparisons and
+        for FP64 fields beyond the latter's range (OWT_OPT_FFT_STOCKHAM)."""
         self._chk(self.L.owt_set_option(self.h, 3, 1 if on else 0))
 
     def use_mean_split(self, on=True):
