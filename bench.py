@@ -100,20 +100,21 @@ class ClockSampler:
 # algorithmic work per stage (fixed formulas, derived from the kernels' loops)
 # ---------------------------------------------------------------------------
 def stage_work(p, precision="fp64"):
-    """Algorithmic flops and bytes per launch of each kernel: band solves as LAPACK counts
-    them, FFTs at 5 N log2 N, 9 flops per physical point for the products, and the
-    spectral fields / z-padded planes each kernel must read and write once."""
+    """Algorithmic flops and bytes per launch of each kernel: band solves by the entries
+    their factors keep, FFTs at 5 N log2 N, 9 flops per physical point for the products,
+    and the spectral fields / z-padded planes each kernel must read and write once."""
     import math
     NY, M, NXH, NZ2, NX2 = p.NY, p.NZ * p.NXH, p.NXH, p.NZ2, p.NX2
     S = 16.0 * NY * M  # bytes per spectral field (complex128)
     P = (16.0 if precision == "fp64" else 8.0) * NY * NZ2 * NXH  # one z-padded plane set
-    # banded systems: v-system 4NY+4 unknowns (kl 15, ku 13: its band with the unknowns in
-    # node order, kept as the fixed count), omega_y-system 2NY (6, 6); per column and
-    # complex rhs: 2 * 2 * (2 kl + ku) flops (forward + backward)
-    fl_modes = M * ((4 * NY + 4) * 4 * (2 * 15 + 13) + 2 * NY * 4 * (2 * 6 + 6) + 120 * NY)
+    # banded systems: v-system 4NY+4 unknowns with 21.5 entries of L and U a column and the
+    # diagonal, omega_y-system 2NY with 9 (the eighth-order interior masks' means); a
+    # multiply-add per entry and a product per diagonal, each on two real components, and
+    # 60 more flops a node and component around the solves
+    fl_modes = M * ((4 * NY + 4) * 2 * (2 * 21.5 + 1) + 2 * NY * 2 * (2 * 9 + 1) + 120 * NY)
     fl_fft = lambda n: 5.0 * n * math.log2(n)
     unique = NXH * (p.NZ // 2 + 1)
-    factor_bytes = 8.0 * unique * ((4 * NY + 4) * (2 * 15 + 13 + 1) + 2 * NY * (2 * 6 + 6 + 1))
+    factor_bytes = 8.0 * unique * ((4 * NY + 4) * (21.5 + 1) + 2 * NY * (9 + 1))
     return {
         "modes": {"flops": fl_modes, "bytes": 22 * S + factor_bytes},
         "zback": {"flops": 6 * NXH * NY * fl_fft(NZ2), "bytes": 6 * S + 6 * P},
@@ -124,11 +125,10 @@ def stage_work(p, precision="fp64"):
 
 
 # DRAM traffic per launch from ncu (dram__bytes_read.sum + dram__bytes_write.sum)
-# of the 128x129x128 workload (profiles/k_zback_fx_k_xlamb_fx_k_zfwd_fx_channel180.md
-# and profiles/k_modes_stream_k_mean_channel180.md), scaled to a launch at
-# another size by the units the kernel processes (traffic grows in proportion:
-# y-z lines times kx modes for the transforms, modes times NY for the mode
-# kernel).
+# of the 128x129x128 workload (the fixed-point x pass and the mode kernel on
+# packed streams), scaled to a launch at another size by the units the kernel
+# processes (traffic grows in proportion: y-z lines times kx modes for the
+# transforms, modes times NY for the mode kernel).
 NCU_TRAFFIC_128 = {"xlamb_fp64": 198.95e6, "modes": 1.402e9}
 
 
@@ -344,11 +344,12 @@ def run_ours(args, rank, world, local_rank):
     else:
         roof = {"bound": "fp64", "achieved": fl_dom / t_dom / 1e12, "peak": fp64_peak, "unit": "TFLOP/s"}
     roof["frac"] = roof["achieved"] / roof["peak"]
-    roof["kernel"] = {"modes": "k_modes", "zback": "k_zback", "xlamb": "k_xlamb", "zfwd": "k_zfwd",
-                      "nonlinear": "k_nl"}[dom]
+    kind = "_fx" if args.precision == "fp64" else "_r"
+    roof["kernel"] = {"modes": "k_modes_stream" if "-> stream" in tuning else "k_modes", "zback": "k_zback" + kind,
+                      "xlamb": "k_xlamb" + kind, "zfwd": "k_zfwd" + kind, "nonlinear": "k_nl"}[dom]
     roof["traffic"] = scaled_traffic(dom, p, args.precision)
     roof["algorithmic_bytes"] = work[dom]["bytes"]
-    roof["traffic_source"] = "ncu at 128x129x128, scaled by units processed (profiles/)"
+    roof["traffic_source"] = "ncu at 128x129x128, scaled by units processed"
     roof["peak_source"] = ("cuBLAS DGEMM (torch.matmul float64, 4096^3) measured in this run"
                            if roof["bound"] == "fp64" else f"MEASURED_PEAKS.json hbm_gbs ({peak_kind})")
     if roof["bound"] == "fp64":
@@ -363,6 +364,7 @@ def run_ours(args, rank, world, local_rank):
                                    "source": "2 DFMA per clock per SM x %d SMs x %.0f MHz" % (sms, mhz)}
     roof["stage_ms"] = {k: round(v, 4) for k, v in stage_ms.items()}
     roof["stage_hbm_gbs"] = {k: round(work[k]["bytes"] / (stage_ms[k] * 1e-3) / 1e9, 1) for k in stage_ms}
+    # (the fixed-point transforms by the FP64 flops their integer operations stand for)
     roof["stage_fp64_tflops"] = {k: round(work[k]["flops"] / (stage_ms[k] * 1e-3) / 1e12, 3) for k in stage_ms}
 
     head = results[args.precision]
