@@ -147,13 +147,13 @@ int owt_time_integration(owt_handle *h, int64_t nsteps);
  * to back into staging buffers of their own (the first call allocates them:
  * 12 + 2 fields of device memory, kept by the handle), each field's layout
  * transpose follows its copy, the DY2 v history of the v levels is
- * re-derived while the other fields arrive, with a quad-mapping mode kernel
- * the copies are pipelined with it over chunks of Fourier modes
+ * re-derived while the other fields arrive, with a mode kernel that takes
+ * ranges of modes the copies are pipelined with it over chunks of Fourier modes
  * (OWT_OPT_HOST_CHUNKS), and v and omega_y travel back while the step's
- * transforms run.  History arrays in pinned (page-locked) host memory whose
- * addresses are 16-byte aligned are read by the GPU's own loads at the full
- * host-link rate; other arrays go through the copy engines (pageable memory
- * at a fraction of that rate).
+ * transforms run.  16-byte aligned arrays that lie as a whole in one page-locked
+ * allocation or registration are read and written by the GPU's own loads and
+ * stores at the full host-link rate; other arrays go through the copy engines
+ * (pageable memory at a fraction of that rate).
  * Synchronous: when it returns, the outputs are written. */
 int owt_time_integration_host(owt_handle *h, const double *const *hist, const double *means, const double *fric,
                               double *vely, double *vory, double *fric_out);
@@ -288,7 +288,8 @@ int owt_state_restore(owt_handle *h);
  * OWT_OPT_HOST_CHUNKS: owt_time_integration_host pipelines its uploads with
  *   the mode kernel over this many chunks of Fourier modes (1 .. 8; 0 = the
  *   default: 2, or 1 for channels whose mode kernel has too few blocks to be
- *   shared out) when the mode kernel in use maps threads by quads.
+ *   shared out) when the mode kernel in use takes ranges of modes (the quad and
+ *   stream mappings).
  * OWT_OPT_STREAM_BYTES: device memory the mode kernel's packed copy of the
  *   factors may take, in bytes (-1, the default: what the device has).  Where
  *   it does not fit, the kernel reads the factors themselves: slower, with the

@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kANLThreadsLarge) k_adj_nl(const __grid_consta
 }
 
 void launch_adj_nl(const AdjNLArgs &a, cudaStream_t st) {
-  const int bs = 2 * a.M >= 152 * 4 * kANLThreadsLarge ? kANLThreadsLarge : kANLThreads, gs = (2 * a.M + bs - 1) / bs;
+  const int bs = 2 * a.M >= kSMs * 4 * kANLThreadsLarge ? kANLThreadsLarge : kANLThreads, gs = (2 * a.M + bs - 1) / bs;
   const size_t b = adj_nl_smem(a.NY);
   if (b <= kANLSmem) k_adj_nl<true><<<gs, bs, b, st>>>(a);
   else k_adj_nl<false><<<gs, bs, 0, st>>>(a);

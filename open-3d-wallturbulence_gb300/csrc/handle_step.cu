@@ -555,8 +555,8 @@ void owt_handle::host_step_prepare() {
 // the scheduler places ahead of those of long kernels), the DY2 v history of
 // the chunk's modes is re-derived on a third stream, and the mode kernel
 // runs on the chunk's unique modes while the next chunks arrive.  One chunk
-// (everything) when the mode-kernel variant in use is not the quad mapping,
-// whose unique-mode ranges the chunks are.  History fields in pinned memory
+// (everything) where the mode kernel in use takes no range of unique modes (the
+// pair mapping and the full-band and sixth-order solves).  History fields in pinned memory
 // are uploaded by SM loads (launch_host_load), others by the copy engines:
 // at 384x257x384 copy-engine uploads of pinned memory ran at a tenth of the
 // host link's rate in every fourth or fifth call (about 230 instead of 80 ms
@@ -569,13 +569,13 @@ void owt_handle::step_host(const double *const *hist, const double *means, const
   ensure_tuned();
   ck(cudaStreamSynchronize(st), "host step");
   const int var = variant();
-  const bool quad = modes_sparse() && !sparse_v6 && modes_variant_is_quad(var);
+  const bool ranges = modes_sparse() && !sparse_v6 && modes_variant_has_ranges(var);
   // By default no chunk smaller than twice what is resident at once: a part of
   // the modes of a small channel takes the mode kernel as long as all of them
   // (0.96 against 1.02 ms for half of 128x129x128).
-  const int waves = 2 * str_groups(Uq) / (2 * 7 * 152);
+  const int waves = 2 * str_groups(Uq) / (2 * 7 * kSMs);  // seven resident blocks an SM (modes_stream.cu)
   const int want = host_chunks > 0 ? host_chunks : std::min(HostStep::kDefaultChunks, std::max(waves, 1));
-  const int nchunk = quad ? std::min(std::min(want, HostStep::kChunks), NZH + 1) : 1;
+  const int nchunk = ranges ? std::min(std::min(want, HostStep::kChunks), NZH + 1) : 1;
   // means first (the mean-mode kernel starts with the step)
   for (int w = 0; w < OWT_NUM_MEANS; ++w)
     ck(cudaMemcpyAsync(mean_ptr(w), means + 2 * (size_t)w * NY, NY * sizeof(double2), cudaMemcpyHostToDevice, hs.up),

@@ -21,13 +21,13 @@
 // Every value comes from the operations of mode_body in the same order, so
 // results are bitwise those of the other mappings.
 //
-// Measured, best other mapping -> this one: 384x257x384 13.85 -> 11.7 ms (the
-// FP64 pipe 95% busy, bound by it), 320x160x320 7.5 -> 5.6, 128x129x128
-// 1.81 -> 1.0, 64x97x48 1.38 -> 0.73, 32x65x32 0.62 -> 0.49 (a warp's own FP64
-// instructions 0.53 of the 128x129x128 time; the fullest SMs have four of the
-// 514 blocks there, the average 3.4), the 64-channel ensemble 4.79 -> 3.76.  A
+// Measured, best other mapping -> this one: 384x257x384 13.85 -> 11.6 ms (bound
+// by the FP64 pipe, 84% busy in a capture of 384x33x384), 320x160x320 7.5 -> 5.6,
+// 128x129x128 1.81 -> 1.0, 64x97x48 1.38 -> 0.73, 32x65x32 0.62 -> 0.49 (a warp's
+// own FP64 instructions 0.53 of the 128x129x128 time; the fullest SMs have four of
+// the 520 blocks there, the average 3.4), the 64-channel ensemble 4.79 -> 3.76.  A
 // cp.async ring over the band storage without packing gave 1.50 at
-// 128x129x128: 16 instructions for each FP64 one, against 9.5 here.
+// 128x129x128: 16 instructions for each FP64 one, against 9.8 here.
 //
 // Lanes 2q, 2q + 1 are Re, Im of unique mode 16 g + q (group g = warp / 2) with
 // the sign of kz of the warp (warp & 1: -kz); kz = 0 and the Nyquist row have

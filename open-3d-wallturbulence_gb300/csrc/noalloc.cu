@@ -150,7 +150,7 @@ extern "C" int owt_dy1_noalloc(int64_t NY, int64_t nlines, double alpha_mesh, co
     return fail(OWT_ERR_INVALID, "NY must be within [7, " + std::to_string(OWT_NOALLOC_MAX_NY) + "]");
   if (nlines < 1 || NY * nlines > (int64_t)OWT_NOALLOC_MAX_VALUES)
     return fail(OWT_ERR_INVALID, "NY * nlines must be within [1, " + std::to_string(OWT_NOALLOC_MAX_VALUES) +
-                                     "] complex values (the static scratch holds that many)");
+                                     "] complex values");
   if (!(alpha_mesh > 0)) return fail(OWT_ERR_INVALID, "alpha_mesh must be positive");
   if (!d_in || !d_out || ((uintptr_t)d_in % 16) || ((uintptr_t)d_out % 16))
     return fail(OWT_ERR_INVALID, "d_in and d_out must be 16-byte aligned device pointers");

@@ -311,7 +311,7 @@ bool band_supported(int kl, int ku) {
 int modes_variant_count() { return modes_pair_count() + modes_quad_count() + modes_stream_count(); }
 int modes_band_count() { return modes_pair_count() + modes_quad_count(); }
 // variants whose launches can be limited to a range of unique modes
-bool modes_variant_is_quad(int v) { return v >= modes_pair_count(); }
+bool modes_variant_has_ranges(int v) { return v >= modes_pair_count(); }
 const char *modes_variant_name(int v) {
   if (v < modes_pair_count()) return modes_pair_name(v);
   v -= modes_pair_count();
@@ -578,7 +578,7 @@ void launch_mean_batch(const BatchTable<MeanArgs> &t, bool smem, size_t smem_byt
 // threads a block: 64 spread a small channel (or a batch of them) over every SM,
 // 256 share one copy of the tables where the modes fill the GPU anyway
 constexpr int kNLThreads = 64, kNLThreadsLarge = 256;
-inline int nl_threads(const NLArgs &a) { return 2 * a.M >= 152 * 4 * kNLThreadsLarge ? kNLThreadsLarge : kNLThreads; }
+inline int nl_threads(const NLArgs &a) { return 2 * a.M >= kSMs * 4 * kNLThreadsLarge ? kNLThreadsLarge : kNLThreads; }
 // per row: B1 entries (4), L (2), 1/U_jj, U above the diagonal (4), c11
 constexpr int kNLRow = 12;
 constexpr size_t nl_smem_bytes(int NY) { return (size_t)NY * (kNLRow * sizeof(double) + 1) + 8; }
@@ -1022,7 +1022,7 @@ void launch_lamb_mean_shift(double2 *lx_ring, double2 *lz_ring, const double2 *l
 // this 59 (141 and 100 us a call with the read-back).
 constexpr int kStatsThreads = 256;
 int stats_parts(int NY, int M) {
-  return std::max(1, std::min((4 * 152 + NY - 1) / NY, M / (2 * kStatsThreads)));
+  return std::max(1, std::min((4 * kSMs + NY - 1) / NY, M / (2 * kStatsThreads)));
 }
 __global__ void __launch_bounds__(kStatsThreads)
     k_stats(const double2 *u, const double2 *v, const double2 *w, int NY, int NZ, int NXH, double *partial) {
@@ -1143,7 +1143,7 @@ __global__ void k_host_load(const float4 *__restrict__ src, float4 *__restrict__
 }
 void launch_host_load(const void *src, void *dst, size_t bytes, cudaStream_t st) {
   if (bytes == 0) return;
-  k_host_load<<<152, 256, 0, st>>>(static_cast<const float4 *>(src), static_cast<float4 *>(dst), bytes / 16);
+  k_host_load<<<kSMs, 256, 0, st>>>(static_cast<const float4 *>(src), static_cast<float4 *>(dst), bytes / 16);
 }
 // Physical fields: [y][z][x] (device) <-> [z][x][y] (the reference's
 // Field<double> layout), a rows x cols transpose of doubles.

@@ -15,6 +15,9 @@
 
 namespace owt {
 
+// SMs of the GB300, for rules on sizes; grids of resident blocks ask the device.
+constexpr int kSMs = 152;
+
 // The dynamic shared-memory limit is an attribute of the kernel function on
 // the current device, shared by every handle of the process.  Raise it to
 // what a handle needs, never lower it: a smaller channel created after a
@@ -42,7 +45,7 @@ struct StrRow {
 
 struct ModeArgs {
   int NY, NZ, NXH, NZH, M, U;
-  int u0, u1;  // quad mapping: unique modes u0 <= u < u1 only (0, U: all)
+  int u0, u1;  // quad and stream mappings: unique modes u0 <= u < u1 only (0, U: all)
   double inv_dt, nu;
   const double *kx, *kz;
   double2 *v_ring, *g_ring, *hv_ring, *hg_ring, *q_ring;  // 3 slots each, [slot][y][mode]
@@ -205,13 +208,13 @@ struct StrBuffers {
   double *vf = nullptr, *vb = nullptr, *gf = nullptr, *gb = nullptr, *vrs = nullptr, *grs = nullptr;
 };
 void launch_str_pack(const ModeArgs &a, bool sixth, const StrBuffers &s, int nvrows, int ngrows, cudaStream_t st);
-int modes_pair_count();  // variants below this index use the pair mapping, the others the quad mapping
+int modes_pair_count();  // variants below this index use the pair mapping, the others the quad and stream mappings
 void launch_modes_sixth(const ModeArgs &a, cudaStream_t st);  // masked solve with the sixth-order fill
 // dst[p U + u] = scale[u] src[p U + u], p < n
 void launch_scale_by_mode(double *dst, const double *src, const double *scale, int n, int U, cudaStream_t st);
 int modes_variant_count();  // pair, quad and stream mappings
 int modes_band_count();     // of them those on the band storage, the first ones
-bool modes_variant_is_quad(int v);
+bool modes_variant_has_ranges(int v);  // takes u0 .. u1
 const char *modes_variant_name(int v);
 void launch_check_pattern(int which, const double *ab, const uint8_t *piv, int n, int U, int *bad,
                           cudaStream_t st);
