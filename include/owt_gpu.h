@@ -293,9 +293,9 @@ int owt_state_restore(owt_handle *h);
  * OWT_OPT_STREAM_BYTES: device memory the mode kernel's packed copy of the
  *   factors may take, in bytes (-1, the default: what the device has).  Where
  *   it does not fit, the kernel reads the factors themselves: slower, with the
- *   same results.  The copy is also given back when another allocation of the
- *   handle fails, and made again before the next step; not while the handle
- *   steps in a batch that uses it.
+ *   same results.  The copy is also given back when another allocation fails,
+ *   of this handle or of any other on the device, and made again before the
+ *   next step; not once the handle is in a batch that uses it.
  * OWT_INFO_SPARSE_SOLVE: 1 if the interior-sparse v-system solve is active.
  * OWT_INFO_PATTERN_VIOLATIONS: modes whose factors fell outside the sparse
  *   pattern at setup (any such mode selects the full-band solve).

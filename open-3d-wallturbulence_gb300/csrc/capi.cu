@@ -25,6 +25,7 @@ int owt_create(const owt_params *params, owt_handle **out) {
   owt_handle *h = new owt_handle();
   try {
     h->setup(*params);
+    enlist(h);
   } catch (const OwtError &e) {
     g_create_error = e.what();
     delete h;
@@ -39,6 +40,7 @@ int owt_create(const owt_params *params, owt_handle **out) {
 }
 
 int owt_destroy(owt_handle *h) {
+  delist(h);
   delete h;
   return OWT_OK;
 }
@@ -278,6 +280,7 @@ const char *owt_setup_report(const owt_handle *h) { return h ? h->setup_report.c
 
 int owt_get_info(const owt_handle *h, int what, int64_t *value) {
   if (!h || !value) return OWT_ERR_INVALID;
+  std::lock_guard<std::mutex> lk(h->busy);
   switch (what) {
     case OWT_INFO_SPARSE_SOLVE: *value = ((h->sparse_v || h->sparse_v6) && !h->force_dense) ? 1 : 0; return OWT_OK;
     case OWT_INFO_PATTERN_VIOLATIONS: *value = h->pattern_violations; return OWT_OK;

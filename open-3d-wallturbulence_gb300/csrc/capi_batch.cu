@@ -225,14 +225,7 @@ struct owt_batch {
       for (size_t i = 0; i < hs.size(); ++i) {
         owt_handle *h = hs[i];
         const size_t fs = h->fs;
-        cudaError_t e = cudaMalloc(&snap[i], 13 * fs * sizeof(double2));
-        if (e == cudaErrorMemoryAllocation) {  // streams of the channels' own steps
-          bool any = false;
-          for (owt_handle *r : hs) any = r->release_streams() || any;
-          cudaGetLastError();
-          if (any) e = cudaMalloc(&snap[i], 13 * fs * sizeof(double2));
-        }
-        ck(e, "tuning snapshot");
+        ck(device_malloc(reinterpret_cast<void **>(&snap[i]), 13 * fs * sizeof(double2)), "tuning snapshot");
         double2 *o = snap[i];
         for (double2 *ring : {h->v_ring, h->g_ring, h->q_ring}) {
           ck(cudaMemcpyAsync(o, ring, 3 * fs * sizeof(double2), cudaMemcpyDeviceToDevice, st), "snapshot");
@@ -244,7 +237,11 @@ struct owt_batch {
         }
       }
       bool streams = true;
-      for (int i : by_size(true)) streams = streams && hs[i]->build_streams();
+      for (int i : by_size(true)) {
+        std::lock_guard<std::mutex> lk(hs[i]->busy);
+        streams = streams && hs[i]->build_streams();
+        ++hs[i]->str_users;
+      }
       for (owt_handle *h : hs) ck(cudaStreamSynchronize(h->st), "factor streams");
       ck(cudaEventCreate(&e0), "event");
       ck(cudaEventCreate(&e1), "event");
@@ -286,8 +283,11 @@ struct owt_batch {
       throw;
     }
     cleanup();
-    if (modes_variant >= modes_band_count())
-      for (int i : by_size(true)) hs[i]->str_kept = true;
+    if (modes_variant < modes_band_count())
+      for (int i : by_size(true)) {
+        std::lock_guard<std::mutex> lk(hs[i]->busy);
+        --hs[i]->str_users;
+      }
     tuning += std::string(" -> ") + modes_variant_name(modes_variant);
   }
 };

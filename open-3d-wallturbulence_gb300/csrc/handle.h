@@ -20,6 +20,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -37,8 +38,13 @@ extern thread_local std::string g_create_error;
 extern thread_local size_t *g_alloc_counter;
 // The handle whose entry point the thread is in (guard), or null.
 extern thread_local owt_handle *g_handle;
-// Give back what that handle holds only to be faster; false: nothing to give.
+// Give back device memory that is held only to be faster: that handle's factor
+// streams, else those of the other handles on the current device that no thread
+// is using.  false: nothing to give.
 bool release_for_allocation();
+// Handles that can be asked (owt_create, owt_destroy).
+void enlist(owt_handle *h);
+void delist(owt_handle *h);
 
 struct CudaError : std::runtime_error {
   using std::runtime_error::runtime_error;
@@ -52,15 +58,21 @@ inline void ck(cudaError_t e, const char *what) {
   if (e != cudaSuccess) throw CudaError(std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+// cudaMalloc, once more with that memory where there is none left
+inline cudaError_t device_malloc(void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && release_for_allocation()) {
+    cudaGetLastError();
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
 template <typename T>
 T *dalloc(size_t n, std::vector<void *> &owned) {
   void *p = nullptr;
   if (n == 0) n = 1;
-  cudaError_t e = cudaMalloc(&p, n * sizeof(T));
-  if (e == cudaErrorMemoryAllocation && release_for_allocation()) {
-    cudaGetLastError();
-    e = cudaMalloc(&p, n * sizeof(T));
-  }
+  cudaError_t e = device_malloc(&p, n * sizeof(T));
   if (e != cudaSuccess) {
     cudaGetLastError();
     throw OwtError(OWT_ERR_NOMEM, std::string("cudaMalloc of ") + std::to_string(n * sizeof(T)) +
@@ -88,6 +100,7 @@ struct BandDev {
 }  // namespace owt
 
 struct owt_handle {
+  mutable std::mutex busy;  // a thread is in one of the handle's entry points (guard)
   std::string err;
   owt_params p{};
   int NX = 0, NY = 0, NZ = 0, NXH = 0, NZH = 0, NX2 = 0, NZ2 = 0, M = 0, Uq = 0;
@@ -135,7 +148,7 @@ struct owt_handle {
   owt::StrRow *vrows = nullptr, *grows = nullptr;
   // Packed factor streams (modes_stream.cuh), a second copy of the factors
   // that makes the mode kernel faster.  Built before a step where they fit the
-  // device and their limit; released when another allocation of the handle
+  // device and their limit; released when another allocation of this library
   // fails, and built again before the next step.  Without them the mode kernel
   // reads the band storage (the sixth-order and the adjoint solves the full
   // band), with the same results.
@@ -143,7 +156,7 @@ struct owt_handle {
   size_t str_bytes = 0;
   int64_t str_limit = -1;   // bytes they may take (-1: any number)
   bool str_denied = false;  // they did not fit: not tried again
-  bool str_kept = false;    // a batch holds their addresses: never released
+  int str_users = 0;        // batches made with their addresses: never released
   int n_vrows = 0, n_grows = 0;
   bool build_streams();     // whether the handle has them
   bool release_streams();
@@ -330,12 +343,13 @@ namespace owt {
 template <typename F>
 int guard(owt_handle *h, F &&f) {
   if (!h) return OWT_ERR_INVALID;
-  struct Within {
-    owt_handle *before = g_handle;
-    explicit Within(owt_handle *now) { g_handle = now; }
-    ~Within() { g_handle = before; }
-  } within(h);
   try {
+    std::lock_guard<std::mutex> lk(h->busy);
+    struct Within {
+      owt_handle *before = g_handle;
+      explicit Within(owt_handle *now) { g_handle = now; }
+      ~Within() { g_handle = before; }
+    } within(h);
     f();
     h->err.clear();
     return OWT_OK;

@@ -9,7 +9,43 @@ using namespace owt;
 namespace owt {
 thread_local size_t *g_alloc_counter = nullptr;
 thread_local owt_handle *g_handle = nullptr;
-bool release_for_allocation() { return g_handle && g_handle->release_streams(); }
+
+namespace {
+struct Handles {
+  std::mutex mu;
+  std::vector<owt_handle *> all;
+};
+Handles &handles() {
+  static Handles *h = new Handles;  // outlives handles that static objects destroy
+  return *h;
+}
+}  // namespace
+void enlist(owt_handle *h) {
+  std::lock_guard<std::mutex> lk(handles().mu);
+  handles().all.push_back(h);
+}
+void delist(owt_handle *h) {
+  std::lock_guard<std::mutex> lk(handles().mu);
+  auto &all = handles().all;
+  all.erase(std::remove(all.begin(), all.end(), h), all.end());
+}
+bool release_for_allocation() {
+  if (g_handle && g_handle->release_streams()) return true;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  bool any = false;
+  std::lock_guard<std::mutex> lk(handles().mu);
+  for (owt_handle *h : handles().all) {
+    // (never waits for another thread's handle, so no order of locks matters)
+    if (h == g_handle || h->p.device != dev || !h->busy.try_lock()) continue;
+    std::lock_guard<std::mutex> own(h->busy, std::adopt_lock);
+    try {
+      any = h->release_streams() || any;
+    } catch (const std::exception &) {  // its error is its own: its next call reports it
+    }
+  }
+  return any;
+}
 }  // namespace owt
 
 owt_handle::~owt_handle() {

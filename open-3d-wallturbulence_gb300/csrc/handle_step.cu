@@ -190,12 +190,22 @@ bool owt_handle::build_streams() {
     for (const auto &q : parts) {
       bytes += q.second * sizeof(double);
       if (str_limit >= 0 && bytes > (size_t)str_limit) throw OwtError(OWT_ERR_NOMEM, "factor streams beyond their limit");
-      *q.first = dalloc<double>(q.second, got);
+      // (not dalloc, which would take other handles' streams for this one's)
+      void *d = nullptr;
+      const cudaError_t e = cudaMalloc(&d, std::max(q.second, (size_t)1) * sizeof(double));
+      if (e == cudaErrorMemoryAllocation) throw OwtError(OWT_ERR_NOMEM, "factor streams do not fit");
+      ck(e, "factor streams");
+      got.push_back(d);
+      *q.first = static_cast<double *>(d);
     }
   } catch (const OwtError &) {
+    cudaGetLastError();
     for (void *q : got) cudaFree(q);
     str_denied = true;
     return false;
+  } catch (...) {
+    for (void *q : got) cudaFree(q);
+    throw;
   }
   owned.insert(owned.end(), got.begin(), got.end());
   device_bytes += bytes;
@@ -209,7 +219,9 @@ bool owt_handle::build_streams() {
 }
 
 bool owt_handle::release_streams() {
-  if (!str.vf || str_kept) return false;
+  if (!str.vf || str_users) return false;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
   ck(cudaStreamSynchronize(st), "factor streams");
   drop_graph();  // it holds their addresses
   for (double *q : {str.vf, str.vb, str.gf, str.gb, str.vrs, str.grs}) free_owned(q);
@@ -237,7 +249,7 @@ void owt_handle::ensure_tuned() {
   }
   recompute_dirty_q();
   double2 *snap = nullptr;
-  ck(cudaMalloc(&snap, 13 * fs * sizeof(double2)), "tuning snapshot");
+  ck(device_malloc(reinterpret_cast<void **>(&snap), 13 * fs * sizeof(double2)), "tuning snapshot");
   try {
     build_streams();  // (after the snapshot, which the trials cannot do without)
     double2 *o = snap;

@@ -149,3 +149,59 @@ def test_batch_with_a_channel_without_streams(gpu_lib):
     for x, y in zip(*got):
         for a, c in zip(x, y):
             np.testing.assert_array_equal(a, c)
+
+
+def _fill(s):
+    """An allocation of handle s that no device has room for."""
+    from owt.lib import OwtError
+    s.drag_forward(1, 10 ** 9)
+    with pytest.raises(OwtError) as e:
+        s.drag_backward()
+    assert e.value.code == 5
+
+
+def test_other_handles_give_their_streams(reference):
+    """Where an allocation of one handle fails, idle handles give back their
+    streams, go on with the same bits and build them again; a batch keeps its own."""
+    from owt.batch import Batch
+    order, ref, size = reference
+    s, asking, member = _solver(_params(order)), _solver(_params(8)), _solver(_params(8), seed=4)
+    s.time_Integration(2)
+    asking.time_Integration(1)
+    b = Batch([member])
+    held = [x.info("device_bytes") for x in (s, member)]
+    _fill(asking)  # the first time its own go, the second time the others'
+    assert s.info("device_bytes") == held[0]
+    _fill(asking)
+    asking.limit_stream_bytes(0)
+    _fill(asking)
+    assert s.info("device_bytes") == held[0] - size
+    if "stream" in b.tuning_report().split("->")[1]:
+        assert member.info("device_bytes") == held[1]
+    s.time_Integration(1)
+    assert s.info("device_bytes") == held[0]
+    _same(s, ref)
+    alone = _solver(_params(8), seed=4)
+    alone.time_Integration(2)
+    b.step(2)
+    b.synchronize()
+    _same(member, alone)
+    b.close()
+    for x in (s, asking, member, alone):
+        x.close()
+
+
+def test_giving_streams_while_another_thread_steps(gpu_lib):
+    import threading
+    p = _params(8)
+    ref, s, asking = _solver(p), _solver(p), _solver(p, seed=9)
+    ref.time_Integration(200)
+    asking.limit_stream_bytes(0)
+    t = threading.Thread(target=lambda: [s.time_Integration(1) for _ in range(200)])
+    t.start()
+    while t.is_alive():
+        _fill(asking)
+    t.join()
+    _same(s, ref)
+    for x in (ref, s, asking):
+        x.close()
